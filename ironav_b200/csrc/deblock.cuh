@@ -4,13 +4,11 @@
 // The reference filters macroblocks in raster order (deblock_picture, deblock.rs:410-429); filtering a
 // macroblock changes up to 3 samples on either side of its left and top edges, so macroblock (x, y) must
 // see the final samples of (x - 1, y) and of (x + 1, y - 1) — the dependency deblock_picture_par keeps with
-// its row wavefront (deblock.rs:583-605). Here one warp filters one macroblock row left to right, rows
-// handed out by ticket, and before macroblock x it waits (bounded) until the row above has filtered
-// macroblocks 0..x+1. Inside a macroblock the lanes take lines: 16 luma lines, 8 Cb and 8 Cr lines
-// (rows for the vertical edges, then columns for the horizontal edges), on a staged tile of the
-// macroblock with the 4 (luma) / 2 (chroma) samples left of and above it in shared memory. Samples shared
-// between warps move through L2 only (ld.global.cg / st.global.cg) and are published with a release store
-// of the row's progress.
+// its row wavefront (deblock.rs:583-605). Here the picture's macroblock rows go by groups of 4, a
+// CTA a group and plane kind handed out by ticket, one warp a row left to right. Inside a macroblock the lanes take lines: 16 luma lines, or 8 Cb
+// and 8 Cr lines (rows for the vertical edges, in registers, then columns for the horizontal edges, in shared memory).
+// The rows of a group hand over through rings in shared memory; between groups, samples move through L2 and are
+// published with a release store of the row's progress.
 #pragma once
 #include "common.cuh"
 
@@ -89,66 +87,63 @@ static __device__ bool dbk_motion_differs(const ironav_dbk_mb& p, int pbx, int p
     return (dbk_far(pm0, qm0) || dbk_far(pm1, qm1)) && (dbk_far(pm0, qm1) || dbk_far(pm1, qm0));
 }
 
-// filter_line, deblock.rs:279-333, on the staged line whose first sample past the edge is q[0] (step xs
-// across the edge); the side of a keep macroblock (I_PCM / lossless) is left as it was (filter_edge,
-// deblock.rs:251-272).
-__device__ __forceinline__ void dbk_line(int* q, int xs, int b, int tc0, int alpha, int beta, bool chroma, int maxv, bool keep_p,
-                                         bool keep_q) {
-    const int p0 = q[-xs], q0 = q[0], p1 = q[-2 * xs], q1 = q[xs];
-    if (abs(p0 - q0) >= alpha || abs(p1 - p0) >= beta || abs(q1 - q0) >= beta) return;
-    if (chroma) {
-        int np0, nq0;
-        if (b < 4) {
-            const int tc = tc0 + 1;
-            const int delta = min(max((((q0 - p0) << 2) + (p1 - q1) + 4) >> 3, -tc), tc);
-            np0 = min(max(p0 + delta, 0), maxv);
-            nq0 = min(max(q0 - delta, 0), maxv);
-        } else {
-            np0 = (2 * p1 + p0 + q1 + 2) >> 2;
-            nq0 = (2 * q1 + q0 + p1 + 2) >> 2;
-        }
-        if (!keep_p) q[-xs] = np0;
-        if (!keep_q) q[0] = nq0;
+// An edge as a line's filter wants it: the thresholds at the picture's depth (alpha 0: not filtered, no sample differs
+// by less), tC0 by the line's strength, and which sides are kept.
+struct DbkEdge {
+    int b, alpha, beta, tc0;
+    bool keep_p, keep_q;
+};
+// From an edge word and the line's strength b on it.
+__device__ __forceinline__ DbkEdge dbk_edge(uint32_t wv, int b, int bd) {
+    DbkEdge e;
+    e.b = b;
+    e.alpha = b ? (int)(wv & 0xff) << (bd - 8) : 0;
+    e.beta = (int)((wv >> 8) & 0x1f) << (bd - 8);
+    e.tc0 = (int)((wv >> (8 + 5 * (b & 3))) & 0x1f) << (bd - 8);  // strength 4 has none
+    e.keep_p = (wv >> 28) & 1;
+    e.keep_q = (wv >> 29) & 1;
+    return e;
+}
+
+// filter_line, deblock.rs:279-333, on a line in registers whose first sample past the edge is q[0]; the side of a
+// keep macroblock (I_PCM / lossless) is left as it was (filter_edge, deblock.rs:251-272). OUTER: a macroblock's
+// outer edge, the only kind whose strength can be 4 (all along the edge, so the warp takes one path). Everything a line's own samples decide
+// is selected, not branched on: the filter is a serial chain of eight edges a macroblock on one warp, where a branch costs
+// as much as ten instructions.
+template <bool CHROMA, bool OUTER>
+__device__ __forceinline__ void dbk_line(int* q, const DbkEdge& E, int maxv) {
+    const int p0 = q[-1], q0 = q[0], p1 = q[-2], q1 = q[1];
+    const bool f = abs(p0 - q0) < E.alpha && abs(p1 - p0) < E.beta && abs(q1 - q0) < E.beta;
+    const bool fp = f && !E.keep_p, fq = f && !E.keep_q;
+    const bool strong = OUTER && E.b == 4;
+    if constexpr (CHROMA) {
+        const int tc = E.tc0 + 1;
+        const int delta = min(max((((q0 - p0) << 2) + (p1 - q1) + 4) >> 3, -tc), tc);
+        const int np0 = strong ? (2 * p1 + p0 + q1 + 2) >> 2 : min(max(p0 + delta, 0), maxv);
+        const int nq0 = strong ? (2 * q1 + q0 + p1 + 2) >> 2 : min(max(q0 - delta, 0), maxv);
+        q[-1] = fp ? np0 : p0;
+        q[0] = fq ? nq0 : q0;
         return;
     }
-    const int p2 = q[-3 * xs], q2 = q[2 * xs];
-    const int ap = abs(p2 - p0), aq = abs(q2 - q0);
-    int np0 = p0, np1 = p1, np2 = p2, nq0 = q0, nq1 = q1, nq2 = q2;
-    if (b < 4) {
-        const int tc = tc0 + (ap < beta) + (aq < beta);
+    const int p2 = q[-3], q2 = q[2];
+    const bool ap = abs(p2 - p0) < E.beta, aq = abs(q2 - q0) < E.beta;
+    if (!strong) {
+        const int tc = E.tc0 + ap + aq, avg = (p0 + q0 + 1) >> 1;
         const int delta = min(max((((q0 - p0) << 2) + (p1 - q1) + 4) >> 3, -tc), tc);
-        np0 = min(max(p0 + delta, 0), maxv);
-        nq0 = min(max(q0 - delta, 0), maxv);
-        if (ap < beta) np1 = p1 + min(max((p2 + ((p0 + q0 + 1) >> 1) - (p1 << 1)) >> 1, -tc0), tc0);
-        if (aq < beta) nq1 = q1 + min(max((q2 + ((p0 + q0 + 1) >> 1) - (q1 << 1)) >> 1, -tc0), tc0);
+        q[-1] = fp ? min(max(p0 + delta, 0), maxv) : p0;
+        q[0] = fq ? min(max(q0 - delta, 0), maxv) : q0;
+        q[-2] = fp && ap ? p1 + min(max((p2 + avg - (p1 << 1)) >> 1, -E.tc0), E.tc0) : p1;
+        q[1] = fq && aq ? q1 + min(max((q2 + avg - (q1 << 1)) >> 1, -E.tc0), E.tc0) : q1;
     } else {
-        const bool small = abs(p0 - q0) < (alpha >> 2) + 2;
-        if (ap < beta && small) {
-            const int p3 = q[-4 * xs];
-            np0 = (p2 + 2 * p1 + 2 * p0 + 2 * q0 + q1 + 4) >> 3;
-            np1 = (p2 + p1 + p0 + q0 + 2) >> 2;
-            np2 = (2 * p3 + 3 * p2 + p1 + p0 + q0 + 4) >> 3;
-        } else {
-            np0 = (2 * p1 + p0 + q1 + 2) >> 2;
-        }
-        if (aq < beta && small) {
-            const int q3 = q[3 * xs];
-            nq0 = (p1 + 2 * p0 + 2 * q0 + 2 * q1 + q2 + 4) >> 3;
-            nq1 = (p0 + q0 + q1 + q2 + 2) >> 2;
-            nq2 = (2 * q3 + 3 * q2 + q1 + q0 + p0 + 4) >> 3;
-        } else {
-            nq0 = (2 * q1 + q0 + p1 + 2) >> 2;
-        }
-    }
-    if (!keep_p) {
-        q[-xs] = np0;
-        q[-2 * xs] = np1;
-        q[-3 * xs] = np2;
-    }
-    if (!keep_q) {
-        q[0] = nq0;
-        q[xs] = nq1;
-        q[2 * xs] = nq2;
+        const bool small = abs(p0 - q0) < (E.alpha >> 2) + 2;
+        const bool sp = ap && small, sq = aq && small;
+        const int p3 = q[-4], q3 = q[3], m = p0 + q0;
+        q[-1] = fp ? (sp ? (p2 + 2 * p1 + 2 * m + q1 + 4) >> 3 : (2 * p1 + p0 + q1 + 2) >> 2) : p0;
+        q[0] = fq ? (sq ? (q2 + 2 * q1 + 2 * m + p1 + 4) >> 3 : (2 * q1 + q0 + p1 + 2) >> 2) : q0;
+        q[-2] = fp && sp ? (p2 + p1 + m + 2) >> 2 : p1;
+        q[1] = fq && sq ? (q2 + q1 + m + 2) >> 2 : q1;
+        q[-3] = fp && sp ? (2 * p3 + 3 * p2 + p1 + m + 4) >> 3 : p2;
+        q[2] = fq && sq ? (2 * q3 + 3 * q2 + q1 + m + 4) >> 3 : q2;
     }
 }
 
@@ -265,25 +260,7 @@ static __global__ void __launch_bounds__(DBK_WARPS * 32) deblock_edges_kernel(co
 
 // ---- pass 2: the samples, in the row wavefront ---------------------------------------------------------
 
-// N samples of type T at p (aligned to their size, at most 16 bytes) into ints, through L2; and back.
-template <class T, int N>
-__device__ __forceinline__ void dbk_load(const T* p, int* v) {
-    constexpr int NB = N * (int)sizeof(T);
-    uint32_t w[NB >= 4 ? NB / 4 : 1];
-    if constexpr (NB == 16) {
-        const uint4 q = __ldcg(reinterpret_cast<const uint4*>(p));
-        w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
-    } else if constexpr (NB == 8) {
-        const uint2 q = __ldcg(reinterpret_cast<const uint2*>(p));
-        w[0] = q.x, w[1] = q.y;
-    } else if constexpr (NB == 4) {
-        w[0] = __ldcg(reinterpret_cast<const unsigned*>(p));
-    } else {
-        w[0] = __ldcg(reinterpret_cast<const unsigned short*>(p));
-    }
-#pragma unroll
-    for (int k = 0; k < N; k++) v[k] = (int)((w[(k * (int)sizeof(T)) >> 2] >> ((k * 8 * (int)sizeof(T)) & 31)) & ((1u << (8 * sizeof(T))) - 1));
-}
+// N samples of type T from ints to p (aligned to their size, at most 16 bytes), through L2.
 template <class T, int N>
 __device__ __forceinline__ void dbk_store(T* p, const int* v) {
     constexpr int NB = N * (int)sizeof(T);
@@ -295,40 +272,16 @@ __device__ __forceinline__ void dbk_store(T* p, const int* v) {
     else if constexpr (NB == 4) __stcg(reinterpret_cast<unsigned*>(p), w[0]);
     else __stcg(reinterpret_cast<unsigned short*>(p), (unsigned short)w[0]);
 }
-// Up to 16 samples (two 16-byte pieces for 16 samples of 16 bits).
-template <class T, int N>
-__device__ __forceinline__ void dbk_load_row(const T* p, int* v) {
-    if constexpr (N * sizeof(T) > 16) {
-        dbk_load<T, N / 2>(p, v);
-        dbk_load<T, N / 2>(p + N / 2, v + N / 2);
-    } else {
-        dbk_load<T, N>(p, v);
-    }
-}
-template <class T, int N>
-__device__ __forceinline__ void dbk_store_row(T* p, const int* v) {
-    if constexpr (N * sizeof(T) > 16) {
-        dbk_store<T, N / 2>(p, v);
-        dbk_store<T, N / 2>(p + N / 2, v + N / 2);
-    } else {
-        dbk_store<T, N>(p, v);
-    }
-}
-
-// Filters the edges across one line of NS samples (luma: 20 = 4 before the macroblock + 16; chroma: 10 =
-// 2 + 8) in registers: luma edges at 4, 8, 12, 16; chroma edges at 2 and 6.
+// The four (luma) or two (chroma) edges across one line of NS samples (luma: 20 = 4 before the macroblock + 16; chroma: 10
+// = 2 + 8) in registers: luma edges at 4, 8, 12, 16; chroma edges at 2 and 6.
 template <bool CHROMA, int NS>
-__device__ __forceinline__ void dbk_filter_lines(int (&v)[NS], const uint32_t* words, const uint8_t (*bs)[4], int seg, int bd, int maxv) {
+__device__ __forceinline__ void dbk_outer(int (&v)[NS], const DbkEdge (&e)[CHROMA ? 2 : 4], int maxv) {
+    dbk_line<CHROMA, true>(&v[CHROMA ? 2 : 4], e[0], maxv);
+}
+template <bool CHROMA, int NS>
+__device__ __forceinline__ void dbk_inner(int (&v)[NS], const DbkEdge (&e)[CHROMA ? 2 : 4], int maxv) {
 #pragma unroll
-    for (int k = 0; k < (CHROMA ? 2 : 4); k++) {
-        const uint32_t wv = words[k];
-        const int e = CHROMA ? 2 * k : k;
-        const int b = bs[e][seg];
-        if (wv == 0 || b == 0) continue;
-        const int alpha = (int)(wv & 0xff) << (bd - 8), beta = (int)((wv >> 8) & 0x1f) << (bd - 8);
-        const int tc0 = b < 4 ? (int)((wv >> (8 + 5 * b)) & 0x1f) << (bd - 8) : 0;
-        dbk_line(&v[CHROMA ? 2 + 4 * k : 4 + 4 * k], 1, b, tc0, alpha, beta, CHROMA, maxv, (wv >> 28) & 1, (wv >> 29) & 1);
-    }
+    for (int k = 1; k < (CHROMA ? 2 : 4); k++) dbk_line<CHROMA, false>(&v[CHROMA ? 2 + 4 * k : 4 + 4 * k], e[k], maxv);
 }
 
 __device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
@@ -336,147 +289,379 @@ __device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+// Acquire load and release store of a word in shared memory, ordered within the CTA.
+__device__ __forceinline__ unsigned ld_acquire_cta(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_shared(unsigned* p, unsigned v) {  // relaxed; a fence before it makes a release
+    asm volatile("st.relaxed.cta.shared.u32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_release_cta(unsigned* p, unsigned v) {
+    asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v) : "memory");
+}
 
-// Waits until progress word `w` reaches `need`, at most P.wait_limit polls; false when it gave up or
-// another warp already did (the error word is looked at every 64 polls). Relaxed polls, then one acquire
-// fence: with the writer's release store they order the writer's samples before this warp's loads.
-__device__ __forceinline__ bool dbk_wait(const DbkParams& P, const unsigned* w, unsigned need) {
+// A CTA filters a group of DBK_ROWS macroblock rows of one plane kind, one warp a row, with the rows of a
+// group handing over through shared memory. What bounds the filter is the chain of mb_w + 2 (mb_h - 1)
+// dependent macroblocks, so a step may wait on nothing slower than shared memory:
+//   - a macroblock's samples and edge words come from global memory DBK_AHEAD - 1 steps ahead (cp.async);
+//   - a row leaves the bottom rows (4 luma, 2 chroma) of its macroblocks in a ring that the row below reads,
+//     with a progress word and a consumed word in shared memory (release and acquire at CTA scope);
+//   - the group's first row reads a ring that a fetch warp fills from global memory, several macroblocks at
+//     a time, as the group above publishes its last row; the publishing, with its device-scope fence, is a
+//     warp of its own too. A group boundary then costs its latency once a picture, not once a step;
+//   - a macroblock waits for the row above only when its top edge is filtered, and a direction without a
+//     filtered edge skips its pass (and its transposition through shared memory).
+// Four rows a group: a row's step is one warp's chain of ~650 instructions, and more rows an SM slow each other down (1080p
+// with every edge filtered: 460, 405, 370 and 353 us at 14, 10, 6 and 4 rows), while a group boundary adds ~3 us. A P
+// picture's records at 1080p, 8 bits: 188 us; a warp a row on its own, handing over every step through L2 (a device-scope release and an
+// acquire, ~3 us a step), took 822 us.
+constexpr int DBK_ROWS = 4;
+constexpr int DBK_AHEAD = 4;
+constexpr int DBK_GROUP_THREADS = (DBK_ROWS + 2) * 32;
+constexpr unsigned DBK_SPINS = 1u << 28;  // polls of a shared-memory word before a warp gives up
+
+template <class T>
+struct DbkGroup {
+    static constexpr int RING = sizeof(T) == 1 ? 8 : 4;  // macroblocks a ring holds
+    __align__(16) T ring[DBK_ROWS][RING][64];            // above row j: luma [4][16], chroma [comp][2][8]
+    __align__(16) T own[DBK_ROWS][DBK_AHEAD][256];       // luma [16][16], chroma [comp][8][8]
+    __align__(16) DbkEdges e[DBK_ROWS][DBK_AHEAD];
+    unsigned prog[DBK_ROWS + 1];  // [j]: macroblocks whose bottom rows above row j are final
+    unsigned cons[DBK_ROWS];      // [j]: macroblocks row j has done with
+    unsigned stop, ticket;
+};
+
+template <int NB>
+__device__ __forceinline__ void dbk_cp_async(void* dst, const void* src) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if constexpr (NB == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+
+// Waits until the shared word reaches `need`; false when it gave up or another warp of the group did.
+template <class T>
+__device__ __forceinline__ bool dbk_spin(const DbkParams& P, DbkGroup<T>& G, const unsigned* w, unsigned need) {
     for (unsigned i = 0;; i++) {
-        if (ld_relaxed(w) >= need) {
+        if (ld_acquire_cta(w) >= need) return true;
+        if ((i & 15) == 15) {
+            if (ld_acquire_cta(&G.stop)) return false;
+            if (i >= DBK_SPINS) {
+                atomicOr(P.err, 1u);
+                st_release_cta(&G.stop, 1u);
+                return false;
+            }
+            __nanosleep(20);
+        }
+    }
+}
+
+// NW 32-bit words between registers and memory (16-, 8- or 4-byte pieces; the address aligned to them).
+template <int NW>
+__device__ __forceinline__ void dbk_words_ld(const void* p, uint32_t* w) {
+    if constexpr (NW % 4 == 0) {
+#pragma unroll
+        for (int k = 0; k < NW / 4; k++) {
+            const uint4 q = reinterpret_cast<const uint4*>(p)[k];
+            w[4 * k] = q.x, w[4 * k + 1] = q.y, w[4 * k + 2] = q.z, w[4 * k + 3] = q.w;
+        }
+    } else {
+        const uint2 q = *reinterpret_cast<const uint2*>(p);
+        w[0] = q.x, w[1] = q.y;
+    }
+}
+template <int NW>
+__device__ __forceinline__ void dbk_words_st(void* p, const uint32_t* w) {
+    if constexpr (NW % 4 == 0) {
+#pragma unroll
+        for (int k = 0; k < NW / 4; k++) reinterpret_cast<uint4*>(p)[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+    } else {
+        *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+    }
+}
+// N samples of type T from ints to shared memory at p (aligned to their size).
+template <class T, int N>
+__device__ __forceinline__ void dbk_store_shared(T* p, const int* v) {
+#pragma unroll
+    for (int k = 0; k < N; k++) p[k] = (T)v[k];
+}
+template <class T>
+__device__ __forceinline__ int dbk_sample(const uint32_t* w, int k) {
+    return (int)((w[(k * (int)sizeof(T)) >> 2] >> ((k * 8 * (int)sizeof(T)) & 31)) & ((1u << (8 * sizeof(T))) - 1));
+}
+
+// Row j of the group (macroblock row y), left to right, by one warp. Luma: lanes 0-15 hold the macroblock's
+// 16 rows; chroma: lanes 0-7 the Cb rows, 8-15 the Cr rows; lanes 16-31 work on the same lines and store nothing, so that
+// the warp does not diverge. The vertical edges are filtered in those registers, with the LEFT samples kept from the
+// previous macroblock; the outer one makes the previous macroblock final, so its last columns go out and its bottom rows are
+// published. The horizontal edges are filtered on columns, the macroblock in its staging buffer and the rows above in
+// the ring. below: this group has a row j + 1, which the ring above it is filled for.
+template <class T, bool CHROMA>
+__device__ __forceinline__ void dbk_group_row(const DbkParams& P, const DbkEdges* __restrict__ edges, DbkGroup<T>& G, int j, int y, bool below) {
+    constexpr int W = CHROMA ? 8 : 16;    // samples of a macroblock row (and rows)
+    constexpr int LEFT = CHROMA ? 2 : 4;  // samples kept to its left
+    constexpr int H = CHROMA ? 2 : 4;     // rows above
+    constexpr int NE = CHROMA ? 2 : 4;    // edges a direction
+    constexpr int NW = W * (int)sizeof(T) / 4;
+    constexpr int N = DbkGroup<T>::RING;
+    constexpr int RB = W * (int)sizeof(T);  // bytes of a macroblock row
+    const int lane = threadIdx.x & 31, ln = lane & 15;
+    const bool active = lane < 16;
+    const int comp = CHROMA ? ln >> 3 : 0, line = CHROMA ? ln & 7 : ln;
+    T* const Pl = reinterpret_cast<T*>(P.planes[CHROMA ? 1 + comp : 0]);
+    const int stride = CHROMA ? P.cs : P.ys, mb_w = P.mb_w, bd = P.bd;
+    T* const grow = Pl + (size_t)(y * W + line) * stride;       // this lane's row
+    T* const gtop = Pl + ((ptrdiff_t)y * W - H + line) * stride;  // lanes line < H: a row above
+    const DbkEdges* const erow = edges + (size_t)y * mb_w;
+    const int maxv = (1 << bd) - 1, sh = 8 * (CHROMA ? line >> 1 : line >> 2);
+    const bool bottom = active && below && line >= W - H, above = active && y > 0 && line >= 1 && line < H;
+    const int rrow = (CHROMA ? comp * 16 : 0) + (line - (W - H)) * W;  // a bottom row's place in a ring slot
+    // macroblock x's samples and edge words into stage x % DBK_AHEAD
+    auto issue = [&](int x) {
+        if (x < mb_w) {
+            const int s = x % DBK_AHEAD;
+            if (active) {
+                const uint8_t* g = reinterpret_cast<const uint8_t*>(grow + x * W);
+                uint8_t* d = reinterpret_cast<uint8_t*>(G.own[j][s]) + ln * RB;
+                dbk_cp_async<(RB < 16 ? 8 : 16)>(d, g);
+                if constexpr (RB == 32) dbk_cp_async<16>(d + 16, g + 16);
+            } else if (lane < 22) {
+                dbk_cp_async<16>(reinterpret_cast<uint4*>(&G.e[j][s]) + (lane - 16), reinterpret_cast<const uint4*>(&erow[x]) + (lane - 16));
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int k = 0; k < DBK_AHEAD - 1; k++) issue(k);
+    int left[LEFT];
+#pragma unroll
+    for (int k = 0; k < LEFT; k++) left[k] = 0;
+    for (int x = 0; x < mb_w; x++) {
+        issue(x + DBK_AHEAD - 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(DBK_AHEAD - 1) : "memory");
+        __syncwarp();
+        const int s = x % DBK_AHEAD;
+        T* const own = G.own[j][s];
+        const DbkEdges& E = G.e[j][s];
+        uint32_t rw[NW];
+        dbk_words_ld<NW>(own + ln * W, rw);
+        // the words of the two directions: luma's four edges; chroma's two, of this lane's component
+        uint32_t vw[NE], hw[NE];
+        bool vany, hany, v0, top;
+        if constexpr (CHROMA) {
+            const uint4 a = *reinterpret_cast<const uint4*>(E.chroma[0]), b = *reinterpret_cast<const uint4*>(E.chroma[1]);
+            vany = (a.x | a.y | b.x | b.y) != 0, hany = (a.z | a.w | b.z | b.w) != 0;
+            v0 = (a.x | b.x) != 0, top = y > 0 && (a.z | b.z) != 0;
+            vw[0] = comp ? b.x : a.x, vw[1] = comp ? b.y : a.y, hw[0] = comp ? b.z : a.z, hw[1] = comp ? b.w : a.w;
+        } else {
+            dbk_words_ld<4>(E.luma[0], vw);
+            dbk_words_ld<4>(E.luma[1], hw);
+            vany = (vw[0] | vw[1] | vw[2] | vw[3]) != 0, hany = (hw[0] | hw[1] | hw[2] | hw[3]) != 0;
+            v0 = vw[0] != 0, top = y > 0 && hw[0] != 0;
+        }
+        uint32_t bq[8];
+        dbk_words_ld<8>(E.bs[0], bq);
+        int lv[LEFT + W];
+        DbkEdge ve[NE];
+        if (vany) {
+#pragma unroll
+            for (int k = 0; k < NE; k++) ve[k] = dbk_edge(vw[k], (int)((bq[CHROMA ? 2 * k : k] >> sh) & 0xff), bd);
+#pragma unroll
+            for (int k = 0; k < LEFT; k++) lv[k] = left[k];
+#pragma unroll
+            for (int k = 0; k < W; k++) lv[LEFT + k] = dbk_sample<T>(rw, k);
+            if (v0) {
+                // (x > 0: an outer edge at the picture's left has no word) the previous macroblock's last columns are final now
+                dbk_outer<CHROMA>(lv, ve, maxv);
+                if (active) dbk_store<T, LEFT>(grow + x * W - LEFT, lv);
+                if (bottom) dbk_store_shared<T, LEFT>(G.ring[j + 1][(x - 1) % N] + rrow + W - LEFT, lv);
+            }
+        }
+        __syncwarp();
+        // published as soon as the outer edge is done: the row below waits for no more than that
+        if (lane == 0) {
+            __threadfence_block();
+            st_shared(&G.prog[j + 1], (unsigned)x);
+            st_shared(&G.cons[j], (unsigned)x);
+        }
+        if (vany) {
+            dbk_inner<CHROMA>(lv, ve, maxv);
+#pragma unroll
+            for (int k = 0; k < NW; k++) {
+                constexpr int PER = 4 / (int)sizeof(T);
+                uint32_t w = (uint32_t)lv[LEFT + PER * k];
+#pragma unroll
+                for (int i = 1; i < PER; i++) w |= (uint32_t)lv[LEFT + PER * k + i] << (8 * (int)sizeof(T) * i);
+                rw[k] = w;
+            }
+        }
+        if (hany) {
+            if (vany) {
+                if (active) dbk_words_st<NW>(own + ln * W, rw);
+                __syncwarp();
+            }
+            T* const rg = G.ring[j][x % N] + (CHROMA ? comp * 16 : 0);
+            T* const ow = own + (CHROMA ? comp * 64 : 0);
+            DbkEdge he[NE];
+#pragma unroll
+            for (int k = 0; k < NE; k++) he[k] = dbk_edge(hw[k], (int)((bq[4 + (CHROMA ? 2 * k : k)] >> sh) & 0xff), bd);
+            int cv[H + W];
+#pragma unroll
+            for (int k = 0; k < W; k++) cv[H + k] = (int)ow[k * W + line];
+            if (top) {
+                if (!__all_sync(DBK_ALL, dbk_spin(P, G, &G.prog[j], (unsigned)(x + 1)))) return;
+#pragma unroll
+                for (int k = 0; k < H; k++) cv[k] = (int)rg[k * W + line];
+                dbk_outer<CHROMA>(cv, he, maxv);
+                if (active) {
+#pragma unroll
+                    for (int k = 1; k < H; k++) rg[k * W + line] = (T)cv[k];
+                }
+            }
+            dbk_inner<CHROMA>(cv, he, maxv);
+            if (active) {
+#pragma unroll
+                for (int k = 0; k < W; k++) ow[k * W + line] = (T)cv[H + k];
+            }
+            __syncwarp();
+            dbk_words_ld<NW>(own + ln * W, rw);
+            if (top && above) {
+                // the rows above, final in this macroblock's columns: the row above has applied the next one's left edge
+                uint32_t tw[NW];
+                dbk_words_ld<NW>(rg + line * W, tw);
+                dbk_words_st<NW>(gtop + x * W, tw);
+            }
+        }
+        if (active && (vany || hany)) dbk_words_st<NW>(grow + x * W, rw);
+        if (below) {
+            if (x >= N && !__all_sync(DBK_ALL, dbk_spin(P, G, &G.cons[j + 1], (unsigned)(x - N + 1)))) return;
+            if (bottom) dbk_words_st<NW>(G.ring[j + 1][x % N] + rrow, rw);
+        }
+#pragma unroll
+        for (int k = 0; k < LEFT; k++) left[k] = dbk_sample<T>(rw, W - LEFT + k);
+    }
+    __syncwarp();
+    if (lane == 0) {
+        __threadfence_block();
+        st_shared(&G.prog[j + 1], (unsigned)mb_w);
+        st_shared(&G.cons[j], (unsigned)mb_w);
+    }
+}
+
+// The group's fetch warp: the bottom rows of macroblock row y - 1 (another CTA's, published in `above`) into ring 0,
+// up to eight macroblocks at a time (a lane per macroblock and row), as far as they are published and the ring has room.
+template <class T, bool CHROMA>
+__device__ __forceinline__ void dbk_group_fetch(const DbkParams& P, DbkGroup<T>& G, int y, const unsigned* above) {
+    constexpr int W = CHROMA ? 8 : 16, H = CHROMA ? 2 : 4, NW = W * (int)sizeof(T) / 4;
+    constexpr unsigned N = DbkGroup<T>::RING;
+    const int lane = threadIdx.x & 31, r = lane & 3;
+    const T* const src = CHROMA ? reinterpret_cast<const T*>(P.planes[1 + (r >> 1)]) + (size_t)(y * W - H + (r & 1)) * P.cs
+                                : reinterpret_cast<const T*>(P.planes[0]) + (size_t)(y * W - H + r) * P.ys;
+    unsigned f = 0;
+    const unsigned n = (unsigned)P.mb_w;
+    for (unsigned i = 0; f < n; i++) {
+        // macroblocks the first row has already passed (their top edges are not filtered) need no fetching
+        const unsigned c = __shfl_sync(DBK_ALL, ld_acquire_cta(&G.cons[0]), 0);
+        f = max(f, c);
+        const unsigned p = __shfl_sync(DBK_ALL, ld_relaxed(above), 0);
+        const unsigned lim = min(p, c + N);
+        if (f < lim) {
             asm volatile("fence.acq_rel.gpu;" ::: "memory");
-            return true;
+            const unsigned k = min(lim - f, 8u), m = f + (unsigned)(lane >> 2);
+            if (m < f + k) {
+                const uint4* g = reinterpret_cast<const uint4*>(src + (size_t)m * W);
+                T* d = G.ring[0][m % N] + r * W;
+                if constexpr (NW == 2) {
+                    *reinterpret_cast<uint2*>(d) = __ldcg(reinterpret_cast<const uint2*>(g));
+                } else {
+#pragma unroll
+                    for (int q = 0; q < NW / 4; q++) reinterpret_cast<uint4*>(d)[q] = __ldcg(g + q);
+                }
+            }
+            __syncwarp();
+            f += k;
+            if (lane == 0) st_release_cta(&G.prog[0], f);
+            i = 0;
+            continue;
         }
         if ((i & 63) == 63) {
-            if (ld_acquire(P.err) & 1u) return false;
-            if (i >= P.wait_limit) {
-                atomicOr(P.err, 1u);
-                return false;
+            const bool gone = (ld_acquire(P.err) & 1u) || ld_acquire_cta(&G.stop);
+            if (__any_sync(DBK_ALL, gone) || i >= P.wait_limit) {
+                if (lane == 0) {
+                    atomicOr(P.err, 1u);
+                    st_release_cta(&G.stop, 1u);
+                }
+                return;
             }
         }
         if (i >= 16) __nanosleep(64);
     }
 }
 
-// Pass 2 for one macroblock row of one plane kind, left to right, by one warp. Luma: lanes 0-15 hold the
-// macroblock's 16 rows (each with the 4 samples to its left); chroma: lanes 0-7 the Cb rows, 8-15 the Cr
-// rows (each with 2 to the left); lanes 16-31 idle. The vertical edges are filtered in those registers,
-// the horizontal ones on columns read back from a shared-memory tile that also holds the rows above (4
-// luma / 2 chroma). The next macroblock's own samples and edge words are loaded while the current one
-// waits and filters. The vertical edges come first and need nothing from the row above; they make the
-// previous macroblock final (its last columns are the left edge's p side), so the warp stores those columns
-// and publishes progress x + 1 (macroblocks 0..x-1 final) before it waits for the row above, loads the rows
-// above and filters the horizontal edges.
-template <class T, bool CHROMA>
-__device__ __forceinline__ void dbk_row(const DbkParams& P, const DbkEdges* __restrict__ edges, int y, int (*L)[17],
-                                        DbkEdges& E) {
-    constexpr int W = CHROMA ? 8 : 16;   // samples of a macroblock row
-    constexpr int LEFT = CHROMA ? 2 : 4; // samples kept to its left
-    constexpr int H = CHROMA ? 2 : 4;    // rows above
+// The group's publishing warp: the last row's progress (nr rows in the group) for the group below, each time it moves.
+template <class T>
+__device__ __forceinline__ void dbk_group_publish(const DbkParams& P, DbkGroup<T>& G, int nr, unsigned* mine) {
     const int lane = threadIdx.x & 31;
-    const bool active = lane < 16;
-    const int comp = CHROMA ? lane >> 3 : 0, line = CHROMA ? lane & 7 : lane;
-    T* const Pl = reinterpret_cast<T*>(P.planes[CHROMA ? 1 + comp : 0]);
-    const int stride = CHROMA ? P.cs : P.ys;
-    // the tile: luma rows y0-4..y0+15 in L[0..19]; chroma comp c rows yc-2..yc+7 in L[10c .. 10c+9]
-    int (*Tl)[17] = CHROMA ? L + 10 * comp : L;
-    const size_t lrow = (size_t)(y * (CHROMA ? 8 : 16) + line) * stride;
-    const unsigned* above = P.progress + (CHROMA ? P.mb_h : 0) + (y - 1);
-    unsigned* mine = P.progress + (CHROMA ? P.mb_h : 0) + y;
-    const int maxv = (1 << P.bd) - 1;
-    int lv[LEFT + W];
-    int own[W];
-    uint32_t ew = 0;
-    auto prefetch = [&](int x) {
-        if (active) dbk_load_row<T, W>(Pl + lrow + x * W, own);
-        if (lane < 24) ew = __ldg(reinterpret_cast<const uint32_t*>(&edges[(size_t)y * P.mb_w + x]) + lane);
-    };
-    prefetch(0);
-    for (int x = 0; x < P.mb_w; x++) {
-        if (active) {
-#pragma unroll
-            for (int k = 0; k < W; k++) lv[LEFT + k] = own[k];
+    unsigned last = 0;
+    for (unsigned i = 0; last < (unsigned)P.mb_w; i++) {
+        const unsigned p = __shfl_sync(DBK_ALL, ld_acquire_cta(&G.prog[nr]), 0);
+        if (p > last) {
+            // the row's stores, seen by this warp through the shared word, before the device-scope release
+            asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            if (lane == 0) st_release(mine, p);
+            last = p;
+            i = 0;
+            continue;
         }
-        if (lane < 24) reinterpret_cast<uint32_t*>(&E)[lane] = ew;
-        __syncwarp();
-        // vertical edges, in registers: they touch this row of macroblocks only, so they need nothing
-        // from the row above
-        if (active) {
-            const uint32_t* words = CHROMA ? E.chroma[comp][0] : E.luma[0];
-            dbk_filter_lines<CHROMA, LEFT + W>(lv, words, E.bs[0], CHROMA ? line >> 1 : line >> 2, P.bd, maxv);
-            // the previous macroblock's last columns are final now: store them and publish it
-            if (x > 0) dbk_store<T, LEFT>(Pl + lrow + x * W - LEFT, lv);
-        }
-        __syncwarp();
-        if (lane == 0) st_release(mine, (unsigned)(x + 1));  // the warp's stores, ordered by the barrier above
-        // the next macroblock's samples and edge words (after the fence, which would wait for them)
-        if (x + 1 < P.mb_w) prefetch(x + 1);
-        // macroblocks 0..x+1 of the row above final (its last two macroblocks: the whole row, whose final
-        // publish is mb_w + 1)
-        const unsigned need = x + 2 < P.mb_w ? (unsigned)(x + 2) : (unsigned)P.mb_w + 1;
-        if (y > 0 && !__all_sync(DBK_ALL, dbk_wait(P, above, need))) return;
-        // the rows above, one lane each
-        if (y > 0 && lane < 4) {
-            const int cc = CHROMA ? lane >> 1 : 0, rr = CHROMA ? lane & 1 : lane;
-            const T* src = reinterpret_cast<const T*>(P.planes[CHROMA ? 1 + cc : 0]) + (size_t)(y * (CHROMA ? 8 : 16) - H + rr) * stride + x * W;
-            int r[W];
-            dbk_load_row<T, W>(src, r);
-            int (*dst)[17] = CHROMA ? L + 10 * cc : L;
-#pragma unroll
-            for (int k = 0; k < W; k++) dst[rr][k] = r[k];
-        }
-        if (active) {
-#pragma unroll
-            for (int k = 0; k < W; k++) Tl[H + line][k] = lv[LEFT + k];
-        }
-        __syncwarp();
-        if (active) {
-            // horizontal edges, a lane per column of the tile
-            int cv[H + W];
-#pragma unroll
-            for (int k = 0; k < H + W; k++) cv[k] = Tl[k][line];
-            const uint32_t* words = CHROMA ? E.chroma[comp][1] : E.luma[1];
-            dbk_filter_lines<CHROMA, H + W>(cv, words, E.bs[1], CHROMA ? line >> 1 : line >> 2, P.bd, maxv);
-#pragma unroll
-            for (int k = 1; k < H + W; k++) Tl[k][line] = cv[k];
-        }
-        __syncwarp();
-        if (active) {
-#pragma unroll
-            for (int k = 0; k < W; k++) lv[LEFT + k] = Tl[H + line][k];
-            dbk_store_row<T, W>(Pl + lrow + x * W, &lv[LEFT]);
-            if (y > 0 && line >= 1 && line < H) {
-                int r[W];
-#pragma unroll
-                for (int k = 0; k < W; k++) r[k] = Tl[line][k];
-                dbk_store_row<T, W>(Pl + (size_t)(y * (CHROMA ? 8 : 16) - H + line) * stride + x * W, r);
-            }
-            // this macroblock's last columns are the next one's left samples
-#pragma unroll
-            for (int k = 0; k < LEFT; k++) lv[k] = lv[W + k];
-        }
-        __syncwarp();
+        if ((i & 15) == 15 && (__any_sync(DBK_ALL, ld_acquire_cta(&G.stop) != 0) || i >= DBK_SPINS)) return;
+        __nanosleep(20);
     }
-    // the last macroblock's own rows were stored after the last publish: publish them too
-    __syncwarp();
-    if (lane == 0) st_release(mine, (unsigned)P.mb_w + 1);
 }
 
-// Pass 2: macroblock rows of the two plane kinds handed out by ticket (2y: luma row y, 2y + 1: chroma row y);
-// a row waits only on the row above of its own kind, which holds a smaller ticket.
+// One group of a picture by the whole CTA: local ticket lt = 2 * group + (1 for chroma).
 template <class T>
-__global__ void __launch_bounds__(DBK_WARPS * 32) deblock_rows_kernel(const __grid_constant__ DbkParams P,
-                                                                      const DbkEdges* __restrict__ edges) {
-    __shared__ int Ls[DBK_WARPS][20][17];
-    __shared__ DbkEdges Es[DBK_WARPS];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+__device__ __forceinline__ void dbk_group(const DbkParams& P, const DbkEdges* __restrict__ edges, DbkGroup<T>& G, unsigned lt) {
+    const int tid = threadIdx.x, w = tid >> 5;
+    const bool chroma = (lt & 1u) != 0;
+    const int y0 = (int)(lt >> 1) * DBK_ROWS, nr = min(DBK_ROWS, P.mb_h - y0);
+    if (tid <= DBK_ROWS) G.prog[tid] = 0;
+    if (tid < DBK_ROWS) G.cons[tid] = 0;
+    if (tid == 0) G.stop = 0;
+    __syncthreads();
+    unsigned* const words = P.progress + (chroma ? P.mb_h : 0);
+    if (w < DBK_ROWS) {
+        if (w < nr) {
+            if (chroma) dbk_group_row<T, true>(P, edges, G, w, y0 + w, w + 1 < nr);
+            else dbk_group_row<T, false>(P, edges, G, w, y0 + w, w + 1 < nr);
+            asm volatile("cp.async.wait_all;" ::: "memory");  // none left in flight, also where a wait gave up
+        }
+    } else if (w == DBK_ROWS) {
+        if (y0 > 0) {
+            if (chroma) dbk_group_fetch<T, true>(P, G, y0, words + y0 - 1);
+            else dbk_group_fetch<T, false>(P, G, y0, words + y0 - 1);
+        }
+    } else if (y0 + nr < P.mb_h) {
+        dbk_group_publish<T>(P, G, nr, words + y0 + nr - 1);
+    }
+    __syncthreads();
+}
+
+__host__ __device__ constexpr int dbk_groups(int mb_h) { return (mb_h + DBK_ROWS - 1) / DBK_ROWS; }
+
+// Pass 2: the groups of the two plane kinds handed out by ticket; a group waits only on the group above of
+// its own kind, which holds a smaller ticket.
+template <class T>
+__global__ void __launch_bounds__(DBK_GROUP_THREADS, 2) deblock_rows_kernel(const __grid_constant__ DbkParams P,
+                                                                            const DbkEdges* __restrict__ edges) {
+    __shared__ DbkGroup<T> G;
     for (;;) {
-        unsigned t = 0;
-        if (lane == 0) t = atomicAdd(P.ticket, 1u);
-        t = __shfl_sync(DBK_ALL, t, 0);
-        if (t >= 2u * (unsigned)P.mb_h) return;
-        if (t & 1u) dbk_row<T, true>(P, edges, (int)(t >> 1), Ls[wid], Es[wid]);
-        else dbk_row<T, false>(P, edges, (int)(t >> 1), Ls[wid], Es[wid]);
-        if (ld_acquire(P.err) & 1u) return;
+        if (threadIdx.x == 0) G.ticket = atomicAdd(P.ticket, 1u);
+        __syncthreads();
+        const unsigned t = G.ticket;
+        if (t >= 2u * (unsigned)dbk_groups(P.mb_h)) return;
+        dbk_group<T>(P, edges, G, t);
+        if (__syncthreads_or((int)(ld_acquire(P.err) & 1u))) return;
     }
 }
 
@@ -507,27 +692,29 @@ static __global__ void __launch_bounds__(DBK_WARPS * 32) deblock_edges_batch_ker
     }
 }
 
-// Pass 2 for every stream: ticket t is order[t] = stream << 20 | the stream's own row ticket (2y luma row y,
-// 2y + 1 chroma row y), the streams' rows interleaved by their own tickets, so a row waits only on its own
-// stream's row above, which holds a smaller ticket.
+// Pass 2 for every stream: ticket t is order[t] = stream << 20 | the stream's own group ticket (dbk_group), the
+// streams' groups interleaved by their own tickets, so a group waits only on its own stream's group above, which
+// holds a smaller ticket.
 template <class T>
-__global__ void __launch_bounds__(DBK_WARPS * 32) deblock_rows_batch_kernel(const DbkJob* __restrict__ jobs,
-                                                                                   const uint32_t* __restrict__ order, unsigned ntickets,
-                                                                                   unsigned* ticket, const unsigned* err) {
-    __shared__ int Ls[DBK_WARPS][20][17];
-    __shared__ DbkEdges Es[DBK_WARPS];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+__global__ void __launch_bounds__(DBK_GROUP_THREADS, 2) deblock_rows_batch_kernel(const DbkJob* __restrict__ jobs,
+                                                                                  const uint32_t* __restrict__ order, unsigned ntickets,
+                                                                                  unsigned* ticket, const unsigned* err) {
+    __shared__ DbkGroup<T> G;
+    __shared__ DbkParams P;
+    __shared__ const DbkEdges* edges;
     for (;;) {
-        unsigned t = 0;
-        if (lane == 0) t = atomicAdd(ticket, 1u);
-        t = __shfl_sync(DBK_ALL, t, 0);
-        if (t >= ntickets) return;
-        const uint32_t e = order[t];
-        const DbkJob& J = jobs[e >> 20];
-        const unsigned lt = e & 0xFFFFFu;
-        if (lt & 1u) dbk_row<T, true>(J.P, J.edges, (int)(lt >> 1), Ls[wid], Es[wid]);
-        else dbk_row<T, false>(J.P, J.edges, (int)(lt >> 1), Ls[wid], Es[wid]);
-        if (ld_acquire(err) & 1u) return;
+        if (threadIdx.x == 0) {
+            G.ticket = atomicAdd(ticket, 1u);
+            if (G.ticket < ntickets) {
+                const DbkJob& J = jobs[order[G.ticket] >> 20];
+                P = J.P;
+                edges = J.edges;
+            }
+        }
+        __syncthreads();
+        if (G.ticket >= ntickets) return;
+        dbk_group<T>(P, edges, G, order[G.ticket] & 0xFFFFFu);
+        if (__syncthreads_or((int)(ld_acquire(err) & 1u))) return;
     }
 }
 

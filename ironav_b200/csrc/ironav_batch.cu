@@ -189,13 +189,14 @@ struct ironav_batch {
     int nchains = 0, nchains3 = 0;  // the first nchains3 (the longest bands) on three warps each
     cudaStream_t aux = nullptr;     // the one-warp launch runs beside the three-warp one
     cudaEvent_t fork = nullptr, join = nullptr;
-    // deblocking (allocated on first use): the streams' jobs, their rows' merged ticket order, progress
+    // deblocking (allocated on first use): the streams' jobs, their row groups' merged ticket order, progress
     // words, and the concatenated slice tables (pinned staging reused once the previous copies are done)
     DbkJob* d_kjobs = nullptr;
     DbkJob* h_kjobs = nullptr;
     uint32_t* d_korder = nullptr;
     unsigned* d_kprogress = nullptr;
-    int total_rows2 = 0;  // sum of 2 * mb_h
+    int total_rows2 = 0;  // sum of 2 * mb_h (progress words)
+    int total_groups2 = 0;  // sum of 2 * dbk_groups(mb_h) (tickets)
     ironav_dbk_slice* d_kslices = nullptr;
     ironav_dbk_slice* h_kslices = nullptr;
     int kslice_cap = 0;
@@ -687,17 +688,20 @@ extern "C" int ironav_batch_deblock(ironav_batch* b, void* const* d_y, const int
     if (!b->d_kjobs) {
         CK(cudaMalloc(&b->d_kjobs, sizeof(DbkJob) * b->n));
         CK(cudaHostAlloc(&b->h_kjobs, sizeof(DbkJob) * b->n, cudaHostAllocDefault));
-        // every stream's row tickets merged by the stream's own ticket, then stream
+        // every stream's group tickets merged by the stream's own ticket, then stream
         std::vector<std::pair<int, int>> keys;
-        for (int i = 0; i < b->n; i++)
-            for (int t = 0; t < 2 * b->ctx[i]->mb_h; t++) keys.emplace_back(t, i);
+        b->total_rows2 = 0;
+        for (int i = 0; i < b->n; i++) {
+            b->total_rows2 += 2 * b->ctx[i]->mb_h;
+            for (int t = 0; t < 2 * dbk_groups(b->ctx[i]->mb_h); t++) keys.emplace_back(t, i);
+        }
         std::sort(keys.begin(), keys.end());
         std::vector<uint32_t> order(keys.size());
         for (size_t k = 0; k < keys.size(); k++) order[k] = ((uint32_t)keys[k].second << 20) | (uint32_t)keys[k].first;
-        b->total_rows2 = (int)order.size();
+        b->total_groups2 = (int)order.size();
         CK(cudaMalloc(&b->d_korder, sizeof(uint32_t) * order.size()));
         CK(cudaMemcpy(b->d_korder, order.data(), sizeof(uint32_t) * order.size(), cudaMemcpyHostToDevice));
-        CK(cudaMalloc(&b->d_kprogress, sizeof(unsigned) * order.size()));
+        CK(cudaMalloc(&b->d_kprogress, sizeof(unsigned) * b->total_rows2));
         for (int i = 0; i < b->n; i++)
             if (!b->ctx[i]->d_dbk_edges) CK(cudaMalloc(&b->ctx[i]->d_dbk_edges, sizeof(DbkEdges) * b->ctx[i]->nmb));
     }
@@ -751,12 +755,12 @@ extern "C" int ironav_batch_deblock(ironav_batch* b, void* const* d_y, const int
     const int nsm = b->ctx[0]->nsm;
     deblock_edges_batch_kernel<<<std::min((b->total_mbs + DBK_WARPS - 1) / DBK_WARPS, nsm * 16), DBK_WARPS * 32, 0, b->stream>>>(
         b->d_kjobs, b->n, b->total_mbs);
-    const int rblocks = std::min((b->total_rows2 + DBK_WARPS - 1) / DBK_WARPS, nsm * 16);
+    const int rblocks = std::min(b->total_groups2, nsm * 2);
     if (b->bd > 8)
-        deblock_rows_batch_kernel<uint16_t><<<rblocks, DBK_WARPS * 32, 0, b->stream>>>(b->d_kjobs, b->d_korder, (unsigned)b->total_rows2,
-                                                                                       b->d_counters, b->d_counters + 1);
+        deblock_rows_batch_kernel<uint16_t><<<rblocks, DBK_GROUP_THREADS, 0, b->stream>>>(b->d_kjobs, b->d_korder, (unsigned)b->total_groups2,
+                                                                                         b->d_counters, b->d_counters + 1);
     else
-        deblock_rows_batch_kernel<uint8_t><<<rblocks, DBK_WARPS * 32, 0, b->stream>>>(b->d_kjobs, b->d_korder, (unsigned)b->total_rows2,
-                                                                                      b->d_counters, b->d_counters + 1);
+        deblock_rows_batch_kernel<uint8_t><<<rblocks, DBK_GROUP_THREADS, 0, b->stream>>>(b->d_kjobs, b->d_korder, (unsigned)b->total_groups2,
+                                                                                        b->d_counters, b->d_counters + 1);
     return cuda_status(cudaGetLastError());
 }

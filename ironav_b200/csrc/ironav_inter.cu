@@ -300,9 +300,9 @@ int deblock_launch(ironav_ctx* c, void* d_y, int ys, void* d_cb, void* d_cr, int
     DbkEdges* edges = static_cast<DbkEdges*>(c->d_dbk_edges);
     const int eblocks = std::min((c->nmb + DBK_WARPS - 1) / DBK_WARPS, c->nsm * 16);
     deblock_edges_kernel<<<eblocks, DBK_WARPS * 32, 0, c->stream>>>(p, edges);
-    const int blocks = (2 * c->mb_h + DBK_WARPS - 1) / DBK_WARPS;
-    if (c->bd > 8) deblock_rows_kernel<uint16_t><<<blocks, DBK_WARPS * 32, 0, c->stream>>>(p, edges);
-    else deblock_rows_kernel<uint8_t><<<blocks, DBK_WARPS * 32, 0, c->stream>>>(p, edges);
+    const int blocks = 2 * dbk_groups(c->mb_h);
+    if (c->bd > 8) deblock_rows_kernel<uint16_t><<<blocks, DBK_GROUP_THREADS, 0, c->stream>>>(p, edges);
+    else deblock_rows_kernel<uint8_t><<<blocks, DBK_GROUP_THREADS, 0, c->stream>>>(p, edges);
     return cuda_status(cudaGetLastError());
 }
 
