@@ -51,22 +51,29 @@ EncodeTiled encode_fn() {
     return fn;
 }
 
-// The tensor map of a chunk-major padded tensor (planes x Q pixels x 8 BF16) read in boxes of `box_pixels`
-// pixels of `box_planes` planes (0: every plane): dims (8, Q, planes), byte strides (16, 16 Q). Out-of-range
-// pixels read as zeros.
-int plane_map(CUtensorMap* map, const void* base, long long Q, int planes, int box_pixels, int box_planes = 0) {
+// The tensor map of `pixels` pixels of a chunk-major padded tensor (planes of Q pixels x 8 BF16) from `base`, read in
+// boxes of BOX_PIXELS pixels of `box_planes` planes. A plane's pixels are one run of 16-byte pieces, so the map calls
+// it a row of 64-bit elements, two a pixel: dims (2 * pixels, planes), byte stride 16 Q, and a box moves rows of 2 KB.
+// (With the 8 channels as the innermost dimension a box moved rows of 16 bytes, a piece a clock: 512 samples' weight
+// gradient of 32 channels took 199 us, and with this map and the pipeline around it 79 us; the convolution 631 -> 583 us at 8160.) Out-of-range pixels read as zeros.
+int plane_map(CUtensorMap* map, const void* base, long long Q, long long pixels, int planes, int box_planes) {
     EncodeTiled enc = encode_fn();
     if (!enc) return IRONAV_HARDWARE_UNAVAILABLE;
     if (reinterpret_cast<uintptr_t>(base) & 15) return IRONAV_INVALID_ARGUMENT;
-    const cuuint64_t dims[3] = {8, (cuuint64_t)Q, (cuuint64_t)planes};
-    const cuuint64_t strides[2] = {16, (cuuint64_t)Q * 16};
-    const cuuint32_t box[3] = {8, (cuuint32_t)box_pixels, (cuuint32_t)(box_planes > 0 ? box_planes : planes)};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+    const cuuint64_t dims[2] = {(cuuint64_t)pixels * 2, (cuuint64_t)planes};
+    const cuuint64_t strides[1] = {(cuuint64_t)Q * 16};
+    const cuuint32_t box[2] = {2 * BOX_PIXELS, (cuuint32_t)box_planes};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_INT64, 2, const_cast<void*>(base), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? IRONAV_OK : IRONAV_INVALID_ARGUMENT;
 }
+
+// Samples a launch takes: a box's first element (two a pixel) is a 32-bit coordinate, so a larger batch goes in several launches.
+// A sample's interior pixels depend on its own raster only, so a batch may be cut between any two samples.
+constexpr long long LAUNCH_SAMPLES = 400000;
+static_assert(LAUNCH_SAMPLES * RPIX * 2 < (1ll << 31), "box coordinates fit 32 bits");
 
 int sm_count(int* nsm) {
     int dev = 0;
@@ -81,60 +88,67 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 
 extern "C" {
 
-// The convolution's tile: CONV_MT x 128 output pixels (conv3x3p_kernel's MT).
-constexpr int CONV_MT = 2;
-
 int ironav_prop_conv3x3(const void* d_x, int cin, long long samples, const void* d_w, const float* d_bias, int relu, const void* d_mask,
                         void* d_y, unsigned* d_err, void* stream) {
     if (!d_x || !d_w || !d_y || !d_err || (cin != 16 && cin != 32) || samples < 1 || samples > (1ll << 22)) return IRONAV_INVALID_ARGUMENT;
     if (!aligned16(d_y) || !aligned16(d_mask)) return IRONAV_INVALID_ARGUMENT;
     const long long Q = samples * RPIX;
-    const int tiles = (int)((Q + CONV_MT * TILE - 1) / (CONV_MT * TILE));
-    CUtensorMap map;
-    int s = plane_map(&map, d_x, Q, cin / 8, cp_box<CONV_MT>(), CONV_MT == 1 ? 0 : 1);
-    if (s != IRONAV_OK) return s;
     int nsm = 0;
-    if ((s = sm_count(&nsm)) != IRONAV_OK) return s;
-    // the pipelined form: two persistent CTAs an SM
-    const int grid = std::min(tiles, nsm * 2);
+    int s = sm_count(&nsm);
+    if (s != IRONAV_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(d_w);
-    const __nv_bfloat16* mask = static_cast<const __nv_bfloat16*>(d_mask);
-    __nv_bfloat16* y = static_cast<__nv_bfloat16*>(d_y);
-    if (cin == 32) {
-        constexpr int bytes = conv3x3p_smem_bytes<32, CONV_MT>();
-        CK(cudaFuncSetAttribute(conv3x3p_kernel<32, CONV_MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        conv3x3p_kernel<32, CONV_MT><<<grid, CP_THREADS, bytes, st>>>(map, w, d_bias, relu, mask, y, Q, tiles, d_err);
-    } else {
-        constexpr int bytes = conv3x3p_smem_bytes<16, CONV_MT>();
-        CK(cudaFuncSetAttribute(conv3x3p_kernel<16, CONV_MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        conv3x3p_kernel<16, CONV_MT><<<grid, CP_THREADS, bytes, st>>>(map, w, d_bias, relu, mask, y, Q, tiles, d_err);
+    for (long long s0 = 0; s0 < samples; s0 += LAUNCH_SAMPLES) {
+        const long long q0 = s0 * RPIX, pixels = std::min(samples - s0, LAUNCH_SAMPLES) * RPIX;
+        const int tiles = (int)((pixels + CP_PIXELS - 1) / CP_PIXELS);
+        CUtensorMap map;
+        if ((s = plane_map(&map, static_cast<const uint8_t*>(d_x) + q0 * 16, Q, pixels, cin / 8, 1)) != IRONAV_OK) return s;
+        // two persistent CTAs an SM
+        const int grid = std::min(tiles, nsm * 2);
+        const __nv_bfloat16* mask = d_mask ? static_cast<const __nv_bfloat16*>(d_mask) + q0 * 8 : nullptr;
+        __nv_bfloat16* y = static_cast<__nv_bfloat16*>(d_y) + q0 * 8;
+        if (cin == 32) {
+            constexpr int bytes = conv3x3p_smem_bytes<32>();
+            CK(cudaFuncSetAttribute(conv3x3p_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+            conv3x3p_kernel<32><<<grid, CP_THREADS, bytes, st>>>(map, w, d_bias, relu, mask, y, Q, pixels, tiles, d_err);
+        } else {
+            constexpr int bytes = conv3x3p_smem_bytes<16>();
+            CK(cudaFuncSetAttribute(conv3x3p_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+            conv3x3p_kernel<16><<<grid, CP_THREADS, bytes, st>>>(map, w, d_bias, relu, mask, y, Q, pixels, tiles, d_err);
+        }
+        CK(cudaGetLastError());
     }
-    return cuda_status(cudaGetLastError());
+    return IRONAV_OK;
 }
 
 int ironav_prop_wgrad3x3(const void* d_x, int cin, const void* d_dz, long long samples, float* d_dw, float* d_db, unsigned* d_err,
                          void* stream) {
     if (!d_x || !d_dz || !d_dw || !d_err || (cin != 16 && cin != 32) || samples < 1 || samples > (1ll << 22)) return IRONAV_INVALID_ARGUMENT;
     const long long Q = samples * RPIX;
-    const int tiles = (int)((Q + WG_KT - 1) / WG_KT);
-    CUtensorMap xmap, zmap;
-    int s = plane_map(&xmap, d_x, Q, cin / 8, WG_KT);
-    if (s == IRONAV_OK) s = plane_map(&zmap, d_dz, Q, 4, WG_KT);
-    if (s != IRONAV_OK) return s;
     int nsm = 0;
-    if ((s = sm_count(&nsm)) != IRONAV_OK) return s;
+    int s = sm_count(&nsm);
+    if (s != IRONAV_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (cin == 32) {
-        constexpr int bytes = wgrad3x3_smem_bytes<32>();
-        CK(cudaFuncSetAttribute(wgrad3x3_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        wgrad3x3_kernel<32><<<std::min(tiles, nsm * 2), 128, bytes, st>>>(xmap, zmap, d_dw, d_db, Q, tiles, d_err);
-    } else {
-        constexpr int bytes = wgrad3x3_smem_bytes<16>();
-        CK(cudaFuncSetAttribute(wgrad3x3_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-        wgrad3x3_kernel<16><<<std::min(tiles, nsm * 2), 128, bytes, st>>>(xmap, zmap, d_dw, d_db, Q, tiles, d_err);
+    for (long long s0 = 0; s0 < samples; s0 += LAUNCH_SAMPLES) {
+        const long long q0 = s0 * RPIX, pixels = std::min(samples - s0, LAUNCH_SAMPLES) * RPIX;
+        const int tiles = (int)((pixels + WG_KT - 1) / WG_KT);
+        CUtensorMap xmap, zmap;
+        s = plane_map(&xmap, static_cast<const uint8_t*>(d_x) + q0 * 16, Q, pixels, cin / 8, cin / 8);
+        if (s == IRONAV_OK) s = plane_map(&zmap, static_cast<const uint8_t*>(d_dz) + q0 * 16, Q, pixels, 4, 4);
+        if (s != IRONAV_OK) return s;
+        const int grid = std::min(tiles, nsm);
+        if (cin == 32) {
+            constexpr int bytes = wgrad3x3_smem_bytes<32>();
+            CK(cudaFuncSetAttribute(wgrad3x3_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+            wgrad3x3_kernel<32><<<grid, WG_THREADS, bytes, st>>>(xmap, zmap, d_dw, d_db, tiles, d_err);
+        } else {
+            constexpr int bytes = wgrad3x3_smem_bytes<16>();
+            CK(cudaFuncSetAttribute(wgrad3x3_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+            wgrad3x3_kernel<16><<<grid, WG_THREADS, bytes, st>>>(xmap, zmap, d_dw, d_db, tiles, d_err);
+        }
+        CK(cudaGetLastError());
     }
-    return cuda_status(cudaGetLastError());
+    return IRONAV_OK;
 }
 
 int ironav_prop_prep(const ironav_prop_sample* d_samples, int n, void* d_x, void* stream) {
@@ -162,9 +176,15 @@ int ironav_prop_head_fwd_packed(const void* d_feat, int n, const float* d_hwt, c
     if (!d_feat || !d_hwt || !d_hb || !d_out || n < 1 || n > (1 << 22) || !aligned16(d_hwt)) return IRONAV_INVALID_ARGUMENT;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     CK(cudaMemsetAsync(d_out, 0, (size_t)n * prop::NOUT * sizeof(float), st));
-    const dim3 grid((n + prop::HEAD_SAMPLES - 1) / prop::HEAD_SAMPLES, (48 * 48 + prop::HEAD_PIX - 1) / prop::HEAD_PIX);
-    prop::head_fwd_packed_kernel<<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(d_feat), (long long)n * RPIX, n,
-                                                       reinterpret_cast<const float4*>(d_hwt), d_hb, d_out);
+    int nsm = 0;
+    const int r = sm_count(&nsm);
+    if (r != IRONAV_OK) return r;
+    // pixels a CTA: as few as give two waves of CTAs (one an SM), in whole chunks; at most 128, which the sums over a
+    // picture's samples (two waves already) are fastest with
+    const int sg = (n + prop::HEAD_SAMPLES - 1) / prop::HEAD_SAMPLES, slices = std::max(1, std::min(144, 2 * nsm / sg));
+    const int pix = std::min(128, (2304 / prop::HEAD_CHUNK + slices - 1) / slices * prop::HEAD_CHUNK);
+    prop::head_fwd_packed_kernel<<<dim3(sg, (2304 + pix - 1) / pix), 256, 0, st>>>(static_cast<const __nv_bfloat16*>(d_feat), (long long)n * RPIX, n,
+                                                                                    reinterpret_cast<const float4*>(d_hwt), d_hb, d_out, pix);
     return cuda_status(cudaGetLastError());
 }
 
@@ -181,11 +201,9 @@ int ironav_prop_head_bwd(const void* d_feat, int n, const float* d_dout, const f
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long Q = (long long)n * RPIX;
     const __nv_bfloat16* feat = static_cast<const __nv_bfloat16*>(d_feat);
-    // the ring of dz is zero (its interior is written below)
-    CK(cudaMemsetAsync(d_dz, 0, (size_t)4 * Q * 16, st));
-    prop::head_wgrad_kernel<<<(prop::NFEAT + 255) / 256, 256, 0, st>>>(feat, Q, n, d_dout, d_ghw, d_ghb);
-    const long long total = (long long)n * prop::NFEAT;
-    prop::head_dgrad_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(feat, Q, n, d_dout, d_hw, static_cast<__nv_bfloat16*>(d_dz));
+    prop::head_wgrad_kernel<<<4 * 2304 / 32, 256, 0, st>>>(feat, Q, n, d_dout, d_ghw, d_ghb);
+    const dim3 grid((n + prop::HB_SLICE - 1) / prop::HB_SLICE, (4 * RPIX + prop::HB_UNITS - 1) / prop::HB_UNITS);
+    prop::head_dgrad_kernel<<<grid, prop::HB_UNITS, 0, st>>>(feat, Q, n, d_dout, d_hw, static_cast<__nv_bfloat16*>(d_dz));
     return cuda_status(cudaGetLastError());
 }
 

@@ -8,12 +8,12 @@
 // the nine shifts (dy - 1) * 50 + (dx - 1): output pixel q reads input pixel q + shift, and a shift never leaves
 // the sample's own raster for an interior pixel (outputs on the ring are written as zeros).
 //
-// A CTA takes tiles of 128 consecutive output pixels. Per tile: one TMA 3-D box load brings the input halo
-// (pixels q0 - 51 .. q0 + 180 of every plane, zeros beyond the tensor) into shared memory in the same layout;
+// A CTA takes tiles of 256 consecutive output pixels. Per tile: TMA box loads bring the input halo (pixels
+// q0 - 51 .. q0 + 332 of every plane, zeros beyond the tensor) into shared memory in the same layout;
 // every tap's A operand (128 pixels x 16 channels, K-major, no swizzle) is then just another start address into
 // the halo, so no im2col copy is made. The weights (B: 32 output channels x CIN input channels per tap, K-major)
-// sit in shared memory for the CTA's life. One thread issues 9 taps x CIN / 16 MMAs of M = 128, N = 32, K = 16
-// into a TMEM accumulator (128 lanes x 32 FP32 columns); the epilogue warps read their 32 lanes (pixels) x 32
+// sit in shared memory for the CTA's life. One thread issues 2 x 9 taps x CIN / 16 MMAs of M = 128, N = 32, K = 16
+// into a TMEM accumulator (128 lanes x 2 x 32 FP32 columns); the epilogue warps read their 32 lanes (pixels) x 32
 // columns (channels) back with tcgen05.ld, add the bias, apply ReLU or a gradient mask, zero the ring, and
 // store BF16. Loads, MMAs and epilogues of successive tiles overlap (conv3x3p_kernel, below).
 //
@@ -31,7 +31,7 @@ constexpr int RW = 50;                  // raster width (and height): 48 + 2
 constexpr int RPIX = RW * RW;           // pixels a sample
 constexpr int TILE = 128;               // output pixels a tile (the MMA's M)
 constexpr int HALO_LO = RW + 1;         // the most negative shift
-constexpr int HALO = 232;               // halo pixels staged a tile: 51 + 128 + 51, rounded up to 8
+constexpr int BOX_PIXELS = 128;         // pixels a TMA box (256 64-bit elements, the limit of a box's side)
 constexpr int COUT = 32;                // output channels (the MMA's N)
 constexpr unsigned WAIT_LIMIT = 1u << 26;  // polls of an mbarrier before the kernel gives up
 
@@ -60,11 +60,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
     return false;
 }
 
-// TMA: a 3-D box of the tensor map into shared memory, completion counted on the mbarrier.
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+// TMA: a box of the tensor map (BOX_PIXELS pixels from pixel q, planes from c) into shared memory, completion counted on
+// the mbarrier. The map's elements are half pixels, so any pixel is a 16-byte boundary.
+__device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int q, int c, uint64_t* bar) {
     asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(2 * q), "r"(c), "r"(smem_u32(bar))
         : "memory");
 }
 
@@ -77,12 +78,17 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 // The instruction descriptor of kind::f16 with BF16 A and B, FP32 D, both K-major, M = 128, N = 32.
 constexpr uint32_t IDESC_BF16_M128_N32 = (1u << 4) | (1u << 7) | (1u << 10) | ((COUT >> 3) << 17) | ((TILE >> 4) << 24);
 
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// One MMA, issued by the lane whose `issuer` is set. The whole warp walks the issuing loop, so that the descriptors are
+// warp-uniform values: a loop under a one-lane branch moved every operand of every MMA to the uniform registers on its
+// own, and the issue bound the kernel (8160 samples, 32 and 16 input channels: 583
+// and 420 us, now 553 and 346; shared-memory reads of A, 4 KB for 32 columns of output, bound it now).
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t issuer) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+        "setp.ne.b32 q, %9, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(issuer));
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -113,45 +119,70 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 // tile of KT pixels, TMA stages the nine tap-shifted views of x ([tap slot][plane][pixel][16 B], taps beyond
 // 8 stay zero) and the tile of dz; one thread issues groups x KT / 16 MMAs into one TMEM accumulator per group
 // (32 columns each), accumulating over all the CTA's tiles; at the end each warp reads its 32 rows and adds them
-// to dw. xmap: x as (8, Q, CIN / 8) with boxes of KT pixels; zmap: dz as (8, Q, 4) with the same boxes.
-constexpr int WG_KT = 128;  // pixels a tile (K)
+// to dw. xmap: x with boxes of KT pixels of every plane; zmap: dz with boxes of KT pixels of its 4 planes.
+//
+// One CTA an SM, warp-specialised: warp 4 streams tiles into a ring of two stages, warp 5 issues their MMAs, warps 0-3 sum
+// the bias gradient from the staged dz; a stage is refilled once its MMAs (tcgen05.commit) and the four warps have
+// done with it. The waits are bounded as conv3x3p_kernel's: a role that gives up sets the CTA's failure flag, every other
+// role stops at its next wait, and the copies and MMAs still in flight are waited for (bounded) before the TMEM is freed.
+// 512 samples of 32 channels: 199 us with two CTAs an SM that each loaded, computed and summed one tile after another
+// (and copies of 16-byte rows), now 79.
+constexpr int WG_KT = BOX_PIXELS;  // pixels a tile (K)
+constexpr int WG_STAGES = 2;
+constexpr int WG_THREADS = 192;
 
 template <int CIN>
+__host__ __device__ constexpr int wgrad3x3_stage_bytes() {
+    return ((9 + 128 / CIN - 1) / (128 / CIN)) * 128 * WG_KT * 2 + 4 * WG_KT * 16;
+}
+template <int CIN>
 constexpr int wgrad3x3_smem_bytes() {
-    return ((9 + 128 / CIN - 1) / (128 / CIN)) * 128 * WG_KT * 2 + 4 * WG_KT * 16 + 2 * 8 + 16 + 32 * 4;
+    return WG_STAGES * wgrad3x3_stage_bytes<CIN>() + (2 * WG_STAGES + 1) * 8 + 16 + 32 * 4;
 }
 
 // MN-major operands for the weight gradient: M (or N) 8 channels of a pixel contiguous, K = pixels 16 bytes apart.
 constexpr uint32_t IDESC_BF16_MN_M128_N32 = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((COUT >> 3) << 17) | ((TILE >> 4) << 24);
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 template <int CIN>
-__global__ void __launch_bounds__(128, 1) wgrad3x3_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap zmap,
-                                                          float* __restrict__ dw, float* __restrict__ db, long long Q, int tiles,
-                                                          unsigned* err) {
+__global__ void __launch_bounds__(WG_THREADS, 1) wgrad3x3_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap zmap,
+                                                                 float* __restrict__ dw, float* __restrict__ db, int tiles, unsigned* err) {
     constexpr int KC = CIN / 8, TPG = 128 / CIN, NG = (9 + TPG - 1) / TPG;
     constexpr int PLANE = WG_KT * 16;          // bytes of one plane's tile
     constexpr int ABYTES = NG * 16 * PLANE;    // NG groups x 16 planes (TPG taps x KC planes)
-    constexpr int BBYTES = 4 * PLANE;
-    constexpr unsigned TX = 9 * KC * PLANE + BBYTES;
+    constexpr int SBYTES = wgrad3x3_stage_bytes<CIN>();
+    constexpr unsigned TX = (9 * KC + 4) * PLANE;
     constexpr int NCOL = NG * 32 <= 32 ? 32 : (NG * 32 <= 64 ? 64 : 128);
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* as = smem;
-    uint8_t* bs = smem + ABYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + ABYTES + BBYTES);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + WG_STAGES * SBYTES);  // [WG_STAGES]
+    uint64_t* empty = full + WG_STAGES;                                       // [WG_STAGES]: the MMAs and warps 0-3
+    uint64_t* done = empty + WG_STAGES;                                       // every MMA of the CTA
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+    volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* dbs = reinterpret_cast<float*>(tmem_slot + 4);
+    __shared__ int s_loaded, s_issued;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ntiles = tiles > (int)blockIdx.x ? (tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;  // this CTA's tiles
     // the slots of taps 9.. stay zero (their rows accumulate nothing)
-    for (int i = tid; i < (NG * TPG - 9) * KC * PLANE / 16; i += 128)
-        reinterpret_cast<uint4*>(as + 9 * KC * PLANE)[i] = make_uint4(0, 0, 0, 0);
+    for (int s = 0; s < WG_STAGES; s++)
+        for (int i = tid; i < (NG * TPG - 9) * KC * PLANE / 16; i += WG_THREADS)
+            reinterpret_cast<uint4*>(smem + s * SBYTES + 9 * KC * PLANE)[i] = make_uint4(0, 0, 0, 0);
     if (tid < 32) dbs[tid] = 0.f;
     if (tid == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+        for (int s = 0; s < WG_STAGES; s++) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 5);
+        }
+        mbar_init(done, 1);
+        *failed = 0;
+        s_loaded = s_issued = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (warp == 0) {
+    if (warp == 5) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(NCOL));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
@@ -159,58 +190,80 @@ __global__ void __launch_bounds__(128, 1) wgrad3x3_kernel(const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    bool failed = false, load_pending = false, mma_pending = false, any = false;
-    unsigned it = 0;
-    float dbsum = 0.f;  // this thread's share of db: channel lane, pixels warp, warp + 4, ...
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, it++) {
-        const long long q0 = (long long)tile * WG_KT;
-        if (tid == 0) {
-            mbar_expect_tx(&bars[0], TX);
-            for (int t = 0; t < 9; t++) {
-                const int shift = (t / 3 - 1) * RW + (t % 3 - 1);
-                tma_load_3d(as + (t / TPG) * 16 * PLANE + (t % TPG) * KC * PLANE, &xmap, 0, (int)(q0 + shift), 0, &bars[0]);
+    float dbsum = 0.f;  // warps 0-3: this thread's share of db: channel lane, pixels warp, warp + 4, ...
+    if (warp == 4) {
+        if (lane == 0) {
+            int loaded = 0;
+            for (int it = 0; it < ntiles; it++) {
+                const int s = it % WG_STAGES, k = it / WG_STAGES;
+                if (k > 0 && !mbar_wait(&empty[s], (k - 1) & 1)) {
+                    *failed = 1;
+                    break;
+                }
+                if (*failed) break;
+                const int q0 = ((int)blockIdx.x + it * (int)gridDim.x) * WG_KT;
+                uint8_t* as = smem + s * SBYTES;
+                mbar_expect_tx(&full[s], TX);
+                for (int t = 0; t < 9; t++)
+                    tma_load(as + (t / TPG) * 16 * PLANE + (t % TPG) * KC * PLANE, &xmap, q0 + (t / 3 - 1) * RW + (t % 3 - 1), 0, &full[s]);
+                tma_load(as + ABYTES, &zmap, q0, 0, &full[s]);
+                loaded = it + 1;
             }
-            tma_load_3d(bs, &zmap, 0, (int)q0, 0, &bars[0]);
+            s_loaded = loaded;
         }
-        const bool loaded = mbar_wait(&bars[0], it & 1);
-        if (__syncthreads_or(!loaded)) {
-            failed = load_pending = true;
-            break;
-        }
-        if (tid == 0) {
+    } else if (warp == 5) {
+        const uint32_t issuer = lane == 0;
+        int issued = 0;
+        for (int it = 0; it < ntiles; it++) {
+            const int s = it % WG_STAGES, k = it / WG_STAGES;
+            if (!__all_sync(0xffffffffu, mbar_wait(&full[s], k & 1))) {
+                *failed = 1;
+                break;
+            }
+            if (__any_sync(0xffffffffu, *failed != 0)) break;
             tc_fence_after();
-            const uint32_t a0 = smem_u32(as), b0 = smem_u32(bs);
-#pragma unroll 1
+            const uint32_t a0 = smem_u32(smem) + (uint32_t)(s * SBYTES);
+            const uint64_t ad0 = smem_desc(a0, 128, PLANE), bd0 = smem_desc(a0 + ABYTES, 128, PLANE);
+#pragma unroll
             for (int g = 0; g < NG; g++)
 #pragma unroll
-                for (int k = 0; k < WG_KT / 16; k++) {
-                    const uint64_t ad = smem_desc(a0 + (uint32_t)(g * 16 * PLANE + k * 256), 128, PLANE);
-                    const uint64_t bd = smem_desc(b0 + (uint32_t)(k * 256), 128, PLANE);
-                    mma_bf16(tmem + (uint32_t)(g * 32), ad, bd, IDESC_BF16_MN_M128_N32, (any || k != 0) ? 1u : 0u);
-                }
-            mma_commit(&bars[1]);
+                for (int kk = 0; kk < WG_KT / 16; kk++)
+                    mma_bf16(tmem + (uint32_t)(g * 32), ad0 + (uint64_t)((g * 16 * PLANE + kk * 256) >> 4), bd0 + (uint64_t)((kk * 256) >> 4),
+                             IDESC_BF16_MN_M128_N32, (it != 0 || kk != 0) ? 1u : 0u, issuer);
+            if (issuer) mma_commit(&empty[s]);
+            __syncwarp();
+            issued = it + 1;
         }
-        any = true;
-        // the bias gradient from the staged dz tile: thread (warp, lane) sums channel lane over pixels warp, warp + 4, ...
-        {
-            const __nv_bfloat16* z = reinterpret_cast<const __nv_bfloat16*>(bs);
+        if (issuer) {
+            if (issued > 0) mma_commit(done);
+            s_issued = issued;
+        }
+    } else {
+        for (int it = 0; it < ntiles; it++) {
+            const int s = it % WG_STAGES, k = it / WG_STAGES;
+            const bool ok = mbar_wait(&full[s], k & 1);
+            if (!__all_sync(0xffffffffu, ok)) {
+                if (lane == 0) *failed = 1;
+                break;
+            }
+            const __nv_bfloat16* z = reinterpret_cast<const __nv_bfloat16*>(smem + s * SBYTES + ABYTES);
+#pragma unroll 8
             for (int p = warp; p < WG_KT; p += 4) dbsum += __bfloat162float(z[((lane >> 3) * WG_KT + p) * 8 + (lane & 7)]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[s]);
+            if (__any_sync(0xffffffffu, *failed != 0)) break;
         }
-        const bool computed = mbar_wait(&bars[1], it & 1);
-        if (__syncthreads_or(!computed)) {
-            failed = mma_pending = true;
-            break;
-        }
-        tc_fence_before();
-        __syncthreads();
     }
-    if (failed && tid == 0) atomicOr(err, 1u);
-    if (load_pending) mbar_wait(&bars[0], it & 1);
-    if (mma_pending) mbar_wait(&bars[1], it & 1);
-    tc_fence_before();
     __syncthreads();
+    const bool bad = *failed != 0;
+    if (tid == 0 && bad) atomicOr(err, 1u);
+    // copies issued but never waited for by the MMAs (bounded), then every MMA issued
+    if (warp == 4 && lane == 0)
+        for (int it = s_issued; it < s_loaded; it++) mbar_wait(&full[it % WG_STAGES], (it / WG_STAGES) & 1);
+    const bool computed = s_issued > 0 && mbar_wait(done, 0);
+    if (__syncthreads_or(s_issued > 0 && !computed) && tid == 0) atomicOr(err, 1u);
     tc_fence_after();
-    if (!failed && any) {
+    if (warp < 4 && !bad && computed) {
         atomicAdd(&dbs[lane], dbsum);
         for (int g = 0; g < NG; g++) {
             float v[32];
@@ -220,13 +273,12 @@ __global__ void __launch_bounds__(128, 1) wgrad3x3_kernel(const __grid_constant_
 #pragma unroll
                 for (int o = 0; o < 32; o++) atomicAdd(&dw[(t * COUT + o) * CIN + i], v[o]);
         }
-        __syncthreads();
-        if (tid < 32 && db != nullptr) atomicAdd(&db[tid], dbs[tid]);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(NCOL));
+    if (tid < 32 && !bad && computed && db != nullptr) atomicAdd(&db[tid], dbs[tid]);
+    if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(NCOL));
 }
 
 
@@ -241,45 +293,35 @@ __global__ void __launch_bounds__(128, 1) wgrad3x3_kernel(const __grid_constant_
 // the epilogue while the next tile's MMAs fill the other accumulator. Every wait is bounded: a role that
 // gives up sets the CTA's failure flag, every other role stops at its next wait, and the tile loop ends; the
 // copies and MMAs still in flight are then waited for (bounded) before the TMEM is freed.
-constexpr int CP_STAGES = 4;
 constexpr int CP_THREADS = 192;
 
-// A tile of MT x 128 output pixels: MT MMAs of M = 128 a tap and K chunk. The halo it stages (51 pixels each
-// side): 232 pixels for MT = 1, loaded as one box of every plane; 368 for MT = 2, each plane as two boxes of 184
-// (the box limit is 256 pixels, and every box must land on a 128-byte boundary: 8 pixels). Stages: as many as
-// keep two CTAs an SM (4 of 15 KB, or 3 of 23 KB, at CIN 32).
-template <int MT>
-__host__ __device__ constexpr int cp_halo() { return MT == 1 ? 232 : 368; }
-template <int MT>
-__host__ __device__ constexpr int cp_box() { return MT == 1 ? cp_halo<MT>() : cp_halo<MT>() / 2; }
-template <int MT>
-__host__ __device__ constexpr int cp_stages() { return MT == 1 ? 4 : 3; }
-static_assert(cp_halo<1>() >= TILE + 2 * HALO_LO && cp_halo<2>() >= 2 * TILE + 2 * HALO_LO, "the halo covers every tap's rows");
+// A tile of 256 output pixels: two MMAs of M = 128 a tap and K chunk. The halo it stages (51 pixels each side) is each
+// plane's three boxes of 128 pixels. Stages: as many as keep two CTAs an SM (3 of 24 KB at CIN 32).
+constexpr int CP_MT = 2;
+constexpr int CP_PIXELS = CP_MT * TILE;
+constexpr int CP_HALO = 3 * BOX_PIXELS;
+constexpr int CP_STAGES = 3;
+static_assert(CP_HALO >= CP_PIXELS + 2 * HALO_LO, "the halo covers every tap's rows");
 
-template <int CIN, int MT = 1>
+template <int CIN>
 constexpr int conv3x3p_smem_bytes() {
-    return 9 * (CIN / 8) * COUT * 16 + cp_stages<MT>() * (CIN / 8) * cp_halo<MT>() * 16 + (2 * cp_stages<MT>() + 4) * 8 + 16;
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+    return 9 * (CIN / 8) * COUT * 16 + CP_STAGES * (CIN / 8) * CP_HALO * 16 + (2 * CP_STAGES + 4) * 8 + 16;
 }
 
 // One 3x3 convolution layer (CIN input channels, 32 output channels) over the chunk-major padded rasters:
 // y = act(conv(x, w) + bias), act = ReLU (relu != 0) or the identity, then times (mask > 0) when `mask` is set
 // (the gradient through the layer's ReLU); the ring pixels of y are zero. w is [9 taps][32 out][CIN in] BF16,
-// tap = 3 * dy + dx. x is read through `map` (planes CIN / 8, Q pixels, 8 channels; boxes of cp_box<MT>() pixels of
-// every plane (MT = 1) or of one plane (MT = 2)). tiles = ceil(Q / (MT x 128)).
-template <int CIN, int MT = 1>
+// tap = 3 * dy + dx. x is read through `map` (BOX_PIXELS pixels of one plane a box); planes of mask and y are Q pixels
+// apart, and the launch computes `pixels` of them (whole samples), in tiles = ceil(pixels / CP_PIXELS).
+template <int CIN>
 __global__ void __launch_bounds__(CP_THREADS, 1) conv3x3p_kernel(const __grid_constant__ CUtensorMap map, const __nv_bfloat16* __restrict__ w,
                                                                  const float* __restrict__ bias, int relu, const __nv_bfloat16* __restrict__ mask,
-                                                                 __nv_bfloat16* __restrict__ y, long long Q, int tiles, unsigned* err) {
-    constexpr int KC = CIN / 8;
-    constexpr int CP_STAGES = cp_stages<MT>();  // this form's ring of stages
+                                                                 __nv_bfloat16* __restrict__ y, long long Q, long long pixels, int tiles, unsigned* err) {
+    constexpr int KC = CIN / 8, MT = CP_MT;
     constexpr int WBYTES = 9 * KC * COUT * 16;
-    constexpr int HP = cp_halo<MT>();                          // halo pixels a stage
+    constexpr int HP = CP_HALO;                                // halo pixels a stage
     constexpr int HBYTES = KC * HP * 16;
-    constexpr int TP = MT * TILE;                              // output pixels a tile
+    constexpr int TP = CP_PIXELS;                              // output pixels a tile
     constexpr int ACOLS = MT * COUT;                           // TMEM columns an accumulator
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* ws = smem;                                        // weights: [tap][chunk][out][16 B]
@@ -332,56 +374,48 @@ __global__ void __launch_bounds__(CP_THREADS, 1) conv3x3p_kernel(const __grid_co
                 if (*failed) break;
                 const long long q0 = ((long long)blockIdx.x + (long long)it * gridDim.x) * TP;
                 mbar_expect_tx(&full[s], HBYTES);
-                if constexpr (MT == 1) {
-                    tma_load_3d(halos + s * HBYTES, &map, 0, (int)(q0 - HALO_LO), 0, &full[s]);
-                } else {
 #pragma unroll
-                    for (int c = 0; c < KC; c++)
+                for (int c = 0; c < KC; c++)
 #pragma unroll
-                        for (int m = 0; m < 2; m++)
-                            tma_load_3d(halos + s * HBYTES + (c * HP + m * (HP / 2)) * 16, &map, 0, (int)(q0 - HALO_LO) + m * (HP / 2), c,
-                                        &full[s]);
-                }
+                    for (int m = 0; m < HP / BOX_PIXELS; m++)
+                        tma_load(halos + s * HBYTES + (c * HP + m * BOX_PIXELS) * 16, &map, (int)(q0 - HALO_LO) + m * BOX_PIXELS, c, &full[s]);
                 loaded = it + 1;
             }
             s_loaded = loaded;
         }
     } else if (warp == 5) {
         // the MMA issuer: tile it into accumulator it & 1
+        const uint32_t issuer = lane == 0;
         int issued = 0;
-        if (lane == 0) {
-            for (int it = 0; it < ntiles; it++) {
-                const int s = it % CP_STAGES, k = it / CP_STAGES, a = it & 1, j = it >> 1;
-                if (!mbar_wait(&full[s], k & 1)) {
-                    *failed = 1;
-                    break;
-                }
-                if (j > 0 && !mbar_wait(&acce[a], (j - 1) & 1)) {
-                    *failed = 1;
-                    break;
-                }
-                if (*failed) break;
-                tc_fence_after();
-                const uint32_t h = smem_u32(halos + s * HBYTES), wb = smem_u32(ws), d = tmem + (uint32_t)(a * ACOLS);
-#pragma unroll 1
-                for (int t = 0; t < 9; t++) {
-                    const int shift = (t / 3 - 1) * RW + (t % 3 - 1);
+        for (int it = 0; it < ntiles; it++) {
+            const int s = it % CP_STAGES, k = it / CP_STAGES, a = it & 1, j = it >> 1;
+            bool ok = mbar_wait(&full[s], k & 1);
+            if (j > 0) ok = mbar_wait(&acce[a], (j - 1) & 1) && ok;
+            if (!__all_sync(0xffffffffu, ok)) {
+                *failed = 1;
+                break;
+            }
+            if (__any_sync(0xffffffffu, *failed != 0)) break;
+            tc_fence_after();
+            const uint32_t d = tmem + (uint32_t)(a * ACOLS);
+            const uint64_t ad0 = smem_desc(smem_u32(halos) + (uint32_t)(s * HBYTES), HP * 16, 8 * 16);
+            const uint64_t bd0 = smem_desc(smem_u32(ws), COUT * 16, 8 * 16);
 #pragma unroll
-                    for (int kk = 0; kk < KC / 2; kk++) {
-                        const uint64_t bd = smem_desc(wb + (uint32_t)((t * KC + 2 * kk) * COUT * 16), COUT * 16, 8 * 16);
+            for (int t = 0; t < 9; t++)
 #pragma unroll
-                        for (int mh = 0; mh < MT; mh++) {
-                            const uint64_t ad = smem_desc(h + (uint32_t)((2 * kk * HP + HALO_LO + shift + mh * TILE) * 16), HP * 16, 8 * 16);
-                            mma_bf16(d + (uint32_t)(mh * COUT), ad, bd, IDESC_BF16_M128_N32, (t | kk) != 0);
-                        }
-                    }
-                }
+                for (int kk = 0; kk < KC / 2; kk++)
+#pragma unroll
+                    for (int mh = 0; mh < MT; mh++)
+                        mma_bf16(d + (uint32_t)(mh * COUT), ad0 + (uint64_t)(2 * kk * HP + HALO_LO + (t / 3 - 1) * RW + (t % 3 - 1) + mh * TILE),
+                                 bd0 + (uint64_t)((t * KC + 2 * kk) * COUT), IDESC_BF16_M128_N32, (t | kk) != 0, issuer);
+            if (issuer) {
                 mma_commit(&empty[s]);
                 mma_commit(&accf[a]);
-                issued = it + 1;
             }
-            s_issued = issued;
+            __syncwarp();
+            issued = it + 1;
         }
+        if (issuer) s_issued = issued;
     } else {
         // the epilogue: warp w reads TMEM lanes 32w .. 32w + 31 (pixels), releases the accumulator, stores.
         // The bias stays in registers; a pixel's raster position comes from its tile's (one 64-bit remainder
@@ -409,7 +443,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1) conv3x3p_kernel(const __grid_co
             for (int mh = 0; mh < MT; mh++) {
                 const float (&v)[32] = vv[mh];
                 const long long q = q0 + mh * TILE + warp * 32 + lane;
-                if (q < Q) {
+                if (q < pixels) {
                     int p = r0 + mh * TILE + warp * 32 + lane;
                     if (p >= RPIX) p -= RPIX;
                     const int ry = p / RW, rx = p - ry * RW;
