@@ -683,7 +683,7 @@ def run_encode(args, rank, world):
         # per picture: scene cut 2, source copy 1, chroma 2, decide 1, writer 3 (CABAC: 1), records 1, deblocking 2, planes 1, chroma
         # copies 2 (and their padding)
         "gpu_launches": (14 if args.cabac else 16) * args.steps,
-        "roofline": {"bound": "latency", "kernel": "decide_rd3_kernel<uint8_t>" if args.cabac else "decide_kernel<uint8_t>", "achieved": None,
+        "roofline": {"bound": "latency", "kernel": "decide_rdw_kernel<uint8_t>" if args.cabac else "decide_kernel<uint8_t>", "achieved": None,
                      "peak": None, "unit": None, "frac": None, "traffic": None,
                      "note": ("one stream's slice bands under CABAC: 8 chains of ~1020 dependent macroblocks bound the picture"
                               if args.cabac else "one stream's decide wavefront (a chain of ~136 dependent macroblocks) bounds the picture")},

@@ -48,107 +48,117 @@ struct Counter {
     __device__ __forceinline__ void terminate(int bin) { bits += bin ? 7 * 256 : 1; }
 };
 
-// Bits MSB first into 32-bit words of a region in global memory, stored so that the bytes read in order
-// (BitWriter, enc/bitw.rs:4-25). A write beyond the region sets `over` and is dropped.
-struct BitOut {
+// The arithmetic coder's output: 32-bit pieces of the code value, MSB first, into the words of a region in global memory,
+// stored so that the bytes read in order. A piece may carry into the ones before it, so the newest is held back, with a count of
+// the 0xFFFFFFFF pieces after it that a carry would run through. A write beyond the region sets `over` and is dropped.
+struct WordOut {
     uint32_t* words;
     uint32_t cap;  // words
     uint32_t nw;
-    uint64_t cur;
-    int n;
-    bool over;
-    __device__ __forceinline__ void put(int k, uint32_t v) {  // k <= 32
-        cur = (cur << k) | (uint64_t)v;
-        n += k;
-        if (n >= 32) {
-            n -= 32;
-            const uint32_t w = (uint32_t)(cur >> n);
-            if (nw < cap) words[nw] = __byte_perm(w, 0, 0x0123);
-            else over = true;
-            nw++;
-            cur &= n ? ((1ull << n) - 1) : 0ull;
-        }
+    uint32_t held, ones;
+    bool any, over;
+    __device__ __forceinline__ void store(uint32_t v) {
+        if (nw < cap) words[nw] = __byte_perm(v, 0, 0x0123);
+        else over = true;
+        nw++;
     }
-    // the last word padded with zeros to its byte (into_bytes, enc/bitw.rs:60-67); returns the byte count
-    __device__ __forceinline__ uint32_t finish() {
-        uint32_t bytes = nw * 4;
-        if (n > 0) {
-            const int nb = (n + 7) >> 3;
-            const uint32_t w = (uint32_t)(cur << (32 - n));
-            if (nw < cap) words[nw] = __byte_perm(w, 0, 0x0123);
-            else over = true;
-            bytes += nb;
+    __device__ __forceinline__ void flush(uint32_t carry) {
+        if (any) store(held + carry);
+        for (; ones > 0; ones--) store(carry ? 0u : 0xFFFFFFFFu);
+        any = false;
+    }
+    __device__ __forceinline__ void put(uint64_t v) {  // 32 bits and their carry
+        if (v == 0xFFFFFFFFull && any) {
+            ones++;
+            return;
         }
+        flush((uint32_t)(v >> 32));
+        held = (uint32_t)v;
+        any = true;
+    }
+    // the last k < 32 bits (and their carry), padded with zeros to a byte; returns the byte count
+    __device__ __forceinline__ uint32_t finish(uint64_t v, int k) {
+        flush((uint32_t)(v >> k));
+        const uint32_t bytes = nw * 4 + (uint32_t)((k + 7) >> 3);
+        if (k > 0) store((uint32_t)(v << (32 - k)));
         return bytes;
     }
 };
 
-// The arithmetic coder (9.3.4.2-9.3.4.5) over its contexts.
+// A bin as the coder takes it: of a decision, the LPS range of its state for each quarter of the range (a byte each), that range
+// renormalised (its low byte; the ninth bit is set) and by how many bits; and what kind of bin it is.
+enum CodeKind : uint32_t { CODE_MPS = 0, CODE_LPS = 1, CODE_BYPASS = 2, CODE_TERMINATE = 4 };  // the last two + the bin
+struct __align__(16) CodeBin {
+    uint32_t lps, norm, shift, kind;
+};
+static_assert(sizeof(CodeBin) == 16, "one 16-byte read");
+// The entry of probability state p.
+__device__ __forceinline__ CodeBin code_entry(int p) {
+    CodeBin e = {0, 0, 0, CODE_MPS};
+    for (int q = 0; q < 4; q++) {
+        const uint32_t r = LPS_RANGE[p][q], sh = (uint32_t)__clz((int)r) - 23u;
+        e.lps |= r << (8 * q);
+        e.norm |= ((r << sh) & 0xFFu) << (8 * q);
+        e.shift |= sh << (8 * q);
+    }
+    return e;
+}
+
+// The arithmetic coder (9.3.4.2-9.3.4.5). Its serial chain is the range alone: a bin's probability state is looked up before it, and
+// the code value is a plain sum, kept whole: `low` holds the 10 bits of the standard's codILow below the nb bits already shifted
+// out of it, and a carry above them. nb begins at -1: the first bit of the code is not written (9.3.4.2).
 struct Coder {
-    uint8_t* st;
-    const uint32_t* step;
-    BitOut* out;
-    uint32_t low, range, outstanding;
-    bool first;
-    __device__ __forceinline__ void put_bit(uint32_t b) {
-        if (first) first = false;
-        else out->put(1, b);
-        while (outstanding > 0) {
-            const int k = outstanding < 32 ? (int)outstanding : 32;
-            out->put(k, b ? 0u : (k == 32 ? 0xFFFFFFFFu : (1u << k) - 1));
-            outstanding -= k;
+    WordOut out;
+    uint64_t low;
+    uint32_t range;
+    int nb;
+    __device__ __forceinline__ void shift(uint32_t sh) {
+        low <<= sh;
+        nb += (int)sh;
+        if (nb >= 32) {
+            const int rest = nb - 22;  // 10 + nb - 32
+            out.put(low >> rest);
+            low &= (1ull << rest) - 1;
+            nb -= 32;
         }
     }
-    __device__ __forceinline__ void renorm() {
-        while (range < 256) {
-            if (low < 256) put_bit(0);
-            else if (low >= 512) {
-                low -= 512;
-                put_bit(1);
+    __device__ __forceinline__ void code(const CodeBin& e) {
+        uint32_t sh;
+        if (e.kind <= CODE_LPS) {
+            const uint32_t q = (range >> 3) & 0x18u, mps = range - ((e.lps >> q) & 0xFFu);
+            const bool lps = e.kind == CODE_LPS;
+            low += lps ? mps : 0u;
+            const uint32_t ms = mps < 256u;
+            sh = lps ? (e.shift >> q) & 0xFFu : ms;
+            range = lps ? 256u | ((e.norm >> q) & 0xFFu) : mps << ms;
+        } else if (e.kind < CODE_TERMINATE) {
+            // the bin's share of the range, after the shift: low = 2 low + bin * range
+            low = (low << 1) + ((e.kind & 1u) ? range : 0u);
+            nb += 1;
+            sh = 0;
+        } else {
+            range -= 2;
+            if (e.kind & 1u) {
+                low += range;
+                range = 2;
+                sh = 7;
             } else {
-                low -= 256;
-                outstanding++;
+                sh = range < 256u;
             }
-            range <<= 1;
-            low <<= 1;
+            range <<= sh;
         }
+        shift(sh);
     }
-    __device__ __forceinline__ void decision(int ctx, int bin) {
-        const int s = st[ctx], p = s >> 1, mps = s & 1;
-        bin = bin != 0;
-        const uint32_t lps = LPS_RANGE[p][(range >> 6) & 3];
-        range -= lps;
-        if (bin != mps) {
-            low += range;
-            range = lps;
+    // after the last terminate bin: the flush's bit and two more, the last of them the rbsp_stop_one_bit
+    __device__ __forceinline__ uint32_t finish() {
+        uint64_t v = (low >> 7) | 1u;
+        int k = nb + 3;
+        if (k >= 32) {
+            k -= 32;
+            out.put(v >> k);
+            v &= (1ull << k) - 1;
         }
-        st[ctx] = (uint8_t)step[s * 2 + bin];
-        renorm();
-    }
-    __device__ __forceinline__ void bypass(int bin) {
-        low <<= 1;
-        if (bin) low += range;
-        if (low >= 1024) {
-            put_bit(1);
-            low -= 1024;
-        } else if (low < 512) {
-            put_bit(0);
-        } else {
-            low -= 512;
-            outstanding++;
-        }
-    }
-    __device__ __forceinline__ void terminate(int bin) {
-        range -= 2;
-        if (bin) {
-            low += range;
-            range = 2;
-            renorm();
-            put_bit((low >> 9) & 1);
-            out->put(2, ((low >> 7) & 3) | 1);  // the last of the two bits is the rbsp_stop_one_bit
-        } else {
-            renorm();
-        }
+        return out.finish(v, k);
     }
 };
 
@@ -160,76 +170,6 @@ struct Nb {
     uint8_t nnz[16];
     uint8_t cnnz[2][4];
 };
-
-__device__ __forceinline__ int rects_d(int part, const uint8_t* sub, int4* r) {
-    if (part == 0) {
-        r[0] = make_int4(0, 0, 4, 4);
-        return 1;
-    }
-    if (part == 1) {
-        r[0] = make_int4(0, 0, 4, 2);
-        r[1] = make_int4(0, 2, 4, 2);
-        return 2;
-    }
-    if (part == 2) {
-        r[0] = make_int4(0, 0, 2, 4);
-        r[1] = make_int4(2, 0, 2, 4);
-        return 2;
-    }
-    int n = 0;
-    for (int k = 0; k < 4; k++) {
-        const int ox = (k & 1) * 2, oy = (k >> 1) * 2, s = sub[k];
-        if (s == 0) r[n++] = make_int4(ox, oy, 2, 2);
-        else if (s == 1) {
-            r[n++] = make_int4(ox, oy, 2, 1);
-            r[n++] = make_int4(ox, oy + 1, 2, 1);
-        } else if (s == 2) {
-            r[n++] = make_int4(ox, oy, 1, 2);
-            r[n++] = make_int4(ox + 1, oy, 1, 2);
-        } else {
-            for (int q = 0; q < 4; q++) r[n++] = make_int4(ox + (q & 1), oy + (q >> 1), 1, 1);
-        }
-    }
-    return n;
-}
-
-// The absolute vector differences of an inter, not skipped, macroblock per 4x4 block (mvd_grid).
-__device__ __forceinline__ void mvd_grid(const ironav_mbcode* k, uint8_t (*g)[2]) {
-    for (int i = 0; i < 16; i++) g[i][0] = g[i][1] = 0;
-    if (k->kind != KIND_INTER || k->skip) return;
-    int4 rs[16];
-    const int nr = rects_d(k->part, k->sub, rs);
-    for (int q = 0; q < nr; q++) {
-        const uint8_t ax = (uint8_t)min(abs((int)k->mvds[q][0]), 64), ay = (uint8_t)min(abs((int)k->mvds[q][1]), 64);
-        for (int by = rs[q].y; by < rs[q].y + rs[q].w; by++)
-            for (int bx = rs[q].x; bx < rs[q].x + rs[q].z; bx++) {
-                g[by * 4 + bx][0] = ax;
-                g[by * 4 + bx][1] = ay;
-            }
-    }
-}
-
-// A neighbour's Nb from its code (one lane).
-__device__ __forceinline__ void nb_of(const ironav_mbcode* k, Nb* n) {
-    n->avail = 1;
-    n->skip = k->skip;
-    n->kind = k->kind;
-    n->inter = k->kind == KIND_INTER;
-    n->cbp = k->res.cbp;
-    n->t8x8 = k->res.t8x8;
-    n->chroma_mode = n->inter ? 0 : k->chroma_mode;
-    const int cbpc = k->res.cbp >> 4;
-    int any0 = 0, any1 = 0, any2 = 0;
-    for (int i = 0; i < 16; i++) any0 |= k->dc[i] != 0;
-    for (int i = 0; i < 4; i++) any1 |= k->res.cdc[0][i] != 0, any2 |= k->res.cdc[1][i] != 0;
-    n->cbf_dc = (uint8_t)((k->kind == KIND_I16 && any0) | ((cbpc > 0 && any1) << 1) | ((cbpc > 0 && any2) << 2));
-    for (int i = 0; i < 16; i++) n->nnz[i] = k->res.nnz[i];
-    for (int c = 0; c < 2; c++)
-        for (int i = 0; i < 4; i++) n->cnnz[c][i] = k->res.cnnz[c][i];
-    for (int b8 = 0; b8 < 4; b8++)
-        n->r8[b8] = n->inter ? (int8_t)k->refs[k->part == 0 ? 0 : k->part == 1 ? b8 >> 1 : k->part == 2 ? (b8 & 1) : b8] : (int8_t)-1;
-    mvd_grid(k, n->mvd);
-}
 
 // The partition (rects order) that holds 4x4 block (bx, by) of a P macroblock.
 __device__ __forceinline__ int part_index(int part, const uint8_t* sub, int bx, int by) {
@@ -243,10 +183,29 @@ __device__ __forceinline__ int part_index(int part, const uint8_t* sub, int bx, 
     return n + (s == 0 ? 0 : s == 1 ? (by & 1) : s == 2 ? (bx & 1) : (by & 1) * 2 + (bx & 1));
 }
 
+// The origin of partition n (rects order) of a P macroblock; false beyond the last.
+__device__ __forceinline__ bool part_origin(int part, const uint8_t* sub, int n, int* bx, int* by) {
+    if (part < 3) {
+        *bx = part == 2 ? 2 * n : 0;
+        *by = part == 1 ? 2 * n : 0;
+        return n < (part == 0 ? 1 : 2);
+    }
+    for (int k = 0; k < 4; k++) {
+        const int s = sub[k], count = s == 0 ? 1 : (s == 3 ? 4 : 2);
+        if (n < count) {
+            *bx = (k & 1) * 2 + (s == 2 ? n : (s == 3 ? (n & 1) : 0));
+            *by = (k >> 1) * 2 + (s == 1 ? n : (s == 3 ? (n >> 1) : 0));
+            return true;
+        }
+        n -= count;
+    }
+    return false;
+}
+
 constexpr int NB_WORDS = (int)(sizeof(Nb) / 4);
 static_assert(sizeof(Nb) % 4 == 0, "Nb in whole words");
 
-// nb_of with the warp: every lane calls; the code in shared or global memory.
+// A neighbour's Nb from its code (in shared or global memory); every lane of the warp calls.
 __device__ __forceinline__ void nb_of_warp(const ironav_mbcode* k, Nb* n) {
     const int lane = threadIdx.x & 31;
     const int kind = k->kind, skip = k->skip, cbp = k->res.cbp;
@@ -294,36 +253,31 @@ __device__ __forceinline__ int pred_mode(const int* nbm, const uint8_t* cur, int
     return (a >= 0 && b >= 0) ? min(a, b) : 2;
 }
 
-// write_block, enc/cabac.rs:194-250: coded_block_flag (context cbf, none when < 0) and max levels of
-// category cat in scan order; part 0 all of it, 1 its significance map (coded_block_flag,
-// significant_coeff_flag, last_significant_coeff_flag), 2 its levels (coeff_abs_level_minus1 and the signs):
-// the two parts' contexts are disjoint.
+// write_block, enc/cabac.rs:194-250: coded_block_flag (context cbf, none when < 0), then the significance map
+// (significant_coeff_flag, last_significant_coeff_flag) and the levels (coeff_abs_level_minus1 and the signs) of a block of
+// category cat with max levels in scan order.
 template <class S>
-__device__ __forceinline__ void block(S& c, int cat, int cbf, const int16_t* lv, int max, int part = 0) {
-    int last = -1;
-    for (int i = 0; i < max; i++)
-        if (lv[i]) last = i;
-    if (cbf >= 0 && part != 2) c.decision(cbf, last >= 0);
-    if (last < 0) return;
-    if (part != 2) {
-        const int so = SIG_OFF[0][cat], lo = LAST_OFF[0][cat];
-        for (int i = 0; i < max - 1; i++) {
-            // 4:2:0 chroma DC has three significance contexts, one per position; 8x8 blocks share theirs
-            const int sig = cat == 3 ? min(i, 2) : cat == 5 ? SIG_OFF_8X8[0][i] : i;
-            const int lst = cat == 3 ? min(i, 2) : cat == 5 ? LAST_OFF_8X8[i] : i;
-            c.decision(so + sig, lv[i] != 0);
-            if (lv[i]) {
-                c.decision(lo + lst, i == last);
-                if (i == last) break;
-            }
-        }
+__device__ __forceinline__ void block(S& c, int cat, int cbf, const int16_t* lv, int max) {
+    unsigned long long nz = 0;
+    for (int i = 0; i < max; i++) nz |= (unsigned long long)(lv[i] != 0) << i;
+    if (cbf >= 0) c.decision(cbf, nz != 0);
+    if (nz == 0) return;
+    const int last = 63 - __clzll((long long)nz);
+    const int so = SIG_OFF[0][cat], lo = LAST_OFF[0][cat];
+    for (int i = 0; i < max - 1 && i <= last; i++) {
+        // 4:2:0 chroma DC has three significance contexts, one per position; 8x8 blocks share theirs
+        const int sig = cat == 3 ? min(i, 2) : cat == 5 ? SIG_OFF_8X8[0][i] : i;
+        const int lst = cat == 3 ? min(i, 2) : cat == 5 ? LAST_OFF_8X8[i] : i;
+        const int bit = (int)((nz >> i) & 1u);
+        c.decision(so + sig, bit);
+        if (bit) c.decision(lo + lst, i == last);
     }
-    if (part == 1) return;
     const int base = ABS_OFF[cat];
     int eq1 = 0, gt1 = 0;
-    for (int i = last; i >= 0; i--) {
+    while (nz) {
+        const int i = 63 - __clzll((long long)nz);
+        nz &= ~(1ull << i);
         const int l = lv[i];
-        if (!l) continue;
         const uint32_t a = (uint32_t)abs(l);
         const int inc0 = gt1 ? 0 : min(1 + eq1, 4);
         if (a == 1) {
@@ -389,38 +343,15 @@ struct Slice {
     int p_slice, t8, nref;
 };
 
-// The bins of a macroblock fall in groups whose contexts are disjoint: its syntax up to mb_qp_delta
-// (contexts below 85, and 399-401), and the residual blocks of each category with their coded_block_flag
-// (Intra16x16 DC; the luma blocks, 4x4 or 8x8; chroma DC; chroma AC: contexts 85-104 by category, 105 and
-// up by category). So the bits of a macroblock are the sum of the groups' bits, each group walked on its
-// own from the same contexts, and the contexts after it are the union of the groups' updates.
-// Each category's significance map and levels use disjoint contexts too, so a category is two groups.
-enum Group { ALL = -1, HEAD = 0, DC16_MAP, DC16_LEV, LUMA_MAP, LUMA_LEV, CDC_MAP, CDC_LEV, CAC_MAP, CAC_LEV, NGROUPS };
-
-// The groups of a residual category: whether `group` walks it, and which part of its blocks.
-__device__ __forceinline__ bool in_group(int group, int map_group, int* part) {
-    if (group == ALL) {
-        *part = 0;
-        return true;
-    }
-    *part = group == map_group ? 1 : 2;
-    return group == map_group || group == map_group + 1;
-}
-
-// mb_bins' HEAD group after mb_skip_flag (enc/frame.rs:2046-2244): mb_type, the prediction modes,
-// sub_mb_type, ref_idx, mvd, coded_block_pattern, transform_size_8x8_flag and mb_qp_delta.
+// mb_bins after mb_skip_flag and before the residual (enc/frame.rs:2046-2244), in three pieces in coding order, so that the
+// middle one's parts can be walked side by side: mb_type (with an Intra NxN macroblock's transform_size_8x8_flag),
+// sub_mb_type and ref_idx; the prediction modes or the vector differences; the rest.
 template <class S>
-__device__ __forceinline__ void head_bins(S& c, const Slice& sl, const ironav_mbcode* code, const Nb& L, const Nb& T, const int* nbm) {
+__device__ __forceinline__ void head_first(S& c, const Slice& sl, const ironav_mbcode* code, const Nb& L, const Nb& T) {
     const bool la = L.avail, ta = T.avail;
     const int kind = code->kind, cbp = code->res.cbp, cbpl = cbp & 15, cbpc = cbp >> 4;
     // mb_type
-    if (kind == KIND_INTER) {
-        // P_L0_16x16 000, P_L0_L0_16x8 011, P_L0_L0_8x16 010, P_8x8 001
-        const int b1 = code->part == 1 || code->part == 2, b2 = code->part == 1 || code->part == 3;
-        c.decision(14, 0);
-        c.decision(15, b1);
-        c.decision(b1 ? 17 : 16, b2);
-    } else {
+    if (kind != KIND_INTER) {
         const int pre = sl.p_slice, base = pre ? 17 : 3;
         int first;
         if (pre) {
@@ -441,73 +372,87 @@ __device__ __forceinline__ void head_bins(S& c, const Slice& sl, const ironav_mb
             c.decision(pre ? base + 3 : base + 6, (code->i16_mode >> 1) == 1);
             c.decision(pre ? base + 3 : base + 7, code->i16_mode & 1);
         }
+        return;
     }
-    if (nxn(kind)) {
-        const bool t8 = kind == KIND_I8;
-        uint8_t so_far[16];
-        for (int i = 0; i < 16; i++) so_far[i] = 2;
-        for (int n = 0; n < (t8 ? 4 : 16); n++) {
-            const int bx = t8 ? (n & 1) * 2 : ((n >> 2) & 1) * 2 + (n & 1);
-            const int by = t8 ? (n >> 1) * 2 : ((n >> 3) & 1) * 2 + ((n >> 1) & 1);
-            const int mode = code->modes[by * 4 + bx];
-            const int pred = pred_mode(nbm, so_far, bx, by);
-            so_far[by * 4 + bx] = (uint8_t)mode;
-            if (t8) so_far[by * 4 + bx + 1] = so_far[(by + 1) * 4 + bx] = so_far[(by + 1) * 4 + bx + 1] = (uint8_t)mode;
-            c.decision(68, mode == pred);
-            if (mode != pred) {
-                const int rem = mode < pred ? mode : mode - 1;
-                for (int k = 0; k < 3; k++) c.decision(69, (rem >> k) & 1);
+    // P_L0_16x16 000, P_L0_L0_16x8 011, P_L0_L0_8x16 010, P_8x8 001
+    const int b1 = code->part == 1 || code->part == 2, b2 = code->part == 1 || code->part == 3;
+    c.decision(14, 0);
+    c.decision(15, b1);
+    c.decision(b1 ? 17 : 16, b2);
+    // sub_mb_type of each 8x8 block of P_8x8 (Table 9-38: 1, 00, 011, 010; contexts 21 to 23)
+    if (code->part == 3)
+        for (int k = 0; k < 4; k++) {
+            const int s = code->sub[k];
+            c.decision(21, s == 0);
+            if (s != 0) {
+                c.decision(22, s != 1);
+                if (s != 1) c.decision(23, s == 2);
             }
         }
+    // ref_idx_l0 per partition (per 8x8 block for P_8x8), unary, with the contexts of 9.3.3.1.1.6
+    if (sl.nref > 1) {
+        uint8_t grid[4] = {0, 0, 0, 0};
+        const int np = code->part == 0 ? 1 : code->part == 3 ? 4 : 2;
+        for (int k = 0; k < np; k++) {
+            int bx, by, w, h;
+            if (code->part == 0) bx = 0, by = 0, w = 4, h = 4;
+            else if (code->part == 1) bx = 0, by = 2 * k, w = 4, h = 2;
+            else if (code->part == 2) bx = 2 * k, by = 0, w = 2, h = 4;
+            else bx = (k & 1) * 2, by = (k >> 1) * 2, w = 2, h = 2;
+            const int a = bx > 0 ? grid[(by / 2) * 2 + (bx - 1) / 2] > 0 : (la && L.r8[(by / 2) * 2 + 1] > 0);
+            const int b = by > 0 ? grid[((by - 1) / 2) * 2 + bx / 2] > 0 : (ta && T.r8[2 + bx / 2] > 0);
+            const int r = code->refs[k], base = 54 + a + 2 * b;
+            for (int i = 0; i <= r; i++) c.decision(i == 0 ? base : i == 1 ? 58 : 59, i < r);
+            for (int y8 = by / 2; y8 <= (by + h - 1) / 2; y8++)
+                for (int x8 = bx / 2; x8 <= (bx + w - 1) / 2; x8++) grid[y8 * 2 + x8] = code->refs[k];
+        }
     }
+}
+
+// Part n (0..15, in coding order) of the middle piece: the prediction mode of block n of an Intra NxN macroblock, or the
+// vector difference of partition n of an inter one; nothing beyond the last. The modes of the blocks before it and the
+// differences of the partitions before it are the code's own, so every part can be walked on its own.
+template <class S>
+__device__ __forceinline__ void head_part(S& c, const ironav_mbcode* code, const Nb& L, const Nb& T, const int* nbm, int n) {
+    const int kind = code->kind;
+    if (nxn(kind)) {
+        const bool t8 = kind == KIND_I8;
+        if (t8 && n >= 4) return;
+        const int bx = t8 ? (n & 1) * 2 : ((n >> 2) & 1) * 2 + (n & 1);
+        const int by = t8 ? (n >> 1) * 2 : ((n >> 3) & 1) * 2 + ((n >> 1) & 1);
+        // the blocks to the left and above, at the origin of their 8x8 block for Intra8x8
+        const int step = t8 ? 2 : 1;
+        const int a = bx > 0 ? (int)code->modes[by * 4 + bx - step] : nbm[by], b = by > 0 ? (int)code->modes[(by - step) * 4 + bx] : nbm[4 + bx];
+        const int mode = code->modes[by * 4 + bx], pred = (a >= 0 && b >= 0) ? min(a, b) : 2;
+        c.decision(68, mode == pred);
+        if (mode != pred) {
+            const int rem = mode < pred ? mode : mode - 1;
+            for (int k = 0; k < 3; k++) c.decision(69, (rem >> k) & 1);
+        }
+        return;
+    }
+    if (kind != KIND_INTER) return;
+    int bx, by;
+    if (!part_origin(code->part, code->sub, n, &bx, &by)) return;
+    // the blocks left of and above a partition in the macroblock belong to earlier ones
+    const int pl = bx > 0 ? part_index(code->part, code->sub, bx - 1, by) : 0, pt = by > 0 ? part_index(code->part, code->sub, bx, by - 1) : 0;
+    for (int comp = 0; comp < 2; comp++) {
+        const uint32_t a = bx > 0 ? (uint32_t)min(abs((int)code->mvds[pl][comp]), 64) : (L.avail ? L.mvd[by * 4 + 3][comp] : 0u);
+        const uint32_t b = by > 0 ? (uint32_t)min(abs((int)code->mvds[pt][comp]), 64) : (T.avail ? T.mvd[12 + bx][comp] : 0u);
+        mvd(c, comp, code->mvds[n][comp], a + b);
+    }
+}
+
+template <class S>
+__device__ __forceinline__ void head_last(S& c, const Slice& sl, const ironav_mbcode* code, const Nb& L, const Nb& T) {
+    const bool la = L.avail, ta = T.avail;
+    const int kind = code->kind, cbp = code->res.cbp, cbpl = cbp & 15, cbpc = cbp >> 4;
     if (kind != KIND_INTER) {
         const int m = code->chroma_mode;
         c.decision(64 + (la && !L.inter && L.chroma_mode != 0) + (ta && !T.inter && T.chroma_mode != 0), m > 0);
         if (m > 0) {
             c.decision(67, m > 1);
             if (m > 1) c.decision(67, m > 2);
-        }
-    } else {
-        // sub_mb_type of each 8x8 block of P_8x8 (Table 9-38: 1, 00, 011, 010; contexts 21 to 23)
-        if (code->part == 3)
-            for (int k = 0; k < 4; k++) {
-                const int s = code->sub[k];
-                c.decision(21, s == 0);
-                if (s != 0) {
-                    c.decision(22, s != 1);
-                    if (s != 1) c.decision(23, s == 2);
-                }
-            }
-        // ref_idx_l0 per partition (per 8x8 block for P_8x8), unary, with the contexts of 9.3.3.1.1.6
-        if (sl.nref > 1) {
-            uint8_t grid[4] = {0, 0, 0, 0};
-            const int np = code->part == 0 ? 1 : code->part == 3 ? 4 : 2;
-            for (int k = 0; k < np; k++) {
-                int bx, by, w, h;
-                if (code->part == 0) bx = 0, by = 0, w = 4, h = 4;
-                else if (code->part == 1) bx = 0, by = 2 * k, w = 4, h = 2;
-                else if (code->part == 2) bx = 2 * k, by = 0, w = 2, h = 4;
-                else bx = (k & 1) * 2, by = (k >> 1) * 2, w = 2, h = 2;
-                const int a = bx > 0 ? grid[(by / 2) * 2 + (bx - 1) / 2] > 0 : (la && L.r8[(by / 2) * 2 + 1] > 0);
-                const int b = by > 0 ? grid[((by - 1) / 2) * 2 + bx / 2] > 0 : (ta && T.r8[2 + bx / 2] > 0);
-                const int r = code->refs[k], base = 54 + a + 2 * b;
-                for (int i = 0; i <= r; i++) c.decision(i == 0 ? base : i == 1 ? 58 : 59, i < r);
-                for (int y8 = by / 2; y8 <= (by + h - 1) / 2; y8++)
-                    for (int x8 = bx / 2; x8 <= (bx + w - 1) / 2; x8++) grid[y8 * 2 + x8] = code->refs[k];
-            }
-        }
-        // mvd_l0 per partition; the blocks left of and above a partition in the macroblock belong to earlier ones
-        uint8_t g[16][2];
-        mvd_grid(code, g);
-        int4 rs[16];
-        const int nr = rects_d(code->part, code->sub, rs);
-        for (int k = 0; k < nr; k++) {
-            const int bx = rs[k].x, by = rs[k].y;
-            for (int comp = 0; comp < 2; comp++) {
-                const uint32_t a = bx > 0 ? g[by * 4 + bx - 1][comp] : (la ? L.mvd[by * 4 + 3][comp] : 0);
-                const uint32_t b = by > 0 ? g[(by - 1) * 4 + bx][comp] : (ta ? T.mvd[12 + bx][comp] : 0);
-                mvd(c, comp, code->mvds[k][comp], a + b);
-            }
         }
     }
     if (kind != KIND_I16) {
@@ -529,53 +474,189 @@ __device__ __forceinline__ void head_bins(S& c, const Slice& sl, const ironav_mb
     c.decision(60, 0);  // mb_qp_delta 0, after a macroblock without a change
 }
 
-// mb_bins, enc/frame.rs:2028-2279, for I and P slices: the bins of the macroblock `code` up to
-// end_of_slice_flag (all of them, or one group's); l and t its left and top neighbours (avail 0: not in
-// the slice), nbm their Intra NxN modes as pred_mode reads them.
+// Residual block i (0..RES_BLOCKS - 1, in coding order) of a macroblock: 0 the Intra16x16 DC; 1..16 the luma blocks (4x4 in
+// decoding order, or 1..4 the 8x8 ones); 17, 18 chroma DC; 19..26 chroma AC.
+constexpr int RES_BLOCKS = 27;
 template <class S>
-__device__ __forceinline__ void mb_bins(S& c, const Slice& sl, const ironav_mbcode* code, const Nb& L, const Nb& T, const int* nbm, int group = ALL) {
+__device__ __forceinline__ void res_block(S& c, const ironav_mbcode* code, const Nb& L, const Nb& T, int i) {
     const bool la = L.avail, ta = T.avail;
-    if (sl.p_slice) {
-        if (group == ALL || group == HEAD) c.decision(11 + (la && !L.skip) + (ta && !T.skip), code->skip);
-        if (code->skip) return;
-    }
-    if (group == ALL || group == HEAD) head_bins(c, sl, code, L, T, nbm);
     const int kind = code->kind, cbp = code->res.cbp, cbpl = cbp & 15, cbpc = cbp >> 4;
-    if (!cbp && kind != KIND_I16) return;
     // an unavailable neighbour counts as a coded block for an intra macroblock
     const int un = kind != KIND_INTER;
-    int part;
-    if (kind == KIND_I16 && in_group(group, DC16_MAP, &part))
-        block(c, 0, 85 + (la ? (L.cbf_dc & 1) != 0 : un) + 2 * (ta ? (T.cbf_dc & 1) != 0 : un), code->dc, 16, part);
-    const int cat = kind == KIND_I16 ? 1 : 2, base = kind == KIND_I16 ? 89 : 93;
-    const bool luma = in_group(group, LUMA_MAP, &part);
-    if (code->res.t8x8 && luma) {
-        for (int i8 = 0; i8 < 4; i8++)
-            if (cbpl & (1 << i8)) block(c, 5, -1, code->res.luma8[i8], 64, part);
-    } else if (luma) {
-        for (int n = 0; n < 16; n++) {
-            if (!(cbpl & (1 << (n >> 2)))) continue;
+    int cat, cbf, max;
+    const int16_t* lv;
+    if (i == 0) {
+        if (kind != KIND_I16) return;
+        cat = 0, max = 16, lv = code->dc;
+        cbf = 85 + (la ? (L.cbf_dc & 1) != 0 : un) + 2 * (ta ? (T.cbf_dc & 1) != 0 : un);
+    } else if (i < 17) {
+        const int n = i - 1;
+        if (code->res.t8x8) {
+            if (n >= 4 || !(cbpl & (1 << n))) return;
+            cat = 5, cbf = -1, max = 64, lv = code->res.luma8[n];
+        } else {
+            if (!(cbpl & (1 << (n >> 2)))) return;
             const int bx = ((n >> 2) & 1) * 2 + (n & 1), by = ((n >> 3) & 1) * 2 + ((n >> 1) & 1);
             const int fa = bx > 0 ? code->res.nnz[by * 4 + bx - 1] > 0 : (la ? L.nnz[by * 4 + 3] > 0 : un);
             const int fb = by > 0 ? code->res.nnz[(by - 1) * 4 + bx] > 0 : (ta ? T.nnz[12 + bx] > 0 : un);
-            const int16_t* blk = code->res.luma[by * 4 + bx];
-            block(c, cat, base + fa + 2 * fb, cat == 1 ? blk + 1 : blk, cat == 1 ? 15 : 16, part);
+            const bool i16 = kind == KIND_I16;
+            cat = i16 ? 1 : 2, cbf = (i16 ? 89 : 93) + fa + 2 * fb, max = i16 ? 15 : 16;
+            lv = code->res.luma[by * 4 + bx] + (i16 ? 1 : 0);
         }
+    } else if (i < 19) {
+        if (cbpc == 0) return;
+        const int comp = i - 17, m = 2 << comp;
+        cat = 3, max = 4, lv = code->res.cdc[comp];
+        cbf = 97 + (la ? (L.cbf_dc & m) != 0 : un) + 2 * (ta ? (T.cbf_dc & m) != 0 : un);
+    } else {
+        if (cbpc != 2) return;
+        const int comp = (i - 19) >> 2, blk = (i - 19) & 3, bx = blk & 1, by = blk >> 1;
+        const uint8_t* cur = code->res.cnnz[comp];
+        const int fa = bx > 0 ? cur[by * 2] > 0 : (la ? L.cnnz[comp][by * 2 + 1] > 0 : un);
+        const int fb = by > 0 ? cur[bx] > 0 : (ta ? T.cnnz[comp][2 + bx] > 0 : un);
+        cat = 4, max = 15, lv = code->res.cac[comp][blk] + 1, cbf = 101 + fa + 2 * fb;
     }
-    if (cbpc > 0 && in_group(group, CDC_MAP, &part))
-        for (int comp = 0; comp < 2; comp++) {
-            const int m = 2 << comp;
-            block(c, 3, 97 + (la ? (L.cbf_dc & m) != 0 : un) + 2 * (ta ? (T.cbf_dc & m) != 0 : un), code->res.cdc[comp], 4, part);
+    block(c, cat, cbf, lv, max);
+}
+
+// mb_skip_flag of a P slice's macroblock.
+template <class S>
+__device__ __forceinline__ void skip_bin(S& c, const ironav_mbcode* code, const Nb& L, const Nb& T) {
+    c.decision(11 + (L.avail && !L.skip) + (T.avail && !T.skip), code->skip);
+}
+
+// The bins of a macroblock, mb_bins (enc/frame.rs:2028-2279) for I and P slices, are listed by a warp: a lane walks each piece (the
+// head's pieces, then the residual blocks, all independent given the code and its neighbours), once to count its bins and
+// once, at the offset a scan of the counts gives, to list them. (One lane walking a macroblock's bins one by one spent 40 us on a
+// coded macroblock's candidates and 49 us on writing an intra macroblock.) A listed bin: its context, bin << 10, and
+// whether it is a bypass (or, with both, a terminate) bin.
+constexpr uint32_t BIN_BYPASS = 1u << 11, BIN_TERMINATE = 1u << 12;
+
+// What a piece holds: its bins and, where only contexts are listed (the price), the cost of the others.
+struct PriceCount {
+    int n = 0;
+    uint32_t bits = 0;
+    __device__ __forceinline__ void decision(int, int) { n++; }
+    __device__ __forceinline__ void bypass(int) { bits += 256; }
+    __device__ __forceinline__ void terminate(int bin) { bits += bin ? 7 * 256 : 1; }
+};
+struct PriceList {
+    uint16_t* p;
+    __device__ __forceinline__ void decision(int ctx, int bin) { *p++ = (uint16_t)(ctx | (bin != 0) << 10); }
+    __device__ __forceinline__ void bypass(int) {}
+    __device__ __forceinline__ void terminate(int) {}
+};
+struct BinCount {
+    int n = 0;
+    __device__ __forceinline__ void decision(int, int) { n++; }
+    __device__ __forceinline__ void bypass(int) { n++; }
+    __device__ __forceinline__ void terminate(int) { n++; }
+};
+struct BinList {
+    uint16_t* p;
+    __device__ __forceinline__ void decision(int ctx, int bin) { *p++ = (uint16_t)(ctx | (bin != 0) << 10); }
+    __device__ __forceinline__ void bypass(int bin) { *p++ = (uint16_t)(BIN_BYPASS | (bin != 0) << 10); }
+    __device__ __forceinline__ void terminate(int bin) { *p++ = (uint16_t)(BIN_TERMINATE | (bin != 0) << 10); }
+};
+
+// This lane's two pieces of a macroblock's bins, in coding order over (piece, lane): the head (lane 0 the skip flag and
+// head_first, lanes 1-16 the parts, lane 17 head_last) and a residual block.
+template <class S>
+__device__ __forceinline__ void lane_head(S& c, const Slice& sl, const ironav_mbcode* code, const Nb& L, const Nb& T, const int* nbm) {
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) {
+        if (sl.p_slice) skip_bin(c, code, L, T);
+        if (!code->skip) head_first(c, sl, code, L, T);
+    } else if (!code->skip && lane <= 16) {
+        head_part(c, code, L, T, nbm, lane - 1);
+    } else if (!code->skip && lane == 17) {
+        head_last(c, sl, code, L, T);
+    }
+}
+template <class S>
+__device__ __forceinline__ void lane_block(S& c, const ironav_mbcode* code, const Nb& L, const Nb& T) {
+    const int lane = threadIdx.x & 31;
+    if (lane < RES_BLOCKS && !code->skip && (code->res.cbp || code->kind == KIND_I16)) res_block(c, code, L, T, lane);
+}
+
+// The exclusive prefix sum of v over the warp; the total on every lane.
+__device__ __forceinline__ int warp_scan(int v, int* total) {
+    const int lane = threadIdx.x & 31;
+    int x = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
+    }
+    *total = __shfl_sync(0xffffffffu, x, 31);
+    return x - v;
+}
+
+// Bins a price's list holds. A piece never has more (63 positions of an 8x8 block with two map bins each, 64 levels of at most 14
+// context bins); a macroblock's pieces that together do are listed in several turns.
+constexpr int PRICE_CAP = 1152;
+static_assert(2 * 63 + 64 * 14 <= PRICE_CAP, "one block fits the list");
+
+// The cost in 1/256 bits of the listed decisions, their contexts advanced in st (CabacCost, enc/cabac.rs:150-192). 32 bins a
+// turn, in order: the bins of a context form a chain, walked by its first lane, the contexts side by side.
+__device__ __forceinline__ uint32_t price_list(const uint16_t* list, int n, uint8_t* st, const uint32_t* step) {
+    const int lane = threadIdx.x & 31;
+    uint32_t bits = 0;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+        const bool in = i0 + lane < n;
+        const uint32_t e = in ? list[i0 + lane] : 0u;
+        const int ctx = in ? (int)(e & 1023u) : 1024 + lane;
+        uint32_t m = __match_any_sync(0xffffffffu, ctx);
+        const uint32_t ones = __ballot_sync(0xffffffffu, (e >> 10) & 1u);
+        if (in && (m & ((1u << lane) - 1u)) == 0) {
+            uint32_t s = st[ctx];
+            do {
+                const uint32_t v = step[s * 2 + ((ones >> (__ffs(m) - 1)) & 1u)];
+                m &= m - 1;
+                bits += v >> 8;
+                s = v & 0xffu;
+            } while (m);
+            st[ctx] = (uint8_t)s;
         }
-    if (cbpc == 2 && in_group(group, CAC_MAP, &part))
-        for (int comp = 0; comp < 2; comp++)
-            for (int blk = 0; blk < 4; blk++) {
-                const int bx = blk & 1, by = blk >> 1;
-                const uint8_t* cur = code->res.cnnz[comp];
-                const int fa = bx > 0 ? cur[by * 2] > 0 : (la ? L.cnnz[comp][by * 2 + 1] > 0 : un);
-                const int fb = by > 0 ? cur[bx] > 0 : (ta ? T.cnnz[comp][2 + bx] > 0 : un);
-                block(c, 4, 101 + fa + 2 * fb, code->res.cac[comp][blk] + 1, 15, part);
-            }
+        __syncwarp();
+    }
+    return bits;
+}
+
+// The bits of macroblock `code` (1/256 bits, on every lane) from the contexts `live`, and the contexts after it in st. list: PRICE_CAP
+// entries of the warp's own.
+__device__ __forceinline__ uint32_t price(const uint8_t* live, uint8_t* st, const uint32_t* step, uint16_t* list, const Slice& sl,
+                                          const ironav_mbcode* code, const Nb& L, const Nb& T, const int* nbm) {
+    const int lane = threadIdx.x & 31;
+    const uint4* s16 = reinterpret_cast<const uint4*>(live);
+    uint4* d16 = reinterpret_cast<uint4*>(st);
+    d16[lane] = s16[lane];
+    d16[lane + 32] = s16[lane + 32];
+    PriceCount h, r;
+    lane_head(h, sl, code, L, T, nbm);
+    lane_block(r, code, L, T);
+    int nh, nr;
+    const int oh = warp_scan(h.n, &nh), orr = nh + warp_scan(r.n, &nr), total = nh + nr;
+    uint32_t bits = h.bits + r.bits;
+    __syncwarp();
+    int base = 0;
+    do {
+        // the pieces that lie in [base, base + PRICE_CAP): a run of whole ones from base on
+        const bool fh = h.n && oh >= base && oh + h.n <= base + PRICE_CAP, fr = r.n && orr >= base && orr + r.n <= base + PRICE_CAP;
+        if (fh) {
+            PriceList c = {list + (oh - base)};
+            lane_head(c, sl, code, L, T, nbm);
+        }
+        if (fr) {
+            PriceList c = {list + (orr - base)};
+            lane_block(c, code, L, T);
+        }
+        const int end = __reduce_max_sync(0xffffffffu, max(fh ? oh + h.n : 0, fr ? orr + r.n : 0));
+        __syncwarp();
+        bits += price_list(list, end - base, st, step);
+        base = end;
+    } while (base < total);
+    return __reduce_add_sync(0xffffffffu, bits);
 }
 
 }  // namespace cab

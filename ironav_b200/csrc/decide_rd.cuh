@@ -3,14 +3,12 @@
 // slice writer.
 //
 // Under CABAC a macroblock's rate-distortion cost counts its bins against the slice's contexts as the
-// macroblocks before it left them, so a slice band is one chain in raster order: a warp walks a band (one
-// CTA a band, the bands side by side). For each macroblock the warp codes every candidate the reference
-// tries, in its order (P_Skip, best_inter's partitioning with the 4x4 and, with transform8, the 8x8
-// transform, Intra16x16, Intra4x4, Intra8x8, each intra one with its chroma), each into the picture and
-// then into shared memory (code and reconstruction), with its squared error; then the candidates' bins are
-// counted, each on its own copy of the contexts (the counter of cabac.cuh), a lane per group of disjoint
-// contexts (nine a candidate); lane 0 keeps the least SSD + lambda2 * bits in the reference's order (strict
-// '<'), and the warp copies the kept candidate's code, reconstruction and advanced contexts into place.
+// macroblocks before it left them, so a slice band is one chain in raster order: a CTA walks a band, one warp or (the wide form)
+// five. For each macroblock every candidate the reference tries is coded (P_Skip, best_inter's partitioning with the 4x4 and, with
+// transform8, the 8x8 transform, Intra16x16, Intra4x4, Intra8x8, each intra one with its chroma), into the picture or a scratch
+// plane and then into shared memory (code and reconstruction), with its squared error, and its bins are priced on its own copy
+// of the contexts (cab::price); the least SSD + lambda2 * bits in the reference's order (strict '<') is kept, and its code,
+// reconstruction and advanced contexts are copied into place.
 //
 // The candidates reuse decide mode's warp-level coders (decide.cuh, residual.cuh); Intra8x8 (code_i8,
 // enc/frame.rs:1307-1388) is coded here: block by block, its edges filtered (8.3.2.2.1), nine modes'
@@ -32,9 +30,9 @@ struct RdParams {
     double lam2;            // 1.6 * 2^((QP'Y - 12) / 3), computed on the host in f64 as the reference does
     int nbands;
     int t8;                 // transform_8x8_mode_flag
-    // the three-warp form: warps 1 and 2's scratch planes (luma, Cb, Cr of warp 1, then of warp 2), pw x ph and
-    // cw x ch samples, rows scr_ys and scr_cs samples apart
-    uint8_t* scr[6];
+    // the wide form: the scratch planes of warps 1 to 4 (luma, Cb, Cr of each), pw x ph and cw x ch samples, rows scr_ys
+    // and scr_cs samples apart
+    uint8_t* scr[12];
     int scr_ys, scr_cs;
 };
 
@@ -43,8 +41,9 @@ struct RdSmem {
     DecideSmem<T> s[W];              // each warp's working set
     ironav_mbcode cand[RD_CANDS];    // the candidates' codes
     T crec[RD_CANDS][384];           // and reconstructions (luma, Cb, Cr)
-    uint8_t live[1024];              // the chain's contexts after the macroblocks before this one
-    uint8_t cst[RD_CANDS][1024];     // each candidate's copy, advanced by its bins
+    __align__(16) uint8_t live[1024];           // the chain's contexts after the macroblocks before this one
+    __align__(16) uint8_t cst[RD_CANDS][1024];  // each candidate's copy, advanced by its bins
+    uint16_t list[W][cab::PRICE_CAP];           // each warp's list of bins
     uint32_t step[cab::STEP_ENTRIES];
     cab::Nb nb[2];                   // the left and top neighbours as the contexts see them
     cab::Nb done;                    // the macroblock just decided, the next one's left
@@ -54,9 +53,12 @@ struct RdSmem {
     unsigned bits[RD_CANDS];
     int valid[RD_CANDS];
     int best;
-    int skip;                        // the three-warp form: the P_Skip tests' verdict and the skip vector; the
-    int2 sv;                         // intra chroma's coded block pattern bits; best_inter's decision for the
-    uint32_t ccbp;                   // 8x8-transform candidate (warp 2), and whether that candidate is tried
+    // the wide form: of the macroblocks a group tests for P_Skip, the verdict, the skip vector and the top neighbour; the intra
+    // chroma's coded block pattern bits; best_inter's decision for the 8x8-transform candidate, and whether that is tried
+    int skip[W];
+    int2 sv[W];
+    cab::Nb top[W], nbs[W];          // (nbs: the P_Skip macroblocks' own)
+    uint32_t ccbp;
     uint16_t idec[40];
     int try_t8;
     // the Intra8x8 trial
@@ -384,34 +386,44 @@ __device__ __forceinline__ void rd_chroma_copy(const ironav_mbcode& from, ironav
     __syncwarp();
 }
 
-// Candidates k0 .. k0 + nk - 1 priced on this warp (rd_cost, enc/frame.rs:1453-1457): each from its own copy
-// of the contexts, a lane per (candidate, group of disjoint contexts), the groups' bits summed into R.bits.
-// coarse: five lanes a candidate, each residual category's map and levels on one lane (six candidates fit
-// the warp at once).
+// Candidate k priced on warp w (rd_cost, enc/frame.rs:1453-1457), from its own copy of the contexts.
 template <class T, int W>
-__device__ void rd_count(RdSmem<T, W>& R, const cab::Slice& sl, const int* nbm, int k0, int nk, bool coarse = false) {
+__device__ __forceinline__ void rd_price(RdSmem<T, W>& R, const cab::Slice& sl, const int* nbm, int k, int w) {
+    const uint32_t bits = cab::price(R.live, R.cst[k], R.step, R.list[w], sl, &R.cand[k], R.nb[0], R.nb[1], nbm);
+    if ((threadIdx.x & 31) == 0) R.bits[k] = bits;
+    __syncwarp();
+}
+
+// Intra candidate k's chroma: Intra16x16's code, reconstruction and squared error (the wide form; k's luma is coded).
+template <class T, int W>
+__device__ __forceinline__ void rd_take_chroma(RdSmem<T, W>& R, int k) {
     const int lane = threadIdx.x & 31;
-    for (int k = k0; k < k0 + nk; k++) {
-        if (!R.valid[k]) continue;
-        const uint32_t* s32 = reinterpret_cast<const uint32_t*>(R.live);
-        uint32_t* d32 = reinterpret_cast<uint32_t*>(R.cst[k]);
-        for (int i = lane; i < 256; i += 32) d32[i] = s32[i];
+    rd_chroma_copy(R.cand[3], &R.cand[k]);
+    if (lane == 0) {
+        R.cand[k].res.cbp |= (uint8_t)R.ccbp;
+        R.ssd[k] += R.cssd[3];
     }
-    if (lane < nk) R.bits[k0 + lane] = 0;
+    for (int i = 256 + lane; i < 384; i += 32) R.crec[k][i] = R.crec[3][i];
     __syncwarp();
-    const int ng = coarse ? (cab::NGROUPS + 1) / 2 : cab::NGROUPS;
-    const int k = k0 + lane / ng, g = lane % ng;
-    if (lane < nk * ng && R.valid[k]) {
-        cab::Counter c = {R.cst[k], R.step, 0};
-        if (!coarse || g == 0) {
-            cab::mb_bins(c, sl, &R.cand[k], R.nb[0], R.nb[1], nbm, g);
-        } else {
-            cab::mb_bins(c, sl, &R.cand[k], R.nb[0], R.nb[1], nbm, 2 * g - 1);
-            cab::mb_bins(c, sl, &R.cand[k], R.nb[0], R.nb[1], nbm, 2 * g);
-        }
-        if (c.bits) atomicAdd(&R.bits[k], c.bits);
+}
+
+// The candidate of least SSD + lam2 * bits, the first of them in the reference's order (strict '<'), in f64 rounded as the reference's
+// expression is (no fused multiply-add); on every lane.
+template <class T, int W>
+__device__ __forceinline__ int rd_best(const RdParams& P, const RdSmem<T, W>& R) {
+    const int lane = threadIdx.x & 31;
+    const bool in = lane < RD_CANDS && R.valid[lane < RD_CANDS ? lane : 0];
+    double j = 0.0;
+    if (in) j = __dadd_rn(__ll2double_rn(R.ssd[lane]), __dmul_rn(P.lam2, __dmul_rn((double)R.bits[lane], 0.00390625)));
+    const unsigned valid = __ballot_sync(FULL, in);
+    int best = -1;
+    double bj = 0.0;
+#pragma unroll
+    for (int k = 0; k < RD_CANDS; k++) {
+        const double jk = __shfl_sync(FULL, j, k);
+        if (((valid >> k) & 1u) && (best < 0 || jk < bj)) best = k, bj = jk;
     }
-    __syncwarp();
+    return best;
 }
 
 // The MbState of a coded candidate: the inter ones' from inter_tail (S.a.out), the intra ones' without motion.
@@ -458,7 +470,7 @@ __device__ void rd_mb(const RdParams& P, RdSmem<T, 1>& R, const unsigned* i4tab,
         // P_Skip without a rate-distortion choice; its one bin still moves the contexts
         if (lane == 0) {
             cab::Counter c = {R.live, R.step, 0};
-            cab::mb_bins(c, sl, out, R.nb[0], R.nb[1], S.nbm);
+            cab::skip_bin(c, out, R.nb[0], R.nb[1]);
         }
         if (lane < 18) reinterpret_cast<uint32_t*>(&A.states_out[mb])[lane] = reinterpret_cast<const uint32_t*>(&S.a.out)[lane];
         __syncwarp();
@@ -606,22 +618,9 @@ __device__ void rd_mb(const RdParams& P, RdSmem<T, 1>& R, const unsigned* i4tab,
         rd_state(R, S, 5, false);
         rd_take(C, R, S, 5, mbx, mby);
     }
-    // rd_cost (1453-1457): the candidates priced at once (five lanes each); then lane 0 keeps the least SSD +
-    // lam2 * bits in the reference's order (strict '<'), in f64 rounded as the reference's expression is (no
-    // fused multiply-add).
-    rd_count(R, sl, S.nbm, 0, RD_CANDS, true);
-    if (lane == 0) {
-        int best = -1;
-        double bj = 0.0;
-        for (int k = 0; k < RD_CANDS; k++) {
-            if (!R.valid[k]) continue;
-            const double j = __dadd_rn(__ll2double_rn(R.ssd[k]), __dmul_rn(P.lam2, __dmul_rn((double)R.bits[k], 0.00390625)));
-            if (best < 0 || j < bj) best = k, bj = j;
-        }
-        R.best = best;
-    }
-    __syncwarp();
-    const int b = R.best;
+    for (int k = 0; k < RD_CANDS; k++)
+        if (R.valid[k]) rd_price(R, sl, S.nbm, k, 0);
+    const int b = rd_best(P, R);
     {
         const uint32_t* s32 = reinterpret_cast<const uint32_t*>(&cand[b]);
         uint32_t* d32 = reinterpret_cast<uint32_t*>(out);
@@ -698,151 +697,175 @@ __global__ void __launch_bounds__(32) decide_rd_batch_kernel(const RdParams* __r
     rd_chain<T>(prm, R, i4tab, (int)(e & 0xFFFFu));
 }
 
-// ---- the three-warp form: one chain's macroblock on three warps ----------------------------------------
-// Warp 0 runs code_mb's P_Skip tests; when the macroblock passes them, warp 0 runs best_inter and codes its
-// partitioning with the 4x4 transform into the picture, warp 1 codes P_Skip, Intra4x4 and Intra8x8, and warp 2
-// Intra16x16 (with the intra chroma) and then the partitioning with the 8x8 transform (best_inter's
-// decision handed over through named barrier 1, which warp 0 arrives at and warp 2 waits on), warps 1 and
-// 2 each into their own scratch planes (their edges read from the picture, which warp 0 writes only inside
-// the macroblock). The three warps then price two candidates each, and warp 0 commits the kept one. The
-// warps meet at CTA barriers (after the P_Skip tests; when there are candidates, after them and after the
-// pricing; after the commit), every warp at every one.
-constexpr int RD3_WARPS = 3;
+// ---- the wide form: one chain on five warps -------------------------------------------------------------
+// Few chains leave the chip idle, and a chain's time is the picture's, so each gets five warps:
+//   - the P_Skip tests of five macroblocks at once (warp i the i-th, on the assumption that those before it in the group are
+//     P_Skip: their states are then their skip vectors, a chain of a few instructions each). The leading ones that pass are
+//     P_Skip, and the test of the first that does not pass is good too. Tested one by one, the P_Skip macroblocks (most of a P
+//     picture's) took 12 us each;
+//   - the candidates of a macroblock that does not pass, side by side: warp 0 best_inter and its partitioning with the 4x4
+//     transform, into the picture; warp 4 P_Skip and then the partitioning with the 8x8 transform (best_inter's decision
+//     handed over through named barrier 1); warp 1 Intra4x4, warp 2 Intra16x16 with the intra chroma, and warp 3 Intra8x8
+//     (the chroma handed over through named barrier 2), warps 1 to 4 each into their own scratch planes (their edges read
+//     from the picture, which warp 0 writes only inside the macroblock). Each warp prices what it coded;
+//   - the commit of the kept one (code, reconstruction, contexts, state) by a warp each.
+// The warps meet at CTA barriers (after the tests; after the P_Skip macroblocks' commits; and, when there are candidates, after
+// them and after the commit), every warp at every one. An IDR and three P pictures at 1080p, 8 bands: 248 ms with three warps a
+// chain (P_Skip tested one macroblock at a time, each candidate's bins walked by nine lanes), 138 ms in this form.
+constexpr int RDW_WARPS = 5;
 
+// skip_mv (enc/frame.rs:597-603) from a macroblock's table of neighbours, with its left neighbour's block a.
+__device__ __forceinline__ int2 skip_mv_from(const Blk* ext, const Blk& a) {
+    const Blk b = ext[1];
+    Blk c = ext[5];
+    if (!c.w) c = ext[0];
+    if (!a.w || !b.w || (a.z == 0 && a.x == 0 && a.y == 0) || (b.z == 0 && b.x == 0 && b.y == 0)) return make_int2(0, 0);
+    const int ra = a.z == 0, rb = b.z == 0, rc = c.z == 0;
+    if (ra + rb + rc == 1) return ra ? make_int2(a.x, a.y) : (rb ? make_int2(b.x, b.y) : make_int2(c.x, c.y));
+    return make_int2(median3_d(a.x, b.x, c.x), median3_d(a.y, b.y, c.y));
+}
+
+// The next macroblocks of the chain from (mbx0, mby) on: returns how many were decided (1 to RDW_WARPS).
 template <class T>
-__device__ void rd_mb3(const RdParams& P, const DecideParams* dw, RdSmem<T, RD3_WARPS>& R, const unsigned* i4tab, int mb, int mbx,
-                       int mby) {
+__device__ int rd_group(const RdParams& P, const DecideParams* dw, RdSmem<T, RDW_WARPS>& R, const unsigned* i4tab, int mbx0, int mby) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const DecideParams& D = P.D;
     const AnalyseParams& A = D.C.A;
     const CodeParams& C = D.C;
     DecideSmem<T>& S = R.s[w];
-    const bool ta = mby > A.band_start[mby], la = mbx > 0, tra = ta && mbx + 1 < A.mb_w;
+    const bool ta = mby > A.band_start[mby];
     const cab::Slice sl = {D.intra ? 0 : 1, P.t8, D.intra ? 0 : A.nact};
-    ironav_mbcode* out = &D.codes[mb];
     ironav_mbcode* cand = R.cand;
-    if (lane == 0) {
-        S.a.mb = mb;
-        S.a.mbx = mbx;
-        S.a.mby = mby;
-    }
-    __syncwarp();
-    stage_source(A, S.a);
-    int2 sv = make_int2(0, 0);
-    if (w == 0) {
-        load_neighbours(A, S.a, A.states_out);
-        code_init(out);
-        if (lane < cab::NB_WORDS) {
-            reinterpret_cast<uint32_t*>(&R.nb[0])[lane] = la ? reinterpret_cast<const uint32_t*>(&R.done)[lane] : 0u;
-            reinterpret_cast<uint32_t*>(&R.nb[1])[lane] = ta ? P.nbs[(size_t)(mb - A.mb_w) * cab::NB_WORDS + lane] : 0u;
-        }
-        if (lane < RD_CANDS) R.valid[lane] = 0;
-        __syncwarp();
-        const bool skip = !D.intra && skip_tests_d<T>(D, S, mb, mbx, mby, out, &sv);
+    const int mb0 = mby * A.mb_w + mbx0, n = D.intra ? 0 : min(RDW_WARPS, A.mb_w - mbx0);
+    const bool la0 = mbx0 > 0, left_skip = la0 && R.done.skip;
+    auto copy_nb = [&](cab::Nb* d, const cab::Nb* s) {  // zeros when s is nullptr
+        if (lane < cab::NB_WORDS) reinterpret_cast<uint32_t*>(d)[lane] = s ? reinterpret_cast<const uint32_t*>(s)[lane] : 0u;
+    };
+    auto begin = [&](int x) {
         if (lane == 0) {
-            R.skip = skip;
-            R.sv = sv;
+            S.a.mb = mby * A.mb_w + x;
+            S.a.mbx = x;
+            S.a.mby = mby;
         }
+        __syncwarp();
+        stage_source(A, S.a);
+    };
+    if (w < n) {
+        begin(mbx0 + w);
+        load_neighbours(A, S.a, A.states_out);
+        copy_nb(&R.top[w], ta ? reinterpret_cast<const cab::Nb*>(P.nbs + (size_t)(mb0 + w - A.mb_w) * cab::NB_WORDS) : nullptr);
+    } else if (n == 0 && w == 0) {
+        copy_nb(&R.top[0], ta ? reinterpret_cast<const cab::Nb*>(P.nbs + (size_t)(mb0 - A.mb_w) * cab::NB_WORDS) : nullptr);
+    }
+    __syncthreads();  // every macroblock's table of neighbours
+    if (w < n) {
+        ironav_mbcode* out = &D.codes[mb0 + w];
+        if (w > 0) {
+            // the left neighbour is P_Skip by assumption, with the vector that the same assumption gives it (only the
+            // tables' rows above are read from other warps, and only the left column is changed here)
+            int2 sv = skip_mv_from(R.s[0].a.ext, R.s[0].a.ext[6]);
+            for (int j = 1; j < w; j++) sv = skip_mv_from(R.s[j].a.ext, make_int4(sv.x, sv.y, 0, 1));
+            if (lane < 4) S.a.ext[(lane + 1) * 6] = make_int4(sv.x, sv.y, 0, 1);
+        }
+        code_init(out);
+        int2 sv = make_int2(0, 0);
+        const bool skip = skip_tests_d<T>(D, S, mb0 + w, mbx0 + w, mby, out, &sv);
+        if (lane == 0) {
+            R.skip[w] = skip;
+            R.sv[w] = sv;
+        }
+    }
+    if (n > 0) __syncthreads();  // the verdicts
+    int m = 0;
+    while (m < n && R.skip[m]) m++;
+    // the leading P_Skip macroblocks, and the neighbours of the one after them
+    if (w < m) {
+        const ironav_mbcode* out = &D.codes[mb0 + w];
+        if (lane < 18) reinterpret_cast<uint32_t*>(&A.states_out[mb0 + w])[lane] = reinterpret_cast<const uint32_t*>(&S.a.out)[lane];
+        cab::Nb* nb = w == m - 1 ? &R.done : &R.nbs[w];
+        cab::nb_of_warp(out, nb);
+        if (lane < cab::NB_WORDS) P.nbs[(size_t)(mb0 + w) * cab::NB_WORDS + lane] = reinterpret_cast<const uint32_t*>(nb)[lane];
+        if (w == m - 1) copy_nb(&R.nb[0], nb);
+    }
+    if (w == 0 && lane == 0) {
+        // their one bin each still moves the contexts (mb_skip_flag; the left one of all but the first is P_Skip)
+        for (int j = 0; j < m; j++) {
+            const int ctx = 11 + (j == 0 && la0 && !left_skip) + (R.top[j].avail && !R.top[j].skip);
+            R.live[ctx] = (uint8_t)R.step[R.live[ctx] * 2 + 1];
+        }
+    }
+    if (m < n || n == 0) {
+        if (w == RDW_WARPS - 1) {
+            copy_nb(&R.nb[1], &R.top[m]);
+            if (lane < RD_CANDS) R.valid[lane] = 0;
+        }
+        if (w == 0 && m == 0) copy_nb(&R.nb[0], la0 ? &R.done : nullptr);
     }
     __syncthreads();
-    if (R.skip) {
-        if (w == 0) {
-            // P_Skip without a rate-distortion choice; its one bin still moves the contexts
-            if (lane == 0) {
-                cab::Counter c = {R.live, R.step, 0};
-                cab::mb_bins(c, sl, out, R.nb[0], R.nb[1], S.nbm);
-            }
-            if (lane < 18) reinterpret_cast<uint32_t*>(&A.states_out[mb])[lane] = reinterpret_cast<const uint32_t*>(&S.a.out)[lane];
-            __syncwarp();
-            cab::nb_of_warp(out, &R.done);
-            if (lane < cab::NB_WORDS) P.nbs[(size_t)mb * cab::NB_WORDS + lane] = reinterpret_cast<const uint32_t*>(&R.done)[lane];
-            __syncwarp();
-        }
-        __syncthreads();
-        return;
-    }
-    load_intra_neighbours(D, S, mb, mbx, mby, ta, la, tra);
-    if (w == 0 && !D.intra) {
-        // best_inter, enc/frame.rs:839-849; its decision goes to warp 2 (the 8x8-transform candidate) through
-        // named barrier 1, and warp 0 codes it with the 4x4 transform
-        int part = 0, cost = BIG, bestr = 0;
-        uint32_t sub = 0;
-        for (int r = 0; r < A.nact; r++) {
-            const int4 bi = best_inter_or_learned(A, S.a, r);
-            if (r == 0 || bi.x < cost) {
-                part = bi.y;
-                cost = bi.x;
-                bestr = r;
-                sub = (uint32_t)bi.z;
-                if (lane < 16) {
-                    S.a.win_mvs[lane][0] = S.a.best_mvs[lane][0];
-                    S.a.win_mvs[lane][1] = S.a.best_mvs[lane][1];
-                }
-                __syncwarp();
-            }
-        }
-        ironav_interdec& Dd = *reinterpret_cast<ironav_interdec*>(S.c.dec);
-        if (lane == 0) {
-            Dd.mode = 2;
-            Dd.part = (uint8_t)part;
-            Dd.t8 = 0;
-            for (int k = 0; k < 4; k++) {
-                Dd.sub[k] = (uint8_t)((sub >> (8 * k)) & 0xff);
-                Dd.refs[k] = (uint8_t)bestr;
-            }
-            R.try_t8 = P.t8 && sub == 0;
-        }
-        if (lane < 16) {
-            Dd.mvs[lane][0] = S.a.win_mvs[lane][0];
-            Dd.mvs[lane][1] = S.a.win_mvs[lane][1];
-        }
-        __syncwarp();
-        if (P.t8) {
-            for (int i = lane; i < 40; i += 32) R.idec[i] = S.c.dec[i];
-            __threadfence_block();
-            __syncwarp();
-            asm volatile("bar.arrive 1, 64;" ::: "memory");
-        }
-        ironav_mbcode* o = &cand[1];
-        code_init(o);
-        const uint32_t cbp = code_inter_mb<T>(C, S.c, mb, &o->res);
-        inter_tail(D, S, Dd, o);
-        rd_state(R, S, 1, true);
-        rd_take(C, R, S, 1, mbx, mby);
-        const int2 sv = R.sv;
-        if (lane == 0 && cbp == 0 && part == 0 && Dd.mvs[0][0] == sv.x && Dd.mvs[0][1] == sv.y && bestr == 0) R.valid[1] = 0;
-        __syncwarp();
-    } else if (w == 1) {
-        const DecideParams& Dw = dw[0];
+    if (n > 0 && m == n) return n;
+    // the candidates of macroblock mb
+    const int mb = mb0 + m, mbx = mbx0 + m;
+    const bool la = mbx > 0, tra = ta && mbx + 1 < A.mb_w;
+    begin(mbx);
+    __syncwarp();
+    if (w == 0) {
         if (!D.intra) {
-            // P_Skip: the skip vector's prediction is the reconstruction (put_inter_pred, 1391-1394), into warp
-            // 1's planes; a P_Skip code carries no differences, its state the vector over the macroblock
-            const int2 sv = R.sv;
-            ironav_mbcode* o = &cand[0];
-            code_init(o);
+            // best_inter, enc/frame.rs:839-849
+            load_neighbours(A, S.a, A.states_out);
+            int part = 0, cost = BIG, bestr = 0;
+            uint32_t sub = 0;
+            for (int r = 0; r < A.nact; r++) {
+                const int4 bi = best_inter_or_learned(A, S.a, r);
+                if (r == 0 || bi.x < cost) {
+                    part = bi.y;
+                    cost = bi.x;
+                    bestr = r;
+                    sub = (uint32_t)bi.z;
+                    if (lane < 16) {
+                        S.a.win_mvs[lane][0] = S.a.best_mvs[lane][0];
+                        S.a.win_mvs[lane][1] = S.a.best_mvs[lane][1];
+                    }
+                    __syncwarp();
+                }
+            }
             ironav_interdec& Dd = *reinterpret_cast<ironav_interdec*>(S.c.dec);
             if (lane == 0) {
-                Dd.mode = 1;
-                Dd.part = 0;
+                Dd.mode = 2;
+                Dd.part = (uint8_t)part;
                 Dd.t8 = 0;
-                for (int k = 0; k < 4; k++) Dd.sub[k] = Dd.refs[k] = 0;
-                o->kind = KIND_INTER;
-                o->skip = 1;
+                for (int k = 0; k < 4; k++) {
+                    Dd.sub[k] = (uint8_t)((sub >> (8 * k)) & 0xff);
+                    Dd.refs[k] = (uint8_t)bestr;
+                }
+                R.try_t8 = P.t8 && sub == 0;
             }
             if (lane < 16) {
-                Dd.mvs[lane][0] = (int16_t)sv.x;
-                Dd.mvs[lane][1] = (int16_t)sv.y;
-                o->mvs[lane][0] = (int16_t)sv.x;
-                o->mvs[lane][1] = (int16_t)sv.y;
+                Dd.mvs[lane][0] = S.a.win_mvs[lane][0];
+                Dd.mvs[lane][1] = S.a.win_mvs[lane][1];
             }
             __syncwarp();
-            code_inter_mb<T>(Dw.C, S.c, mb, &o->res);
-            uint32_t* d = reinterpret_cast<uint32_t*>(&R.state[0]);
-            if (lane < 18) d[lane] = lane == 0 ? 1u : (lane == 1 ? 0u : ((uint32_t)(uint16_t)sv.x | (uint32_t)(uint16_t)sv.y << 16));
+            if (P.t8) {
+                for (int i = lane; i < 40; i += 32) R.idec[i] = S.c.dec[i];
+                __threadfence_block();
+                __syncwarp();
+                asm volatile("bar.arrive 1, 64;" ::: "memory");
+            }
+            ironav_mbcode* o = &cand[1];
+            code_init(o);
+            const uint32_t cbp = code_inter_mb<T>(C, S.c, mb, &o->res);
+            inter_tail(D, S, Dd, o);
+            rd_state(R, S, 1, true);
+            rd_take(C, R, S, 1, mbx, mby);
+            // with nothing coded and the skip vector, it would be P_Skip at a higher price
+            const int2 sv = R.sv[m];
+            if (lane == 0 && cbp == 0 && part == 0 && Dd.mvs[0][0] == sv.x && Dd.mvs[0][1] == sv.y && bestr == 0) R.valid[1] = 0;
             __syncwarp();
-            rd_take(Dw.C, R, S, 0, mbx, mby);
+            if (R.valid[1]) rd_price(R, sl, S.nbm, 1, w);
         }
-        // Intra4x4 into warp 1's luma plane; its chroma is Intra16x16's (taken after the barrier)
+    } else if (w == 1) {
+        // Intra4x4 into warp 1's luma plane, with Intra16x16's chroma
+        const DecideParams& Dw = dw[0];
+        load_intra_neighbours(D, S, mb, mbx, mby, ta, la, tra);
         ironav_mbcode* o = &cand[4];
         code_init(o);
         code_i4_trial(Dw, S, i4tab, ta, la, tra);
@@ -867,18 +890,13 @@ __device__ void rd_mb3(const RdParams& P, const DecideParams* dw, RdSmem<T, RD3_
         }
         rd_state(R, S, 4, false);
         rd_take(Dw.C, R, S, 4, mbx, mby, false);
-        if (P.t8) {
-            // Intra8x8 into warp 1's luma plane (its edges from the picture); its chroma too is Intra16x16's
-            o = &cand[5];
-            code_init(o);
-            const uint32_t cbp8 = code_i8_d(D, S, R, mbx, mby, ta, la, tra, o, reinterpret_cast<T*>(Dw.C.rec[0]), Dw.C.ys);
-            if (lane == 0) o->res.cbp = (uint8_t)cbp8;
-            rd_state(R, S, 5, false);
-            rd_take(Dw.C, R, S, 5, mbx, mby, false);
-        }
+        asm volatile("bar.sync 2, 96;" ::: "memory");
+        rd_take_chroma(R, 4);
+        rd_price(R, sl, S.nbm, 4, w);
     } else if (w == 2) {
-        // Intra16x16 in best_i16's mode with the intra chroma, then Intra8x8, into warp 2's planes
+        // Intra16x16 in best_i16's mode with the intra chroma, into warp 2's planes
         const DecideParams& Dw = dw[1];
+        load_intra_neighbours(D, S, mb, mbx, mby, ta, la, tra);
         const int2 i16 = best_i16_d(Dw, S, ta, la);
         ironav_mbcode* o = &cand[3];
         code_init(o);
@@ -893,15 +911,64 @@ __device__ void rd_mb3(const RdParams& P, const DecideParams* dw, RdSmem<T, RD3_
         }
         rd_state(R, S, 3, false);
         rd_take(Dw.C, R, S, 3, mbx, mby);
-        if (P.t8 && !D.intra) {
+        __threadfence_block();
+        __syncwarp();
+        asm volatile("bar.arrive 2, 96;" ::: "memory");
+        rd_price(R, sl, S.nbm, 3, w);
+    } else if (w == 3) {
+        // Intra8x8 into warp 3's luma plane (its edges from the picture), with Intra16x16's chroma
+        const DecideParams& Dw = dw[2];
+        if (P.t8) {
+            load_intra_neighbours(D, S, mb, mbx, mby, ta, la, tra);
+            ironav_mbcode* o = &cand[5];
+            code_init(o);
+            const uint32_t cbp = code_i8_d(D, S, R, mbx, mby, ta, la, tra, o, reinterpret_cast<T*>(Dw.C.rec[0]), Dw.C.ys);
+            if (lane == 0) o->res.cbp = (uint8_t)cbp;
+            rd_state(R, S, 5, false);
+            rd_take(Dw.C, R, S, 5, mbx, mby, false);
+        }
+        asm volatile("bar.sync 2, 96;" ::: "memory");
+        if (P.t8) {
+            rd_take_chroma(R, 5);
+            rd_price(R, sl, S.nbm, 5, w);
+        }
+    } else if (!D.intra) {
+        // P_Skip: the skip vector's prediction is the reconstruction (put_inter_pred, 1391-1394), into warp 4's
+        // planes; a P_Skip code carries no differences, its state the vector over the macroblock
+        const DecideParams& Dw = dw[3];
+        const int2 sv = R.sv[m];
+        ironav_mbcode* o = &cand[0];
+        code_init(o);
+        ironav_interdec& Dd = *reinterpret_cast<ironav_interdec*>(S.c.dec);
+        if (lane == 0) {
+            Dd.mode = 1;
+            Dd.part = 0;
+            Dd.t8 = 0;
+            for (int k = 0; k < 4; k++) Dd.sub[k] = Dd.refs[k] = 0;
+            o->kind = KIND_INTER;
+            o->skip = 1;
+        }
+        if (lane < 16) {
+            Dd.mvs[lane][0] = (int16_t)sv.x;
+            Dd.mvs[lane][1] = (int16_t)sv.y;
+            o->mvs[lane][0] = (int16_t)sv.x;
+            o->mvs[lane][1] = (int16_t)sv.y;
+        }
+        __syncwarp();
+        code_inter_mb<T>(Dw.C, S.c, mb, &o->res);
+        uint32_t* d = reinterpret_cast<uint32_t*>(&R.state[0]);
+        if (lane < 18) d[lane] = lane == 0 ? 1u : (lane == 1 ? 0u : ((uint32_t)(uint16_t)sv.x | (uint32_t)(uint16_t)sv.y << 16));
+        __syncwarp();
+        rd_take(Dw.C, R, S, 0, mbx, mby);
+        rd_price(R, sl, S.nbm, 0, w);
+        if (P.t8) {
             // best_inter's partitioning with the 8x8 transform (when no 8x8 block is split; without luma levels it
             // would be the 4x4 candidate again), once warp 0 has handed its decision over
+            load_neighbours(A, S.a, A.states_out);
             asm volatile("bar.sync 1, 64;" ::: "memory");
             if (R.try_t8) {
-                load_neighbours(A, S.a, A.states_out);
                 for (int i = lane; i < 40; i += 32) S.c.dec[i] = R.idec[i];
                 __syncwarp();
-                ironav_interdec& Dd = *reinterpret_cast<ironav_interdec*>(S.c.dec);
                 if (lane == 0) Dd.t8 = 1;
                 __syncwarp();
                 o = &cand[2];
@@ -912,68 +979,44 @@ __device__ void rd_mb3(const RdParams& P, const DecideParams* dw, RdSmem<T, RD3_
                 rd_take(Dw.C, R, S, 2, mbx, mby);
                 if (lane == 0 && !o->res.t8x8) R.valid[2] = 0;
                 __syncwarp();
+                if (R.valid[2]) rd_price(R, sl, S.nbm, 2, w);
             }
         }
     }
     __syncthreads();
-    // the candidates priced two a warp (warp 2 first gives Intra4x4 and Intra8x8 Intra16x16's chroma: code,
-    // reconstruction and squared error), then warp 0 keeps the least cost in order and commits it
-    if (w == 2) {
-        for (int k = 4; k <= (P.t8 ? 5 : 4); k++) {
-            rd_chroma_copy(cand[3], &cand[k]);
-            if (lane == 0) {
-                cand[k].res.cbp |= (uint8_t)R.ccbp;
-                R.ssd[k] += R.cssd[3];
-                R.cssd[k] = R.cssd[3];
-            }
-            for (int i = 256 + lane; i < 384; i += 32) R.crec[k][i] = R.crec[3][i];
-            __syncwarp();
-        }
-    }
-    rd_count(R, sl, S.nbm, 2 * w, 2);
-    __syncthreads();
+    // the least cost in order, and its commit
+    const int b = rd_best(P, R);
     if (w == 0) {
-        if (lane == 0) {
-            int best = -1;
-            double bj = 0.0;
-            for (int k = 0; k < RD_CANDS; k++) {
-                if (!R.valid[k]) continue;
-                const double j = __dadd_rn(__ll2double_rn(R.ssd[k]), __dmul_rn(P.lam2, __dmul_rn((double)R.bits[k], 0.00390625)));
-                if (best < 0 || j < bj) best = k, bj = j;
-            }
-            R.best = best;
-        }
-        __syncwarp();
-        const int b = R.best;
-        const uint32_t* s32 = reinterpret_cast<const uint32_t*>(&cand[b]);
-        uint32_t* d32 = reinterpret_cast<uint32_t*>(out);
-        for (int i = lane; i < (int)(sizeof(ironav_mbcode) / 4); i += 32) d32[i] = s32[i];
-        const uint32_t* c32 = reinterpret_cast<const uint32_t*>(R.cst[b]);
-        uint32_t* l32 = reinterpret_cast<uint32_t*>(R.live);
-        for (int i = lane; i < 256; i += 32) l32[i] = c32[i];
-        const T* rec = R.crec[b];
-        for (int i = lane; i < 384; i += 32) {
-            if (i < 256) {
-                reinterpret_cast<T*>(C.rec[0])[(size_t)(mby * 16 + (i >> 4)) * C.ys + mbx * 16 + (i & 15)] = rec[i];
-            } else {
-                const int cc = (i - 256) >> 6, j = (i - 256) & 63;
-                reinterpret_cast<T*>(C.rec[1 + cc])[(size_t)(mby * 8 + (j >> 3)) * C.cs + mbx * 8 + (j & 7)] = rec[i];
-            }
-        }
         if (lane < 18) reinterpret_cast<uint32_t*>(&A.states_out[mb])[lane] = reinterpret_cast<const uint32_t*>(&R.state[b])[lane];
-        __syncwarp();
         cab::nb_of_warp(&cand[b], &R.done);
         if (lane < cab::NB_WORDS) P.nbs[(size_t)mb * cab::NB_WORDS + lane] = reinterpret_cast<const uint32_t*>(&R.done)[lane];
-        __syncwarp();
+    } else if (w == 1) {
+        const uint32_t* s32 = reinterpret_cast<const uint32_t*>(&cand[b]);
+        uint32_t* d32 = reinterpret_cast<uint32_t*>(&D.codes[mb]);
+        for (int i = lane; i < (int)(sizeof(ironav_mbcode) / 4); i += 32) d32[i] = s32[i];
+    } else if (w == 2) {
+        const T* rec = R.crec[b];
+        for (int i = lane; i < 256; i += 32) reinterpret_cast<T*>(C.rec[0])[(size_t)(mby * 16 + (i >> 4)) * C.ys + mbx * 16 + (i & 15)] = rec[i];
+    } else if (w == 3) {
+        const T* rec = R.crec[b] + 256;
+        for (int i = lane; i < 128; i += 32) {
+            const int cc = i >> 6, j = i & 63;
+            reinterpret_cast<T*>(C.rec[1 + cc])[(size_t)(mby * 8 + (j >> 3)) * C.cs + mbx * 8 + (j & 7)] = rec[i];
+        }
+    } else {
+        const uint4* c16 = reinterpret_cast<const uint4*>(R.cst[b]);
+        uint4* l16 = reinterpret_cast<uint4*>(R.live);
+        l16[lane] = c16[lane];
+        l16[lane + 32] = c16[lane + 32];
     }
     __syncthreads();
+    return m + 1;
 }
 
-// The three-warp form's set-up and chain walk for the parameters P (in parameter space or shared memory):
-// warps 1 and 2's parameter copies writing into their scratch planes, the CTA's tables and contexts, then
-// slice band `band` in raster order.
+// The wide form's set-up and chain walk for the parameters P (in parameter space or shared memory): warps 1 to 4's parameter
+// copies writing into their scratch planes, the CTA's tables and contexts, then slice band `band` in raster order.
 template <class T>
-__device__ void rd3_chain(const RdParams& P, DecideParams* dw, RdSmem<T, RD3_WARPS>& R, unsigned* i4tab, int band) {
+__device__ void rdw_chain(const RdParams& P, DecideParams* dw, RdSmem<T, RDW_WARPS>& R, unsigned* i4tab, int band) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (w > 0) {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(&P.D);
@@ -993,38 +1036,38 @@ __device__ void rd3_chain(const RdParams& P, DecideParams* dw, RdSmem<T, RD3_WAR
     cab::init_states(R.live, P.D.intra != 0, 0, P.D.C.qp, threadIdx.x, blockDim.x);
     __syncthreads();
     for (int mby = P.band_rows[band]; mby < P.band_rows[band + 1]; mby++)
-        for (int mbx = 0; mbx < A.mb_w; mbx++) rd_mb3<T>(P, dw, R, i4tab, mby * A.mb_w + mbx, mbx, mby);
+        for (int mbx = 0; mbx < A.mb_w;) mbx += rd_group<T>(P, dw, R, i4tab, mbx, mby);
 }
 
-// Decide mode under CABAC for one stream, three warps a chain: CTA i walks slice band i.
+// Decide mode under CABAC for one stream in the wide form: CTA i walks slice band i.
 template <class T>
-__global__ void __launch_bounds__(RD3_WARPS * 32) decide_rd3_kernel(const __grid_constant__ RdParams P) {
-    extern __shared__ __align__(16) unsigned char rd3_smem[];
-    __shared__ DecideParams dw[2];
+__global__ void __launch_bounds__(RDW_WARPS * 32) decide_rdw_kernel(const __grid_constant__ RdParams P) {
+    extern __shared__ __align__(16) unsigned char rdw_smem[];
+    __shared__ DecideParams dw[RDW_WARPS - 1];
     __shared__ unsigned i4tab[9 * 17];
     if ((int)blockIdx.x >= P.nbands) return;
-    rd3_chain<T>(P, dw, *reinterpret_cast<RdSmem<T, RD3_WARPS>*>(rd3_smem), i4tab, blockIdx.x);
+    rdw_chain<T>(P, dw, *reinterpret_cast<RdSmem<T, RDW_WARPS>*>(rdw_smem), i4tab, blockIdx.x);
 }
 
 // The same for many streams' chains: CTA i walks chains[i] = stream << 16 | band with the stream's
 // parameters from table[stream] (copied into shared memory).
 template <class T>
-__global__ void __launch_bounds__(RD3_WARPS * 32) decide_rd3_batch_kernel(const RdParams* __restrict__ table,
+__global__ void __launch_bounds__(RDW_WARPS * 32) decide_rdw_batch_kernel(const RdParams* __restrict__ table,
                                                                           const uint32_t* __restrict__ chains, int nchains) {
-    extern __shared__ __align__(16) unsigned char rd3_smem[];
+    extern __shared__ __align__(16) unsigned char rdw_smem[];
     __shared__ RdParams prm;
-    __shared__ DecideParams dw[2];
+    __shared__ DecideParams dw[RDW_WARPS - 1];
     __shared__ unsigned i4tab[9 * 17];
     if ((int)blockIdx.x >= nchains) return;
     const uint32_t e = chains[blockIdx.x];
     const uint32_t* src = reinterpret_cast<const uint32_t*>(&table[e >> 16]);
     for (int k = threadIdx.x; k < (int)(sizeof(RdParams) / 4); k += blockDim.x) reinterpret_cast<uint32_t*>(&prm)[k] = src[k];
     __syncthreads();
-    rd3_chain<T>(prm, dw, *reinterpret_cast<RdSmem<T, RD3_WARPS>*>(rd3_smem), i4tab, (int)(e & 0xFFFFu));
+    rdw_chain<T>(prm, dw, *reinterpret_cast<RdSmem<T, RDW_WARPS>*>(rdw_smem), i4tab, (int)(e & 0xFFFFu));
 }
 
 template <class T>
-constexpr size_t rd3_smem_bytes() { return sizeof(RdSmem<T, RD3_WARPS>); }
+constexpr size_t rdw_smem_bytes() { return sizeof(RdSmem<T, RDW_WARPS>); }
 
 // ---- the CABAC slice writer ---------------------------------------------------------------------------
 
@@ -1067,66 +1110,194 @@ static __global__ void __launch_bounds__(128) cabac_nb_kernel(const __grid_const
 
 // A slice band's data (FrameCoder::encode with write_mb_cabac, enc/frame.rs:461-486): each macroblock's bins
 // (mb_bins) then end_of_slice_flag, arithmetic coded from the slice's contexts; the data starts on the byte
-// that follows the header's cabac_alignment_one_bit (written on the host). CTA i walks slice band i: lane 0
-// codes a macroblock's bins while lanes 1-31 bring the next one's code and its neighbours' WrNb into the
-// other half of a double buffer in shared memory.
-static __global__ void __launch_bounds__(32) cabac_write_kernel(const __grid_constant__ CabacWriteParams P) {
-    __shared__ uint8_t st[1024];
-    __shared__ uint32_t step[cab::STEP_ENTRIES];
-    __shared__ ironav_mbcode code[2];
-    __shared__ WrNb nb[2][2];  // [buffer][left, top]
-    __shared__ int over;
-    const int chain = blockIdx.x, lane = threadIdx.x & 31;
-    if (chain >= P.nbands) return;
-    for (int i = lane; i < cab::STEP_ENTRIES; i += 32) step[i] = P.step[i];
-    cab::init_states(st, P.intra != 0, 0, P.qp, lane, 32);
-    if (lane == 0) over = 0;
-    cab::BitOut bo = {P.out + (size_t)chain * P.region_words, P.region_words, 0, 0ull, 0, false};
-    cab::Coder k = {st, step, &bo, 0u, 510u, 0u, true};
-    const cab::Slice sl = {P.intra ? 0 : 1, P.t8, P.intra ? 0 : P.nref};
-    const int r0 = P.band_rows[chain], r1 = P.band_rows[chain + 1];
-    const int first = r0 * P.mb_w, end = r1 * P.mb_w;
-    constexpr int W = (int)(sizeof(ironav_mbcode) / 4);
-    // macroblock `mb`'s code and its neighbours' WrNb into buffer b, by lanes lo..31 (zeros: not in the slice)
-    auto fetch = [&](int mb, int b, int lo) {
-        const int mbx = mb % P.mb_w;
-        const bool la = mbx > 0, ta = mb - P.mb_w >= first;
-        const uint32_t* g = reinterpret_cast<const uint32_t*>(&P.codes[mb]);
-        uint32_t* c = reinterpret_cast<uint32_t*>(&code[b]);
-        for (int i = lane - lo; i < W; i += 32 - lo) c[i] = g[i];
-        uint32_t* l = reinterpret_cast<uint32_t*>(&nb[b][0]);
-        uint32_t* t = reinterpret_cast<uint32_t*>(&nb[b][1]);
-        const uint32_t* gl = reinterpret_cast<const uint32_t*>(&P.nbs[la ? mb - 1 : mb]);
-        const uint32_t* gt = reinterpret_cast<const uint32_t*>(&P.nbs[ta ? mb - P.mb_w : mb]);
-        for (int i = lane - lo; i < 2 * WRNB_WORDS; i += 32 - lo) {
-            if (i < WRNB_WORDS) l[i] = la ? gl[i] : 0u;
-            else t[i - WRNB_WORDS] = ta ? gt[i - WRNB_WORDS] : 0u;
-        }
-    };
-    fetch(first, 0, 0);
-    __syncwarp();
-    for (int mb = first; mb < end; mb++) {
-        const int b = (mb - first) & 1;
-        if (lane == 0) {
-            int nbm[8];
-            const bool la = nb[b][0].nb.avail, ta = nb[b][1].nb.avail;
-            for (int q = 0; q < 4; q++) {
-                nbm[q] = la ? nb[b][0].rmodes[q] : -1;
-                nbm[4 + q] = ta ? nb[b][1].bmodes[q] : -1;
+// that follows the header's cabac_alignment_one_bit (written on the host). CTA i walks slice band i, as a pipeline of warps:
+//   - warps 2 and up list the macroblocks' bins, each every WR_LISTERS-th macroblock, in as many turns as its list needs;
+//   - warp 1 takes the lists in order and looks up each bin's probability state (32 bins a turn; the bins of a context are a
+//     chain, the contexts side by side), leaving what the coder needs of it in a ring;
+//   - lane 0 of warp 0 runs the coder's own chain, the range, over the ring.
+// One lane doing all three took 62 ms for an IDR and three P pictures at 1080p, the pipeline 27 ms. Every wait is on shared memory and
+// bounded; a warp that gives up stops the others, and the picture is reported like one that outgrew its region.
+constexpr int WR_LISTERS = 6;
+constexpr int WR_THREADS = (2 + WR_LISTERS) * 32;
+constexpr int WR_CAP = 3328;   // bins a list holds: at least one piece's most (126 map bins and 64 levels of up to 48)
+constexpr int WR_RING = 512;   // bins between the states and the coder
+constexpr unsigned WR_SPINS = 1u << 28;
+
+struct WrSmem {
+    cab::CodeBin ring[WR_RING];
+    cab::CodeBin entry[64];  // per probability state
+    ironav_mbcode code[WR_LISTERS];
+    WrNb nb[WR_LISTERS][2];
+    uint32_t step[cab::STEP_ENTRIES];
+    uint8_t st[1024];
+    uint16_t list[WR_LISTERS][WR_CAP];
+    uint8_t pre[32];                  // a turn's states before its bins
+    unsigned count[WR_LISTERS];       // a list's bins, | WR_LAST when they are its macroblock's last
+    unsigned listed[WR_LISTERS], taken[WR_LISTERS];  // turns of each lister
+    unsigned head, tail;              // bins put into and taken from the ring
+    unsigned stop;
+};
+constexpr unsigned WR_LAST = 1u << 31;
+
+// Waits until the shared word is at least `need` (as a difference, the counts wrap); false when it gave up or another warp did.
+__device__ __forceinline__ bool wr_wait(WrSmem& S, const unsigned* w, unsigned need) {
+    for (unsigned i = 0;; i++) {
+        if ((int)(ld_acquire_cta(w) - need) >= 0) return true;
+        if ((i & 15) == 15) {
+            if (ld_acquire_cta(&S.stop)) return false;
+            if (i >= WR_SPINS) {
+                st_release_cta(&S.stop, 1u);
+                return false;
             }
-            cab::mb_bins(k, sl, &code[b], nb[b][0].nb, nb[b][1].nb, nbm);
-            k.terminate(mb + 1 == end);
-            over = bo.over;
-        } else if (mb + 1 < end) {
-            fetch(mb + 1, b ^ 1, 1);
+            __nanosleep(20);
         }
-        __syncwarp();
-        if (over) break;
     }
-    if (lane == 0) {
-        const uint32_t bytes = bo.finish();
-        P.slice_bytes[chain] = bytes;
-        if (bo.over) atomicOr(&P.slice_bytes[P.nbands], 1u);
+}
+
+static __global__ void __launch_bounds__(WR_THREADS) cabac_write_kernel(const __grid_constant__ CabacWriteParams P) {
+    extern __shared__ __align__(16) unsigned char wr_smem[];
+    WrSmem& S = *reinterpret_cast<WrSmem*>(wr_smem);
+    const int chain = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (chain >= P.nbands) return;
+    for (int i = threadIdx.x; i < cab::STEP_ENTRIES; i += WR_THREADS) S.step[i] = P.step[i];
+    if (threadIdx.x < 64) S.entry[threadIdx.x] = cab::code_entry(threadIdx.x);
+    if (threadIdx.x < WR_LISTERS) S.listed[threadIdx.x] = S.taken[threadIdx.x] = 0;
+    if (threadIdx.x == 0) S.head = S.tail = S.stop = 0;
+    cab::init_states(S.st, P.intra != 0, 0, P.qp, threadIdx.x, WR_THREADS);
+    const cab::Slice sl = {P.intra ? 0 : 1, P.t8, P.intra ? 0 : P.nref};
+    const int first = P.band_rows[chain] * P.mb_w, end = P.band_rows[chain + 1] * P.mb_w;
+    __syncthreads();
+    if (w == 0) {
+        if (lane == 0) {
+            cab::Coder k = {{P.out + (size_t)chain * P.region_words, P.region_words, 0, 0, 0, false, false}, 0ull, 510u, -1};
+            unsigned at = 0, avail = 0;
+            bool more = true;
+            while (more) {
+                if (at == avail) {
+                    st_release_cta(&S.tail, at);
+                    if (!wr_wait(S, &S.head, at + 1)) break;
+                    avail = ld_acquire_cta(&S.head);
+                }
+                // up to eight bins from here, read before the chain begins; slots beyond `avail` are read and not used
+                cab::CodeBin e[8];
+                const unsigned nb = min(avail - at, 8u);
+#pragma unroll
+                for (int i = 0; i < 8; i++) e[i] = S.ring[(at + i) % WR_RING];
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (i < (int)nb) {
+                        k.code(e[i]);
+                        more = e[i].kind != (cab::CODE_TERMINATE | 1u);
+                    }
+                at += nb;
+                if (at % (WR_RING / 4) < 8u) st_release_cta(&S.tail, at);  // room for the states' warp well before the ring runs dry
+            }
+            const uint32_t bytes = k.finish();
+            P.slice_bytes[chain] = bytes;
+            if (more || k.out.over) atomicOr(&P.slice_bytes[P.nbands], 1u);
+        }
+    } else if (w == 1) {
+        unsigned head = 0, turns[WR_LISTERS] = {};
+        for (int mb = first; mb < end; mb++) {
+            const int l = (mb - first) % WR_LISTERS;
+            unsigned n;
+            do {
+                unsigned turn = 0;
+#pragma unroll
+                for (int q = 0; q < WR_LISTERS; q++)
+                    if (q == l) turn = ++turns[q];
+                if (!__all_sync(FULL, wr_wait(S, &S.listed[l], turn))) return;
+                n = S.count[l];
+                const int bins = (int)(n & ~WR_LAST);
+                for (int i0 = 0; i0 < bins; i0 += 32) {
+                    const bool in = i0 + lane < bins;
+                    const uint32_t e = in ? S.list[l][i0 + lane] : cab::BIN_BYPASS;
+                    const bool dec = (e & (cab::BIN_BYPASS | cab::BIN_TERMINATE)) == 0;
+                    const int ctx = dec ? (int)(e & 1023u) : 1024 + lane;
+                    uint32_t m = __match_any_sync(FULL, ctx);
+                    const uint32_t ones = __ballot_sync(FULL, (e >> 10) & 1u);
+                    if (dec && (m & ((1u << lane) - 1u)) == 0) {
+                        uint32_t s = S.st[ctx];
+                        do {
+                            const int j = __ffs(m) - 1;
+                            S.pre[j] = (uint8_t)s;
+                            s = S.step[s * 2 + ((ones >> j) & 1u)] & 0xffu;
+                            m &= m - 1;
+                        } while (m);
+                        S.st[ctx] = (uint8_t)s;
+                    }
+                    const int k = min(bins - i0, 32);
+                    if (!__all_sync(FULL, wr_wait(S, &S.tail, head + (unsigned)k - (unsigned)WR_RING))) return;
+                    __syncwarp();
+                    if (in) {
+                        const uint32_t bin = (e >> 10) & 1u;
+                        cab::CodeBin c = {0u, 0u, 0u, ((e & cab::BIN_TERMINATE) ? cab::CODE_TERMINATE : cab::CODE_BYPASS) | bin};
+                        if (dec) {
+                            const uint32_t s = S.pre[lane];
+                            c = S.entry[s >> 1];
+                            c.kind = (s & 1u) != bin ? cab::CODE_LPS : cab::CODE_MPS;
+                        }
+                        S.ring[(head + lane) % WR_RING] = c;
+                    }
+                    __syncwarp();
+                    head += (unsigned)k;
+                    if (lane == 0) st_release_cta(&S.head, head);
+                }
+                __syncwarp();
+                if (lane == 0) st_release_cta(&S.taken[l], turn);
+            } while (!(n & WR_LAST));
+        }
+    } else {
+        const int l = w - 2;
+        unsigned turn = 0;
+        constexpr int W = (int)(sizeof(ironav_mbcode) / 4);
+        ironav_mbcode* const code = &S.code[l];
+        for (int mb = first + l; mb < end; mb += WR_LISTERS) {
+            const int mbx = mb % P.mb_w;
+            const bool la = mbx > 0, ta = mb - P.mb_w >= first;
+            const uint32_t* g = reinterpret_cast<const uint32_t*>(&P.codes[mb]);
+            for (int i = lane; i < W; i += 32) reinterpret_cast<uint32_t*>(code)[i] = g[i];
+            uint32_t* d = reinterpret_cast<uint32_t*>(S.nb[l]);
+            const uint32_t* gl = reinterpret_cast<const uint32_t*>(&P.nbs[la ? mb - 1 : mb]);
+            const uint32_t* gt = reinterpret_cast<const uint32_t*>(&P.nbs[ta ? mb - P.mb_w : mb]);
+            for (int i = lane; i < 2 * WRNB_WORDS; i += 32) d[i] = i < WRNB_WORDS ? (la ? gl[i] : 0u) : (ta ? gt[i - WRNB_WORDS] : 0u);
+            __syncwarp();
+            const WrNb &L = S.nb[l][0], &T = S.nb[l][1];
+            int nbm[8];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                nbm[q] = la ? L.rmodes[q] : -1;
+                nbm[4 + q] = ta ? T.bmodes[q] : -1;
+            }
+            // the pieces' bins, end_of_slice_flag after the last block's
+            cab::BinCount h, r;
+            cab::lane_head(h, sl, code, L.nb, T.nb, nbm);
+            cab::lane_block(r, code, L.nb, T.nb);
+            if (lane == 31) r.terminate(0);
+            int nh, nr;
+            const int oh = cab::warp_scan(h.n, &nh), orr = nh + cab::warp_scan(r.n, &nr), total = nh + nr;
+            for (int base = 0; base < total;) {
+                if (!__all_sync(FULL, wr_wait(S, &S.taken[l], turn))) return;
+                const bool fh = h.n && oh >= base && oh + h.n <= base + WR_CAP, fr = r.n && orr >= base && orr + r.n <= base + WR_CAP;
+                if (fh) {
+                    cab::BinList c = {&S.list[l][oh - base]};
+                    cab::lane_head(c, sl, code, L.nb, T.nb, nbm);
+                }
+                if (fr) {
+                    cab::BinList c = {&S.list[l][orr - base]};
+                    cab::lane_block(c, code, L.nb, T.nb);
+                    if (lane == 31) c.terminate(mb + 1 == end);
+                }
+                const int to = __reduce_max_sync(FULL, max(fh ? oh + h.n : 0, fr ? orr + r.n : 0));
+                __syncwarp();
+                turn++;
+                if (lane == 0) {
+                    S.count[l] = (unsigned)(to - base) | (to == total ? WR_LAST : 0u);
+                    st_release_cta(&S.listed[l], turn);
+                }
+                base = to;
+            }
+        }
     }
 }
 

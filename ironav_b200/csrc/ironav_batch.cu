@@ -186,8 +186,8 @@ struct ironav_batch {
     RdParams* d_rdtable = nullptr;
     RdParams* h_rdtable = nullptr;
     uint32_t* d_chains = nullptr;
-    int nchains = 0, nchains3 = 0;  // the first nchains3 (the longest bands) on three warps each
-    cudaStream_t aux = nullptr;     // the one-warp launch runs beside the three-warp one
+    int nchains = 0, nchainsw = 0;  // the first nchainsw (the longest bands) in the wide form
+    cudaStream_t aux = nullptr;     // the one-warp launch runs beside the wide one
     cudaEvent_t fork = nullptr, join = nullptr;
     // deblocking (allocated on first use): the streams' jobs, their row groups' merged ticket order, progress
     // words, and the concatenated slice tables (pinned staging reused once the previous copies are done)
@@ -541,32 +541,26 @@ static int batch_decide_rd(ironav_batch* b, ironav_mbstate* const* d_states, iro
     if (!b->d_rdtable) {
         CK(cudaMalloc(&b->d_rdtable, sizeof(RdParams) * b->n));
         CK(cudaHostAlloc(&b->h_rdtable, sizeof(RdParams) * b->n, cudaHostAllocDefault));
-        // the longest bands (at least 3/4 of the longest's macroblocks) first, on three warps each; the rest on one
+        // the longest bands first: as many as there are SMs in the wide form, which takes most of an SM, the rest on one warp each
         std::vector<std::pair<int, uint32_t>> len;
-        int most = 0;
         for (int i = 0; i < b->n; i++) {
             const ironav_ctx* c = b->ctx[i];
-            for (int k = 0; k < c->nslices; k++) {
-                const int mbs = (c->band_rows[k + 1] - c->band_rows[k]) * c->mb_w;
-                len.emplace_back(mbs, (uint32_t)i << 16 | (uint32_t)k);
-                most = std::max(most, mbs);
-            }
+            for (int k = 0; k < c->nslices; k++)
+                len.emplace_back((c->band_rows[k + 1] - c->band_rows[k]) * c->mb_w, (uint32_t)i << 16 | (uint32_t)k);
         }
+        std::stable_sort(len.begin(), len.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
         std::vector<uint32_t> chains;
-        for (const auto& e : len)
-            if (4 * e.first >= 3 * most) chains.push_back(e.second);
-        b->nchains3 = (int)chains.size();
-        for (const auto& e : len)
-            if (4 * e.first < 3 * most) chains.push_back(e.second);
+        for (const auto& e : len) chains.push_back(e.second);
+        b->nchainsw = std::min((int)chains.size(), b->ctx[0]->nsm);
         CK(cudaMalloc(&b->d_chains, sizeof(uint32_t) * chains.size()));
         CK(cudaMemcpy(b->d_chains, chains.data(), sizeof(uint32_t) * chains.size(), cudaMemcpyHostToDevice));
         b->nchains = (int)chains.size();
         CK(cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
-        CK(cudaFuncSetAttribute(decide_rd3_batch_kernel<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rd3_smem_bytes<uint8_t>()));
-        CK(cudaFuncSetAttribute(decide_rd3_batch_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)rd3_smem_bytes<uint16_t>()));
+        CK(cudaFuncSetAttribute(decide_rdw_batch_kernel<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rdw_smem_bytes<uint8_t>()));
+        CK(cudaFuncSetAttribute(decide_rdw_batch_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)rdw_smem_bytes<uint16_t>()));
     }
     if (b->pending) CK(cudaEventSynchronize(b->copied));
     for (int i = 0; i < b->n; i++) {
@@ -585,7 +579,7 @@ static int batch_decide_rd(ironav_batch* b, ironav_mbstate* const* d_states, iro
         p.nbands = c->nslices;
         p.t8 = c->t8;
         const size_t B = c->bd > 8 ? 2 : 1, ly = (size_t)c->pw * c->ph * B, cy = (size_t)(c->pw / 2) * (c->ph / 2) * B;
-        for (int k = 0; k < 2; k++) {
+        for (int k = 0; k < RDW_WARPS - 1; k++) {
             uint8_t* base = c->d_rd_scr + k * (ly + 2 * cy);
             p.scr[3 * k] = base;
             p.scr[3 * k + 1] = base + ly;
@@ -598,21 +592,21 @@ static int batch_decide_rd(ironav_batch* b, ironav_mbstate* const* d_states, iro
     CK(cudaEventRecord(b->copied, b->stream));
     b->pending = true;
     CK(cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned) * 2, b->stream));
-    // the short bands' one-warp launch on the side stream, beside the long bands' three-warp launch
-    const int n1 = b->nchains - b->nchains3;
+    // the short bands' one-warp launch on the side stream, beside the long bands' wide launch
+    const int n1 = b->nchains - b->nchainsw;
     if (n1 > 0) {
         CK(cudaEventRecord(b->fork, b->stream));
         CK(cudaStreamWaitEvent(b->aux, b->fork, 0));
-        if (b->bd > 8) decide_rd_batch_kernel<uint16_t><<<n1, 32, 0, b->aux>>>(b->d_rdtable, b->d_chains + b->nchains3, n1);
-        else decide_rd_batch_kernel<uint8_t><<<n1, 32, 0, b->aux>>>(b->d_rdtable, b->d_chains + b->nchains3, n1);
+        if (b->bd > 8) decide_rd_batch_kernel<uint16_t><<<n1, 32, 0, b->aux>>>(b->d_rdtable, b->d_chains + b->nchainsw, n1);
+        else decide_rd_batch_kernel<uint8_t><<<n1, 32, 0, b->aux>>>(b->d_rdtable, b->d_chains + b->nchainsw, n1);
         CK(cudaGetLastError());
     }
     if (b->bd > 8)
-        decide_rd3_batch_kernel<uint16_t><<<b->nchains3, RD3_WARPS * 32, rd3_smem_bytes<uint16_t>(), b->stream>>>(b->d_rdtable, b->d_chains,
-                                                                                                              b->nchains3);
+        decide_rdw_batch_kernel<uint16_t><<<b->nchainsw, RDW_WARPS * 32, rdw_smem_bytes<uint16_t>(), b->stream>>>(b->d_rdtable, b->d_chains,
+                                                                                                              b->nchainsw);
     else
-        decide_rd3_batch_kernel<uint8_t><<<b->nchains3, RD3_WARPS * 32, rd3_smem_bytes<uint8_t>(), b->stream>>>(b->d_rdtable, b->d_chains,
-                                                                                                            b->nchains3);
+        decide_rdw_batch_kernel<uint8_t><<<b->nchainsw, RDW_WARPS * 32, rdw_smem_bytes<uint8_t>(), b->stream>>>(b->d_rdtable, b->d_chains,
+                                                                                                            b->nchainsw);
     CK(cudaGetLastError());
     if (n1 > 0) {
         CK(cudaEventRecord(b->join, b->aux));

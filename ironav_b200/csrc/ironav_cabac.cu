@@ -59,12 +59,12 @@ int cabac_setup(ironav_ctx* c) {
     CK(cudaMalloc(&c->d_band_rows, sizeof(int) * (c->nslices + 1)));
     CK(cudaMemcpy(c->d_band_rows, c->band_rows, sizeof(int) * (c->nslices + 1), cudaMemcpyHostToDevice));
     CK(cudaMalloc(&c->d_rd_nb, sizeof(cab::Nb) * c->nmb));
-    // the three-warp form's scratch planes: luma, Cb and Cr of warp 1, then of warp 2
+    // the wide form's scratch planes: luma, Cb and Cr of each of warps 1 to 4
     const size_t B = c->bd > 8 ? 2 : 1, ly = (size_t)c->pw * c->ph * B, cy = (size_t)(c->pw / 2) * (c->ph / 2) * B;
-    CK(cudaMalloc(&c->d_rd_scr, 2 * (ly + 2 * cy)));
-    const size_t s8 = rd3_smem_bytes<uint8_t>(), s16 = rd3_smem_bytes<uint16_t>();
-    CK(cudaFuncSetAttribute(decide_rd3_kernel<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s8));
-    CK(cudaFuncSetAttribute(decide_rd3_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s16));
+    CK(cudaMalloc(&c->d_rd_scr, (RDW_WARPS - 1) * (ly + 2 * cy)));
+    const size_t s8 = rdw_smem_bytes<uint8_t>(), s16 = rdw_smem_bytes<uint16_t>();
+    CK(cudaFuncSetAttribute(decide_rdw_kernel<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s8));
+    CK(cudaFuncSetAttribute(decide_rdw_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s16));
     return IRONAV_OK;
 }
 
@@ -85,7 +85,7 @@ int launch_decide_rd(ironav_ctx* c, ironav_mbstate* d_states, ironav_mbcode* d_c
     p.nbands = c->nslices;
     p.t8 = c->t8;
     const size_t B = c->bd > 8 ? 2 : 1, ly = (size_t)c->pw * c->ph * B, cy = (size_t)(c->pw / 2) * (c->ph / 2) * B;
-    for (int k = 0; k < 2; k++) {
+    for (int k = 0; k < RDW_WARPS - 1; k++) {
         uint8_t* base = c->d_rd_scr + k * (ly + 2 * cy);
         p.scr[3 * k] = base;
         p.scr[3 * k + 1] = base + ly;
@@ -94,9 +94,9 @@ int launch_decide_rd(ironav_ctx* c, ironav_mbstate* d_states, ironav_mbcode* d_c
     p.scr_ys = c->pw;
     p.scr_cs = c->pw / 2;
     CK(cudaMemsetAsync(c->d_counters, 0, 2 * sizeof(unsigned), c->stream));
-    // one stream: three warps a chain (its bands are few, so each chain's latency is the picture's)
-    if (c->bd > 8) decide_rd3_kernel<uint16_t><<<c->nslices, RD3_WARPS * 32, rd3_smem_bytes<uint16_t>(), c->stream>>>(p);
-    else decide_rd3_kernel<uint8_t><<<c->nslices, RD3_WARPS * 32, rd3_smem_bytes<uint8_t>(), c->stream>>>(p);
+    // one stream: the wide form (its bands are few, so each chain's latency is the picture's)
+    if (c->bd > 8) decide_rdw_kernel<uint16_t><<<c->nslices, RDW_WARPS * 32, rdw_smem_bytes<uint16_t>(), c->stream>>>(p);
+    else decide_rdw_kernel<uint8_t><<<c->nslices, RDW_WARPS * 32, rdw_smem_bytes<uint8_t>(), c->stream>>>(p);
     return cuda_status(cudaGetLastError());
 }
 
@@ -108,6 +108,7 @@ int cabac_slice_data(ironav_ctx* c, int idr, const ironav_mbcode* d_codes, std::
         int most = 0;
         for (int i = 0; i < ns; i++) most = std::max(most, (c->band_rows[i + 1] - c->band_rows[i]) * c->mb_w);
         c->cab_region_words = ((unsigned long long)most * CAB_MB_BYTES) / 4 + 2;
+        CK(cudaFuncSetAttribute(cabac_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WrSmem)));
         CK(cudaMalloc(&c->d_cab_out, sizeof(uint32_t) * c->cab_region_words * ns));
         CK(cudaMalloc(&c->d_cab_bytes, sizeof(uint32_t) * (ns + 1)));
         CK(cudaMalloc(&c->d_cab_wnb, sizeof(WrNb) * c->nmb));
@@ -131,7 +132,7 @@ int cabac_slice_data(ironav_ctx* c, int idr, const ironav_mbcode* d_codes, std::
     p.qp = c->qpp - 6 * (c->bd - 8);
     CK(cudaMemsetAsync(c->d_cab_bytes, 0, sizeof(uint32_t) * (ns + 1), c->stream));
     cabac_nb_kernel<<<std::min((c->nmb + 3) / 4, c->nsm * 16), 128, 0, c->stream>>>(p);
-    cabac_write_kernel<<<ns, 32, 0, c->stream>>>(p);
+    cabac_write_kernel<<<ns, WR_THREADS, sizeof(WrSmem), c->stream>>>(p);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(c->h_cab_bytes, c->d_cab_bytes, sizeof(uint32_t) * (ns + 1), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
