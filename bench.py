@@ -62,7 +62,7 @@ def parse():
     p.add_argument("--streams", type=int, default=64, help="streams of the batched workload")
     p.add_argument("--replay-form", type=int, default=None, choices=[0, 1, 2, 3],
                    help="replay mode's kernel (ironav_set_replay_form): 0 8-lane groups, 1 one macroblock a warp, 2 16-lane "
-                        "groups, 3 4-lane groups; default the library's choice for the depth (0 at 8 bits, 1 at 10)")
+                        "groups, 3 4-lane groups; default the library's choice for the picture (at 1080p 0 at 8 bits, 1 at 10)")
     p.add_argument("--learned-samples", type=int, default=2_000_000, help="training samples of the learned workload's proposer")
     p.add_argument("--e2e-threads", type=int, default=8, help="host threads (each with a context) of the e2e pass")
     p.add_argument("--cabac", action="store_true",

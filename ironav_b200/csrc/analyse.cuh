@@ -7,7 +7,7 @@
 // bookkeeping is kept small:
 //   - integer SAD: 8 candidate vectors per batch, lane group c = lane & 7 scores candidate c (each lane
 //     works out its own candidate), its 4 lanes split the rows; reference rows are read as aligned
-//     32-bit words realigned with funnel shifts and compared with __vsadu4; sums by 2 xor shuffles;
+//     32-bit words realigned with funnel shifts and compared with vsad4; sums by 2 xor shuffles;
 //   - the diamond's greedy rounds (each move relative to the current best, strict '<', enc/frame.rs:
 //     973-988) are resolved exactly: one batch scores the whole 3x3 square of the round's step around
 //     the centre, which holds every point the four sequential moves can visit, and the moves are then
@@ -53,9 +53,22 @@ static __device__ __constant__ int8_t c_nsub[4] = {1, 2, 2, 4};
 // A 4x4 block's list-0 motion as the predictors see it: (mx, my, ref (-1 none), available).
 using Blk = int4;
 
+// The window of a reference's G plane that a macroblock's integer search reads from shared memory: ROWS rows of PITCH bytes,
+// R samples and more around the macroblock moved by its predictor. The eight candidates of a batch lie on a dozen rows, and in
+// L1 every row of a load is a lookup of its own; in the window, whose pitch puts eight rows on disjoint banks, they are one or two
+// passes (1080p on one warp a macroblock 224 -> 219 us, in live coding 77.6 -> 74.1; decide mode's picture 7.90 -> 7.57 ms). At 10 bits the
+// search reads the planes: the window is twice the bytes, and staging it cost what it saved (4K 950 -> 958 us).
+template <class T>
+struct Win {
+    static constexpr bool ON = sizeof(T) == 1;
+    static constexpr int R = 24, ROWS = 16 + 2 * R, PITCH = ROWS + 16, BYTES = ON ? ROWS * PITCH : 16;
+};
+
 // Per-warp shared memory; T is the sample type (uint8_t for 8-bit pictures, uint16_t for 10-bit).
 template <class T>
 struct WarpSmem {
+    __align__(16) uint8_t win[Win<T>::BYTES];  // the staged window, and its place in the plane (columns, rows)
+    int win_x, win_y;
     uint32_t src[64 * sizeof(T)];  // current macroblock, 16 rows of 16 samples (4 * sizeof(T) words each)
     Blk ext[30];              // blocks around the macroblock: index (y + 1) * 6 + (x + 1), x in -1..4, y in -1..3
     Blk st[16];               // P_8x8: blocks decided so far (sub_search's `st`)
@@ -211,60 +224,128 @@ static __device__ int2 skip_mv(const AnalyseParams& __restrict__ P, WarpSmem<T>&
 
 // ---- scoring -------------------------------------------------------------------------------------
 
-// Integer SAD (sad_int, enc/frame.rs:662-671) of the partition at this lane's candidate (px, py): g0 is the
-// reference plane G at the partition's origin (a byte address), src the partition's first source word, w x h
-// its size, sw the plane stride in samples. The lanes of a group (same lane & 7) share a candidate and split
+// c + the sum of the absolute differences of a's and b's bytes, in one instruction.
+__device__ __forceinline__ int vsad4(uint32_t a, uint32_t b, int c) {
+    uint32_t d;
+    asm("vabsdiff4.u32.u32.u32.add %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"((uint32_t)c));
+    return (int)d;
+}
+// c + the absolute differences of a's and b's 16-bit halves, half by half: 10-bit samples leave room for 64 of them, and three
+// instructions a word take a third of the time of __vsadu2's eight.
+__device__ __forceinline__ uint32_t vad2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t hi, lo;
+    asm("max.u16x2 %0, %1, %2;" : "=r"(hi) : "r"(a), "r"(b));
+    asm("min.u16x2 %0, %1, %2;" : "=r"(lo) : "r"(a), "r"(b));
+    return c + hi - lo;
+}
+__device__ __forceinline__ int sum2(uint32_t v) { return (int)((v & 0xffffu) + (v >> 16)); }
+
+// Integer SAD (sad_int, enc/frame.rs:662-671) of the partition at this lane's candidate (px, py). The lanes of a group (same lane & 7) share a candidate and split
 // its rows; every lane of the group gets the sum. Rows are read as aligned 32-bit words realigned with funnel
-// shifts: 4 samples a word compared with __vsadu4 (8-bit), 2 with __vsadu2 (16-bit).
-template <class T>
-static __device__ __forceinline__ int sad_lane(const uint8_t* __restrict__ g0, const uint32_t* __restrict__ src, int sw, int w,
-                                               int h, int px, int py, bool valid) {
-    constexpr int B = sizeof(T);
-    const int lane = threadIdx.x & 31;
-    int sad = 0;
-    if (!valid) px = py = 0;  // scored at a position always inside the planes, and discarded: no divergent branch
-    {
-        const int row0 = lane >> 3;
-        const uint8_t* G = g0 + (((py >> 2) + row0) * sw + (px >> 2)) * B;
-        const int step4 = 4 * sw * B;
-        for (int row = row0; row < h; row += 4, G += step4) {
-            const uintptr_t a = reinterpret_cast<uintptr_t>(G);
-            const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
-            const unsigned sh = (unsigned)(a & 3) * 8u;
-            const uint32_t* sr = src + row * 4 * B;
-            if constexpr (B == 1) {
-                const uint32_t w0 = __ldg(q), w1 = __ldg(q + 1);
-                sad += __vsadu4(sr[0], __funnelshift_r(w0, w1, sh));
-                if (w >= 8) {
-                    const uint32_t w2 = __ldg(q + 2);
-                    sad += __vsadu4(sr[1], __funnelshift_r(w1, w2, sh));
-                    if (w == 16) {
-                        const uint32_t w3 = __ldg(q + 3), w4 = __ldg(q + 4);
-                        sad += __vsadu4(sr[2], __funnelshift_r(w2, w3, sh)) + __vsadu4(sr[3], __funnelshift_r(w3, w4, sh));
-                    }
-                }
-            } else {
-                const uint32_t w0 = __ldg(q), w1 = __ldg(q + 1), w2 = __ldg(q + 2);
-                sad += __vsadu2(sr[0], __funnelshift_r(w0, w1, sh)) + __vsadu2(sr[1], __funnelshift_r(w1, w2, sh));
-                if (w >= 8) {
-                    const uint32_t w3 = __ldg(q + 3), w4 = __ldg(q + 4);
-                    sad += __vsadu2(sr[2], __funnelshift_r(w2, w3, sh)) + __vsadu2(sr[3], __funnelshift_r(w3, w4, sh));
-                    if (w == 16) {
-                        uint32_t pv = w4;
+// shifts: 4 samples a word compared with vsad4 (8-bit), 2 with vad2 (10-bit).
+// Where a partition's integer candidates are read: its origin in the reference plane G (a byte address, the plane's stride in
+// samples), and in the staged window (a shared-memory address; 0: none staged) the origin's column and row.
+struct Ref {
+    const uint8_t* g0;
+    int sw;
+    uint32_t win;
+    int wx, wy;
+};
+
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+
+// One row of sad_lane: w samples from the words q[0..] (ld(k) reads word k) shifted by sh bits, against source words sr.
+template <class T, class L>
+__device__ __forceinline__ void sad_row(L ld, const uint32_t* __restrict__ sr, unsigned sh, int w, int& sad, uint32_t& ad) {
+    if constexpr (sizeof(T) == 1) {
+        const uint32_t w0 = ld(0), w1 = ld(1);
+        sad = vsad4(sr[0], __funnelshift_r(w0, w1, sh), sad);
+        if (w >= 8) {
+            const uint32_t w2 = ld(2);
+            sad = vsad4(sr[1], __funnelshift_r(w1, w2, sh), sad);
+            if (w == 16) {
+                const uint32_t w3 = ld(3), w4 = ld(4);
+                sad = vsad4(sr[3], __funnelshift_r(w3, w4, sh), vsad4(sr[2], __funnelshift_r(w2, w3, sh), sad));
+            }
+        }
+    } else {
+        const uint32_t w0 = ld(0), w1 = ld(1), w2 = ld(2);
+        ad = vad2(sr[1], __funnelshift_r(w1, w2, sh), vad2(sr[0], __funnelshift_r(w0, w1, sh), ad));
+        if (w >= 8) {
+            const uint32_t w3 = ld(3), w4 = ld(4);
+            ad = vad2(sr[3], __funnelshift_r(w3, w4, sh), vad2(sr[2], __funnelshift_r(w2, w3, sh), ad));
+            if (w == 16) {
+                uint32_t pv = w4;
 #pragma unroll
-                        for (int k = 4; k < 8; k++) {
-                            const uint32_t nx = __ldg(q + k + 1);
-                            sad += __vsadu2(sr[k], __funnelshift_r(pv, nx, sh));
-                            pv = nx;
-                        }
-                    }
+                for (int k = 4; k < 8; k++) {
+                    const uint32_t nx = ld(k + 1);
+                    ad = vad2(sr[k], __funnelshift_r(pv, nx, sh), ad);
+                    pv = nx;
                 }
             }
         }
     }
+}
+
+// src: the partition's first source word, w x h its size. The rows' loops are not unrolled in the P kernels: their code is
+// large enough that its copies cost more than the loop (1080p on one warp a macroblock 240 -> 223 us); UNROLL is the B kernel's.
+template <class T, int UNROLL = 1>
+static __device__ __forceinline__ int sad_lane(const Ref& ref, const uint32_t* __restrict__ src, int w, int h, int px, int py, bool valid) {
+    constexpr int B = sizeof(T);
+    const int lane = threadIdx.x & 31;
+    int sad = 0;
+    uint32_t ad = 0;  // 10-bit: the two halves' sums (at most 32 words a lane)
+    if (!valid) px = py = 0;  // scored at a position always inside the planes, and discarded: no divergent branch
+    const int row0 = lane >> 3;
+    const int wr = ref.wy + (py >> 2), wc = (ref.wx + (px >> 2)) * B;
+    const bool in = !valid || ((unsigned)wr <= (unsigned)(Win<T>::ROWS - h) && wc >= 0 && (wc & ~3) + w * B + 4 <= Win<T>::PITCH);
+    if (Win<T>::ON && ref.win != 0 && __all_sync(FULL, in)) {
+        const unsigned sh = (unsigned)(wc & 3) * 8u;
+        uint32_t a = ref.win + (valid ? (uint32_t)((wr + row0) * Win<T>::PITCH + (wc & ~3)) : 0u);
+#pragma unroll 1
+        for (int row = row0; row < h; row += 4, a += 4 * Win<T>::PITCH)
+            sad_row<T>([&](int k) { return lds32(a + 4u * k); }, src + row * 4 * B, sh, w, sad, ad);
+    } else {
+        const uint8_t* G = ref.g0 + (((py >> 2) + row0) * ref.sw + (px >> 2)) * B;
+        const int step4 = 4 * ref.sw * B;
+#pragma unroll UNROLL
+        for (int row = row0; row < h; row += 4, G += step4) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(G);
+            const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
+            sad_row<T>([&](int k) { return __ldg(q + k); }, src + row * 4 * B, (unsigned)(a & 3) * 8u, w, sad, ad);
+        }
+    }
+    if constexpr (B == 2) sad = sum2(ad);
     sad += __shfl_xor_sync(FULL, sad, 8);
     sad += __shfl_xor_sync(FULL, sad, 16);
     return sad;
+}
+
+// Stages the window of reference r around the macroblock moved by (mx, my), a vector clamped as the search's candidates are:
+// rows and columns then lie inside the plane, but for a last row's end, which the planes after G hold.
+template <class T>
+static __device__ __forceinline__ void stage_window(const AnalyseParams& __restrict__ P, WarpSmem<T>& __restrict__ S, int r, int mx, int my) {
+    constexpr int N = Win<T>::PITCH / 16;
+    const int lane = threadIdx.x & 31;
+    const int x = (S.mbx * 16 + PAD + (mx >> 2) - Win<T>::R) & ~15, y = S.mby * 16 + PAD + (my >> 2) - Win<T>::R;
+    const uint8_t* g = P.planes[r] + (size_t)y * P.sw + x;
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(S.win);
+#pragma unroll 1
+    for (int i = lane; i < Win<T>::ROWS * N; i += 32) {
+        const int row = i / N, c = i - row * N;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + (uint32_t)i * 16u), "l"(g + (size_t)row * P.sw + c * 16) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (lane == 0) {
+        S.win_x = x;
+        S.win_y = y;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
 }
 
 // The quarter-sample prediction (HalfPel::predict, enc/subpel.rs:122-145) of the 4x4 block (bxx, byy), in
@@ -327,10 +408,15 @@ __device__ __forceinline__ int score4(const WarpSmem<T>& __restrict__ S, int sbx
         for (int k = 0; k < B; k++) sr[row][k] = sp[row * 4 * B + k];
     int v = 0;
     if (sad) {
+        uint32_t ad = 0;
 #pragma unroll
         for (int row = 0; row < 4; row++)
 #pragma unroll
-            for (int k = 0; k < B; k++) v += B == 1 ? __vsadu4(sr[row][k], pr[row][k]) : __vsadu2(sr[row][k], pr[row][k]);
+            for (int k = 0; k < B; k++) {
+                if constexpr (B == 1) v = vsad4(sr[row][k], pr[row][k], v);
+                else ad = vad2(sr[row][k], pr[row][k], ad);
+            }
+        if constexpr (B == 2) v = sum2(ad);
     } else if constexpr (B == 1) {
         const uint32_t s1[4] = {sr[0][0], sr[1][0], sr[2][0], sr[3][0]}, p1[4] = {pr[0][0], pr[1][0], pr[2][0], pr[3][0]};
         v = satd4_packed(s1, p1);
@@ -351,6 +437,7 @@ static __device__ __forceinline__ void pred_batch(const AnalyseParams& __restric
     __syncwarp();
     const int x0 = S.mbx * 16 + bx * 4, y0 = S.mby * 16 + by * 4;
     const uint8_t* base = P.planes[r];
+#pragma unroll 1
     for (int t = lane; t < total; t += 32) {
         const int c = t >> lg, b = t & ((1 << lg) - 1), bxx = b & ((1 << lgw) - 1), byy = b >> lgw;
         uint32_t pr[4][sizeof(T)];
@@ -367,7 +454,7 @@ static __device__ __forceinline__ void pred_batch(const AnalyseParams& __restric
 // the points it lacks.
 // Returns whether the best moved.
 template <class T>
-static __device__ __noinline__ int4 round_clamped(const AnalyseParams& __restrict__ P, WarpSmem<T>& __restrict__ S, int r, int bx, int by, int w, int h, int mvpx, int mvpy, int step, int cxlo,
+static __device__ __noinline__ int4 round_clamped(const AnalyseParams& __restrict__ P, WarpSmem<T>& __restrict__ S, const Ref ref, int bx, int by, int w, int h, int mvpx, int mvpy, int step, int cxlo,
                                            int cxhi, int cylo, int cyhi, int bxv, int byv, int bc) {
     const int lane = threadIdx.x & 31;
     const int cx = bxv, cy = byv;
@@ -388,8 +475,7 @@ static __device__ __noinline__ int4 round_clamped(const AnalyseParams& __restric
         if (ix >= 0 && iy >= 0) {
             v = S.cost[iy * 3 + ix];
         } else {
-            const uint8_t* g0 = P.planes[r] + ((S.mby * 16 + by * 4 + PAD) * P.sw + S.mbx * 16 + bx * 4 + PAD) * (int)sizeof(T);
-            const int s1 = sad_lane<T>(g0, &S.src[(by * 16 + bx) * (int)sizeof(T)], P.sw, w, h, nx, ny, (lane & 7) == 0);
+            const int s1 = sad_lane<T>(ref, &S.src[(by * 16 + bx) * (int)sizeof(T)], w, h, nx, ny, (lane & 7) == 0);
             v = __shfl_sync(FULL, s1, 0) + P.lambda * mvd_bits_d(nx, ny, mvpx, mvpy);
         }
         if (v < bc) {
@@ -406,9 +492,8 @@ static __device__ __noinline__ int4 round_clamped(const AnalyseParams& __restric
 // kernel's code is large enough that its copies of them inlined at every call cost it instruction-cache
 // misses (0.725 -> 0.662 ms per 1080p B picture out of line); the P kernels keep them inlined.
 template <class T>
-static __device__ __noinline__ int sad_lane_ni(const uint8_t* __restrict__ g0, const uint32_t* __restrict__ src, int sw, int w, int h, int px,
-                                              int py, bool valid) {
-    return sad_lane<T>(g0, src, sw, w, h, px, py, valid);
+static __device__ __noinline__ int sad_lane_ni(const Ref ref, const uint32_t* __restrict__ src, int w, int h, int px, int py, bool valid) {
+    return sad_lane<T, sizeof(T) == 1 ? 2 : 1>(ref, src, w, h, px, py, valid);
 }
 template <class T>
 static __device__ __noinline__ void pred_batch_ni(const AnalyseParams& __restrict__ P, WarpSmem<T>& __restrict__ S, int r, int bx, int by, int lgw,
@@ -419,12 +504,11 @@ static __device__ __noinline__ void pred_batch_ni(const AnalyseParams& __restric
 // One round of the diamond (enc/frame.rs:973-988) at `step` around (bxv, byv) of cost bc: the 3x3 square of the
 // step is scored in one batch (lane group g -> square position k = g < 4 ? g : g + 1), then the reference's four
 // moves are replayed in order (left, else right; then up from that column, else down). Returns whether the
-// centre moved; (bxv, byv, bc) become the new centre. g0 and src0 as for sad_lane, sw the plane stride.
+// centre moved; (bxv, byv, bc) become the new centre. ref and src0 as for sad_lane.
 template <class T, bool MORE>
-static __device__ __forceinline__ bool diamond_round(const AnalyseParams& __restrict__ P, WarpSmem<T>& __restrict__ S, int r, int bx, int by, int w,
+static __device__ __forceinline__ bool diamond_round(const AnalyseParams& __restrict__ P, WarpSmem<T>& __restrict__ S, int bx, int by, int w,
                                                      int h, int mvpx, int mvpy, int step, int cxlo, int cxhi, int cylo, int cyhi,
-                                                     const uint8_t* __restrict__ g0, const uint32_t* __restrict__ src0, int sw, int& bxv,
-                                                     int& byv, int& bc) {
+                                                     const Ref& ref, const uint32_t* __restrict__ src0, int& bxv, int& byv, int& bc) {
     const int lane = threadIdx.x & 31, g = lane & 7;
     const int lam = P.lambda;
     const int k = g < 4 ? g : g + 1, kx = k % 3, ky = k / 3;
@@ -433,7 +517,7 @@ static __device__ __forceinline__ bool diamond_round(const AnalyseParams& __rest
     const int cx = bxv, cy = byv, c0 = bc;
     const int X0 = clx(cx - step), X2 = clx(cx + step), Y0 = cly(cy - step), Y2 = cly(cy + step);
     const int qx = kx == 0 ? X0 : (kx == 1 ? cx : X2), qy = ky == 0 ? Y0 : (ky == 1 ? cy : Y2);
-    const int sc = (MORE ? sad_lane_ni<T>(g0, src0, sw, w, h, qx, qy, true) : sad_lane<T>(g0, src0, sw, w, h, qx, qy, true)) + lam * mvd_bits_d(qx, qy, mvpx, mvpy);
+    const int sc = (MORE ? sad_lane_ni<T>(ref, src0, w, h, qx, qy, true) : sad_lane<T>(ref, src0, w, h, qx, qy, true)) + lam * mvd_bits_d(qx, qy, mvpx, mvpy);
     bool moved;
     if (X0 == cx - step && X2 == cx + step && Y0 == cy - step && Y2 == cy + step) {
         // no clamp: left, else right; then up from that column, else down
@@ -463,7 +547,7 @@ static __device__ __forceinline__ bool diamond_round(const AnalyseParams& __rest
         if (lane < 8) S.cost[k] = sc;
         if (lane == 0) S.cost[4] = c0;
         __syncwarp();
-        const int4 rc = round_clamped(P, S, r, bx, by, w, h, mvpx, mvpy, step, cxlo, cxhi, cylo, cyhi, bxv, byv, bc);
+        const int4 rc = round_clamped(P, S, ref, bx, by, w, h, mvpx, mvpy, step, cxlo, cxhi, cylo, cyhi, bxv, byv, bc);
         moved = rc.x != 0;
         bxv = rc.y;
         byv = rc.z;
@@ -520,10 +604,11 @@ static __device__ __noinline__ int4 motion_search(const AnalyseParams& __restric
             py = intr(cly(more[0].y));
         }
     }
-    const int sw = P.sw;
-    const uint8_t* const g0 = P.planes[r] + ((y0 + PAD) * sw + x0 + PAD) * (int)sizeof(T);
+    // the window is the P searches' (best_inter_ref stages it)
+    const Ref ref = {P.planes[r] + ((y0 + PAD) * P.sw + x0 + PAD) * (int)sizeof(T), P.sw,
+                     MORE || !Win<T>::ON ? 0u : (uint32_t)__cvta_generic_to_shared(S.win), x0 + PAD - S.win_x, y0 + PAD - S.win_y};
     const uint32_t* const src0 = &S.src[(by * 16 + bx) * (int)sizeof(T)];
-    int cost = MORE ? sad_lane_ni<T>(g0, src0, sw, w, h, px, py, valid) : sad_lane<T>(g0, src0, sw, w, h, px, py, valid);
+    int cost = MORE ? sad_lane_ni<T>(ref, src0, w, h, px, py, valid) : sad_lane<T>(ref, src0, w, h, px, py, valid);
     cost = valid ? cost + lam * mvd_bits_d(px, py, mvpx, mvpy) : BIG;
     const unsigned vmask = __ballot_sync(FULL, valid) & 0xffu;
     if (lane == 0) S.sad_px += (uint32_t)(__popc(vmask) * w * h);
@@ -537,7 +622,7 @@ static __device__ __noinline__ int4 motion_search(const AnalyseParams& __restric
             qx = intr(clx(more[g + 1].x));
             qy = intr(cly(more[g + 1].y));
         }
-        int c2 = sad_lane_ni<T>(g0, src0, sw, w, h, qx, qy, v2);
+        int c2 = sad_lane_ni<T>(ref, src0, w, h, qx, qy, v2);
         c2 = v2 ? c2 + lam * mvd_bits_d(qx, qy, mvpx, mvpy) : BIG;
         const unsigned vm2 = __ballot_sync(FULL, v2) & 0xffu;
         if (lane == 0) S.sad_px += (uint32_t)(__popc(vm2) * w * h);
@@ -561,7 +646,7 @@ static __device__ __noinline__ int4 motion_search(const AnalyseParams& __restric
         const int iters = step == 4 ? 32 : 4;
         for (int it = 0; it < iters; it++) {
             rounds++;
-            if (!diamond_round<T, MORE>(P, S, r, bx, by, w, h, mvpx, mvpy, step, cxlo, cxhi, cylo, cyhi, g0, src0, sw, bxv, byv, bc)) break;
+            if (!diamond_round<T, MORE>(P, S, bx, by, w, h, mvpx, mvpy, step, cxlo, cxhi, cylo, cyhi, ref, src0, bxv, byv, bc)) break;
         }
     }
     if (lane == 0) S.sad_px += (uint32_t)(4 * w * h * rounds);
@@ -687,6 +772,13 @@ static __device__ __noinline__ int4 best_inter_ref(const AnalyseParams& __restri
     else if (P.nact > 2) rb = lam * (2 * (31 - __clz(r + 1)) + 1);
     const int2 mvp = pred_mv(P, S, S.ext, nullptr, 0, 0, 4, 0, r);
     const ColMv col = P.col[S.mb];
+    if constexpr (Win<T>::ON) {
+        // around the search's first candidate
+        const int x0 = S.mbx * 16, y0 = S.mby * 16;
+        const int cx = min(max(mvp.x, max(-(x0 + 24) * 4, -2048)), min((P.mb_w * 16 - x0 + 8) * 4, 2047));
+        const int cy = min(max(mvp.y, max(-(y0 + 24) * 4, -512)), min((P.mb_h * 16 - y0 + 8) * 4, 511));
+        stage_window(P, S, r, (cx + 2) & ~3, (cy + 2) & ~3);
+    }
     const int4 ms = motion_search<T, false>(P, S, S.ext, r, r, 0, 0, 4, 4, mvp.x, mvp.y, col.mv[0], col.mv[1], 0, 0, col.valid ? 1 : 0, nullptr, 0);
     const int c = ms.x, mx = ms.y, my = ms.z;
     int best_part = 0, best_cost = c + lam * (mvd_bits_d(mx, my, mvp.x, mvp.y) + 1) + rb;
@@ -796,8 +888,7 @@ static __device__ __noinline__ int4 learned_inter(const AnalyseParams& __restric
     auto cly = [&](int v) { return min(max(v, cylo), cyhi); };
     auto intr = [](int v) { return (v + 2) & ~3; };
     const int16_t* cand = P.learned + (size_t)S.mb * 8;
-    const int sw = P.sw;
-    const uint8_t* const g0 = P.planes[r] + ((y0 + PAD) * sw + x0 + PAD) * (int)sizeof(T);
+    const Ref ref = {P.planes[r] + ((y0 + PAD) * P.sw + x0 + PAD) * (int)sizeof(T), P.sw, 0u, 0, 0};
     const uint32_t* const src0 = &S.src[0];
     unsigned best = 0xffffffffu, start = 0xffffffffu;
     for (int b = 0; b < 13; b++) {
@@ -809,7 +900,7 @@ static __device__ __noinline__ int4 learned_inter(const AnalyseParams& __restric
             px = clx(intr(clx(cand[2 * k])) + 4 * (d % 5 - 2));
             py = cly(intr(cly(cand[2 * k + 1])) + 4 * (d / 5 - 2));
         }
-        const int sad = sad_lane<T>(g0, src0, sw, 16, 16, px, py, valid);
+        const int sad = sad_lane<T>(ref, src0, 16, 16, px, py, valid);
         const unsigned cost = (unsigned)(sad + lam * mvd_bits_d(px, py, mvp.x, mvp.y));
         unsigned kp = (valid && i < 100) ? ((cost << 7) | (unsigned)i) : 0xffffffffu;
         unsigned ks = (i == 100) ? cost : 0xffffffffu;
@@ -834,7 +925,7 @@ static __device__ __noinline__ int4 learned_inter(const AnalyseParams& __restric
         int rounds = 0;
         for (int it = 0; it < 32; it++) {
             rounds++;
-            if (!diamond_round<T, false>(P, S, r, 0, 0, 16, 16, mvp.x, mvp.y, 4, cxlo, cxhi, cylo, cyhi, g0, src0, sw, bxv, byv, bc)) break;
+            if (!diamond_round<T, false>(P, S, 0, 0, 16, 16, mvp.x, mvp.y, 4, cxlo, cxhi, cylo, cyhi, ref, src0, bxv, byv, bc)) break;
         }
         if (lane == 0) S.sad_px += (uint32_t)(4 * 256 * rounds);
     }

@@ -70,17 +70,18 @@ __device__ __forceinline__ int row_sad(const uint8_t* G, const uint32_t* sr, int
     const unsigned sh = (unsigned)(a & 3) * 8u;
     const int nw = (w * B) >> 2;
     int sad = 0;
-    uint32_t pv = __ldg(q);
+    uint32_t ad = 0, pv = __ldg(q);
 #pragma unroll
     for (int k = 0; k < 4 * B; k++) {
         if (k < nw) {
             const uint32_t nx = __ldg(q + k + 1);
             const uint32_t v = __funnelshift_r(pv, nx, sh);
-            sad += B == 1 ? __vsadu4(sr[k], v) : __vsadu2(sr[k], v);
+            if constexpr (B == 1) sad = vsad4(sr[k], v, sad);
+            else ad = vad2(sr[k], v, ad);
             pv = nx;
         }
     }
-    return sad;
+    return B == 1 ? sad : sum2(ad);
 }
 
 // Integer SAD (sad_int, enc/frame.rs:662-671) of the w x h partition for two vectors at once: the first half
@@ -96,6 +97,7 @@ __device__ __forceinline__ int2 sad2(const Grp<GW>& g, const uint8_t* __restrict
     const int r0 = g.gl & (H - 1);
     const uint8_t* G = g0 + (((py >> 2) + r0) * sw + (px >> 2)) * B;
     int s = 0;
+#pragma unroll 1
     for (int row = r0; row < h; row += H, G += H * sw * B) s += row_sad<T>(G, src + row * 4 * B, w);
 #pragma unroll
     for (int off = 1; off < H; off <<= 1) s += __shfl_xor_sync(g.mask, s, off, GW);
@@ -115,10 +117,15 @@ __device__ __forceinline__ int score4_src(const uint32_t* __restrict__ src, int 
         for (int k = 0; k < B; k++) sr[row][k] = sp[row * 4 * B + k];
     int v = 0;
     if (sad) {
+        uint32_t ad = 0;
 #pragma unroll
         for (int row = 0; row < 4; row++)
 #pragma unroll
-            for (int k = 0; k < B; k++) v += B == 1 ? __vsadu4(sr[row][k], pr[row][k]) : __vsadu2(sr[row][k], pr[row][k]);
+            for (int k = 0; k < B; k++) {
+                if constexpr (B == 1) v = vsad4(sr[row][k], pr[row][k], v);
+                else ad = vad2(sr[row][k], pr[row][k], ad);
+            }
+        if constexpr (B == 2) v = sum2(ad);
     } else if constexpr (B == 1) {
         const uint32_t s1[4] = {sr[0][0], sr[1][0], sr[2][0], sr[3][0]}, p1[4] = {pr[0][0], pr[1][0], pr[2][0], pr[3][0]};
         v = satd4_packed(s1, p1);
@@ -141,6 +148,7 @@ __device__ __forceinline__ void pred_points(const AnalyseParams& __restrict__ P,
     __syncwarp(g.mask);
     const int x0 = mbx * 16 + bx * 4, y0 = mby * 16 + by * 4;
     const uint8_t* base = P.planes[r];
+#pragma unroll 1
     for (int t = g.gl; t < total; t += GW) {
         const int c = t >> lg, b = t & ((1 << lg) - 1), bxx = b & ((1 << lgw) - 1), byy = b >> lgw;
         uint32_t pr[4][sizeof(T)];

@@ -971,7 +971,8 @@ template <class T>
 __global__ void __launch_bounds__(K7_WARPS * 32, K7_MIN_BLOCKS) decide_batch_kernel(const DecideParams* __restrict__ table,
                                                                                   const uint32_t* __restrict__ order, unsigned ntickets,
                                                                                   unsigned* ticket, const unsigned* err) {
-    __shared__ DecideSmem<T> smem[K7_WARPS];
+    extern __shared__ __align__(16) unsigned char decide_smem[];  // K7_WARPS working sets
+    DecideSmem<T>* const smem = reinterpret_cast<DecideSmem<T>*>(decide_smem);
     __shared__ DecideParams prm[K7_WARPS];
     __shared__ unsigned i4tab[9 * 17];
     fill_i4tab(i4tab);

@@ -1041,7 +1041,7 @@ __device__ void rdw_chain(const RdParams& P, DecideParams* dw, RdSmem<T, RDW_WAR
 
 // Decide mode under CABAC for one stream in the wide form: CTA i walks slice band i.
 template <class T>
-__global__ void __launch_bounds__(RDW_WARPS * 32) decide_rdw_kernel(const __grid_constant__ RdParams P) {
+__global__ void __launch_bounds__(RDW_WARPS * 32, 1) decide_rdw_kernel(const __grid_constant__ RdParams P) {
     extern __shared__ __align__(16) unsigned char rdw_smem[];
     __shared__ DecideParams dw[RDW_WARPS - 1];
     __shared__ unsigned i4tab[9 * 17];
@@ -1052,7 +1052,7 @@ __global__ void __launch_bounds__(RDW_WARPS * 32) decide_rdw_kernel(const __grid
 // The same for many streams' chains: CTA i walks chains[i] = stream << 16 | band with the stream's
 // parameters from table[stream] (copied into shared memory).
 template <class T>
-__global__ void __launch_bounds__(RDW_WARPS * 32) decide_rdw_batch_kernel(const RdParams* __restrict__ table,
+__global__ void __launch_bounds__(RDW_WARPS * 32, 1) decide_rdw_batch_kernel(const RdParams* __restrict__ table,
                                                                           const uint32_t* __restrict__ chains, int nchains) {
     extern __shared__ __align__(16) unsigned char rdw_smem[];
     __shared__ RdParams prm;

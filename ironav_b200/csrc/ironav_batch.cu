@@ -624,8 +624,11 @@ extern "C" int ironav_batch_decide(ironav_batch* b, ironav_mbstate* const* d_sta
         CK(cudaMalloc(&b->d_dtable, sizeof(DecideParams) * b->n));
         CK(cudaHostAlloc(&b->h_dtable, sizeof(DecideParams) * b->n, cudaHostAllocDefault));
         int per_sm = 0;
-        if (b->bd > 8) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decide_batch_kernel<uint16_t>, K7_WARPS * 32, 0));
-        else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decide_batch_kernel<uint8_t>, K7_WARPS * 32, 0));
+        const int s16 = K7_WARPS * (int)sizeof(DecideSmem<uint16_t>), s8 = K7_WARPS * (int)sizeof(DecideSmem<uint8_t>);
+        CK(cudaFuncSetAttribute(decide_batch_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, s16));
+        CK(cudaFuncSetAttribute(decide_batch_kernel<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, s8));
+        if (b->bd > 8) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decide_batch_kernel<uint16_t>, K7_WARPS * 32, s16));
+        else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decide_batch_kernel<uint8_t>, K7_WARPS * 32, s8));
         b->k7_blocks = std::max(1, per_sm) * b->ctx[0]->nsm;
     }
     // the staging table is reused: the previous step's copies must have left it
@@ -655,10 +658,10 @@ extern "C" int ironav_batch_decide(ironav_batch* b, ironav_mbstate* const* d_sta
     CK(cudaMemsetAsync(b->d_flags, 0, sizeof(unsigned) * b->total_mbs, b->stream));
     CK(cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned) * 2, b->stream));
     if (b->bd > 8)
-        decide_batch_kernel<uint16_t><<<b->k7_blocks, K7_WARPS * 32, 0, b->stream>>>(b->d_dtable, b->d_order, (unsigned)b->total_mbs,
+        decide_batch_kernel<uint16_t><<<b->k7_blocks, K7_WARPS * 32, K7_WARPS * sizeof(DecideSmem<uint16_t>), b->stream>>>(b->d_dtable, b->d_order, (unsigned)b->total_mbs,
                                                                                      b->d_counters, b->d_counters + 1);
     else
-        decide_batch_kernel<uint8_t><<<b->k7_blocks, K7_WARPS * 32, 0, b->stream>>>(b->d_dtable, b->d_order, (unsigned)b->total_mbs,
+        decide_batch_kernel<uint8_t><<<b->k7_blocks, K7_WARPS * 32, K7_WARPS * sizeof(DecideSmem<uint8_t>), b->stream>>>(b->d_dtable, b->d_order, (unsigned)b->total_mbs,
                                                                                     b->d_counters, b->d_counters + 1);
     return cuda_status(cudaGetLastError());
 }

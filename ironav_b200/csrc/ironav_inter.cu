@@ -168,6 +168,22 @@ int launch_planes(ironav_ctx* c, const void* d_luma, int stride, int w, int h, c
     return cuda_status(cudaGetLastError());
 }
 
+// Replay mode's kernel, when the caller has not chosen one, by how many waves of one macroblock a warp the picture is. A small
+// picture lasts as long as its slowest macroblock, which a whole warp has done soonest; a large one as long as its
+// instructions take, which groups share. Live coding's searches are short, so that 16-lane groups gain between; splitting 8x8 blocks lengthens them,
+// and the groups gain sooner; at 10 bits a group's lanes carry twice the words, and gain later. Measured (us, forms 1 / 2 / 0):
+//   352x288 82 / 105 / 142; 854x480 90 / 116 / 157, with 8x8 splits and two references 522 / 679 / 803; 1280x720 137 / 136 / 178, splits
+//   934 / 895 / 1023, live 50 / 46 / 57; 1600x900 179 / 193 / 200; 1920x1080 219 / 208 / 212, splits 1726 / 1526 / 1186, live 74 / 71 / 75;
+//   3840x2160 737 / 693 / 589, live 245 / 208 / 192; 10 bits: 1920x1080 266 / 275 / 298, splits 1926 / 1992 / 1656; 2560x1440 439 / 458 / 448;
+//   3840x2160 944 / 971 / 877.
+int replay_form(const ironav_ctx* c) {
+    if (c->replay_form >= 0) return c->replay_form;
+    const int wave = c->k2_blocks * K2_WARPS;
+    if (c->fast) return c->nmb <= wave ? 1 : (c->nmb <= 7 * wave ? 2 : 0);
+    if (c->sub8) return c->nmb <= wave ? 1 : (c->nmb <= 2 * wave ? (c->bd > 8 ? 1 : 2) : 0);
+    return c->nmb <= (c->bd > 8 ? 7 : 3) * wave ? 1 : 0;
+}
+
 int launch_analyse(ironav_ctx* c, bool auto_mode, const ironav_mbstate* d_in, ironav_mbstate* d_out, ironav_mbresult* d_res) {
     AnalyseParams p;
     fill_params(c, p);
@@ -183,7 +199,8 @@ int launch_analyse(ironav_ctx* c, bool auto_mode, const ironav_mbstate* d_in, ir
     p.wait_limit = c->wait_limit;
     if (auto_mode) p.epoch = ++c->epoch;
     CK(cudaMemsetAsync(c->d_counters, 0, 2 * sizeof(unsigned), c->stream));
-    if (!auto_mode && c->replay_form != 1 && p.learned == nullptr) {
+    const int form = replay_form(c);
+    if (!auto_mode && form != 1 && p.learned == nullptr) {
         // replay mode: one macroblock per group of 8 (or 16) lanes
         // a grid of at most the CTAs the picture's macroblocks fill (one macroblock a group), so that no
         // SM holds warps that find no work while others hold more than their share
@@ -191,10 +208,10 @@ int launch_analyse(ironav_ctx* c, bool auto_mode, const ironav_mbstate* d_in, ir
             const int per_cta = g8::warps_for(gw) * (32 / gw);
             return std::max(1, std::min(resident, (c->nmb + per_cta - 1) / per_cta));
         };
-        if (c->replay_form == 2) {
+        if (form == 2) {
             if (c->bd > 8) g8::analyse_replay_g8_kernel<uint16_t, 16><<<grid(c->g16_blocks, 16), g8::warps_for(16) * 32, 0, c->stream>>>(p);
             else g8::analyse_replay_g8_kernel<uint8_t, 16><<<grid(c->g16_blocks, 16), g8::warps_for(16) * 32, 0, c->stream>>>(p);
-        } else if (c->replay_form == 3) {
+        } else if (form == 3) {
             if (c->bd > 8) g8::analyse_replay_g8_kernel<uint16_t, 4><<<grid(c->g4_blocks, 4), g8::warps_for(4) * 32, 0, c->stream>>>(p);
             else g8::analyse_replay_g8_kernel<uint8_t, 4><<<grid(c->g4_blocks, 4), g8::warps_for(4) * 32, 0, c->stream>>>(p);
         } else {
@@ -358,7 +375,6 @@ int ironav_ctx_create(ironav_ctx** out, int width, int height, int bd, int max_r
     c->width = width;
     c->height = height;
     c->bd = bd;
-    c->replay_form = bd > 8 ? 1 : 0;  // the faster replay kernel at each depth (8-lane groups at 8 bits)
     c->mb_w = mb_w;
     c->mb_h = mb_h;
     c->pw = mb_w * 16;
