@@ -253,62 +253,6 @@ __device__ __forceinline__ int pred_mode(const int* nbm, const uint8_t* cur, int
     return (a >= 0 && b >= 0) ? min(a, b) : 2;
 }
 
-// write_block, enc/cabac.rs:194-250: coded_block_flag (context cbf, none when < 0), then the significance map
-// (significant_coeff_flag, last_significant_coeff_flag) and the levels (coeff_abs_level_minus1 and the signs) of a block of
-// category cat with max levels in scan order.
-template <class S>
-__device__ __forceinline__ void block(S& c, int cat, int cbf, const int16_t* lv, int max) {
-    unsigned long long nz = 0;
-    for (int i = 0; i < max; i++) nz |= (unsigned long long)(lv[i] != 0) << i;
-    if (cbf >= 0) c.decision(cbf, nz != 0);
-    if (nz == 0) return;
-    const int last = 63 - __clzll((long long)nz);
-    const int so = SIG_OFF[0][cat], lo = LAST_OFF[0][cat];
-    for (int i = 0; i < max - 1 && i <= last; i++) {
-        // 4:2:0 chroma DC has three significance contexts, one per position; 8x8 blocks share theirs
-        const int sig = cat == 3 ? min(i, 2) : cat == 5 ? SIG_OFF_8X8[0][i] : i;
-        const int lst = cat == 3 ? min(i, 2) : cat == 5 ? LAST_OFF_8X8[i] : i;
-        const int bit = (int)((nz >> i) & 1u);
-        c.decision(so + sig, bit);
-        if (bit) c.decision(lo + lst, i == last);
-    }
-    const int base = ABS_OFF[cat];
-    int eq1 = 0, gt1 = 0;
-    while (nz) {
-        const int i = 63 - __clzll((long long)nz);
-        nz &= ~(1ull << i);
-        const int l = lv[i];
-        const uint32_t a = (uint32_t)abs(l);
-        const int inc0 = gt1 ? 0 : min(1 + eq1, 4);
-        if (a == 1) {
-            c.decision(base + inc0, 0);
-            eq1++;
-        } else {
-            c.decision(base + inc0, 1);
-            const int incn = base + 5 + min(gt1, 4 - (cat == 3));
-            // abs - 2 ones and a zero, the ones capped at 13 with the rest in an Exp-Golomb suffix
-            const uint32_t ones = a - 2 < 13 ? a - 2 : 13;
-            for (uint32_t k = 0; k < ones; k++) c.decision(incn, 1);
-            if (a < 15) c.decision(incn, 0);
-            else {
-                uint32_t v = a - 15, k = 0;  // exp_golomb(abs - 15, 0), enc/cabac.rs:17-29
-                while (v >= (1u << k)) {
-                    c.bypass(1);
-                    v -= 1u << k;
-                    k++;
-                }
-                c.bypass(0);
-                while (k > 0) {
-                    k--;
-                    c.bypass((v >> k) & 1);
-                }
-            }
-            gt1++;
-        }
-        c.bypass(l < 0);
-    }
-}
-
 // mvd_bins, enc/frame.rs:2393-2414
 template <class S>
 __device__ __forceinline__ void mvd(S& c, int comp, int d, uint32_t sum) {
@@ -474,28 +418,73 @@ __device__ __forceinline__ void head_last(S& c, const Slice& sl, const ironav_mb
     c.decision(60, 0);  // mb_qp_delta 0, after a macroblock without a change
 }
 
-// Residual block i (0..RES_BLOCKS - 1, in coding order) of a macroblock: 0 the Intra16x16 DC; 1..16 the luma blocks (4x4 in
-// decoding order, or 1..4 the 8x8 ones); 17, 18 chroma DC; 19..26 chroma AC.
-constexpr int RES_BLOCKS = 27;
-template <class S>
-__device__ __forceinline__ void res_block(S& c, const ironav_mbcode* code, const Nb& L, const Nb& T, int i) {
+// The exclusive prefix sum of v over the warp; the total on every lane.
+__device__ __forceinline__ int warp_scan(int v, int* total) {
+    const int lane = threadIdx.x & 31;
+    int x = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
+    }
+    *total = __shfl_sync(0xffffffffu, x, 31);
+    return x - v;
+}
+
+// The map contexts per scan position, a nibble each: a position's own number, or for the quarters of an 8x8 block significant_coeff_flag's
+// and last_significant_coeff_flag's of Table 9-43 (frame coded).
+constexpr unsigned long long MAP_OWN = 0xFEDCBA9876543210ull;
+__device__ __forceinline__ unsigned long long map_sig8(int part) {
+    return part == 0 ? 0x5544433445543210ull : part == 1 ? 0x789A987776334444ull : part == 2 ? 0xB689AE9876BDCB67ull : 0x0CAEBDCB9AE96BDCull;
+}
+__device__ __forceinline__ unsigned long long map_last8(int part) {
+    return part == 0 ? 0x1111111111111110ull : part == 1 ? 0x2222222222222222ull : part == 2 ? 0x4444444433333333ull : 0x0888777766665555ull;
+}
+
+// A lane's share of a macroblock's residual bins (write_block, enc/cabac.rs:194-250: coded_block_flag, the significance map and the
+// levels of a block): a block of up to 16 levels, or a quarter of an 8x8 block's 64. Its map bins lie together, and so do its level
+// bins, which run from the last position down; `os` and `ol` are where in the macroblock's residual bins. Lane 0: the Intra16x16
+// DC; 1-16: the luma blocks (4x4 in decoding order, or four lanes an 8x8 block); 17, 18: chroma DC; 19-26: chroma AC. What its
+// bins hang on across the quarters is known from the block's masks of non-zero levels and of those above 1, so that the quarters
+// are counted without a walk and listed side by side. (With a lane an 8x8 block, each block walked twice, the price of an
+// Intra8x8 macroblock took 12 to 16 us, of an Intra4x4 one 10; with the quarters, the decide of an IDR and three P pictures at
+// 1080p went from 126 to 118 ms.)
+struct ResPiece {
+    const int16_t* lv;           // its levels, in scan order
+    unsigned long long sig, lst;  // its positions' map contexts
+    int so, lo, ab, cbf;         // the contexts' bases; coded_block_flag's context (-1: none)
+    int cnt, last;               // its positions in the map; the block's last non-zero position, from its first
+    unsigned nz;                 // its non-zero levels
+    int eq, gt;                  // the block's levels of 1 and above 1 after its own
+    int capn;                    // contexts of a level's further bins
+    int os, ns, ol, nl;
+    bool coded;                  // the block has a non-zero level
+};
+
+// Every lane's share; BYP: the bypass bins count as bins, and otherwise as 256 of `bits` each. Returns all lanes' bins.
+template <bool BYP>
+__device__ __forceinline__ int res_pieces(ResPiece& r, const ironav_mbcode* code, const Nb& L, const Nb& T, uint32_t* bits) {
+    const int i = threadIdx.x & 31;
     const bool la = L.avail, ta = T.avail;
     const int kind = code->kind, cbp = code->res.cbp, cbpl = cbp & 15, cbpc = cbp >> 4;
+    const bool t8 = code->res.t8x8;
     // an unavailable neighbour counts as a coded block for an intra macroblock
     const int un = kind != KIND_INTER;
-    int cat, cbf, max;
-    const int16_t* lv;
-    if (i == 0) {
-        if (kind != KIND_I16) return;
-        cat = 0, max = 16, lv = code->dc;
-        cbf = 85 + (la ? (L.cbf_dc & 1) != 0 : un) + 2 * (ta ? (T.cbf_dc & 1) != 0 : un);
+    int cat = 0, cbf = -1, max = 0, part = 0;
+    const int16_t* lv = code->dc;
+    if (code->skip || !(cbp || kind == KIND_I16)) {
+    } else if (i == 0) {
+        if (kind == KIND_I16) {
+            max = 16;
+            cbf = 85 + (la ? (L.cbf_dc & 1) != 0 : un) + 2 * (ta ? (T.cbf_dc & 1) != 0 : un);
+        }
     } else if (i < 17) {
         const int n = i - 1;
-        if (code->res.t8x8) {
-            if (n >= 4 || !(cbpl & (1 << n))) return;
-            cat = 5, cbf = -1, max = 64, lv = code->res.luma8[n];
+        if (!(cbpl & (1 << (n >> 2)))) {
+        } else if (t8) {
+            part = n & 3;
+            cat = 5, max = 16, lv = code->res.luma8[n >> 2] + 16 * part;
         } else {
-            if (!(cbpl & (1 << (n >> 2)))) return;
             const int bx = ((n >> 2) & 1) * 2 + (n & 1), by = ((n >> 3) & 1) * 2 + ((n >> 1) & 1);
             const int fa = bx > 0 ? code->res.nnz[by * 4 + bx - 1] > 0 : (la ? L.nnz[by * 4 + 3] > 0 : un);
             const int fb = by > 0 ? code->res.nnz[(by - 1) * 4 + bx] > 0 : (ta ? T.nnz[12 + bx] > 0 : un);
@@ -504,19 +493,130 @@ __device__ __forceinline__ void res_block(S& c, const ironav_mbcode* code, const
             lv = code->res.luma[by * 4 + bx] + (i16 ? 1 : 0);
         }
     } else if (i < 19) {
-        if (cbpc == 0) return;
-        const int comp = i - 17, m = 2 << comp;
-        cat = 3, max = 4, lv = code->res.cdc[comp];
-        cbf = 97 + (la ? (L.cbf_dc & m) != 0 : un) + 2 * (ta ? (T.cbf_dc & m) != 0 : un);
-    } else {
-        if (cbpc != 2) return;
+        if (cbpc != 0) {
+            const int comp = i - 17, m = 2 << comp;
+            cat = 3, max = 4, lv = code->res.cdc[comp];
+            cbf = 97 + (la ? (L.cbf_dc & m) != 0 : un) + 2 * (ta ? (T.cbf_dc & m) != 0 : un);
+        }
+    } else if (i < 27 && cbpc == 2) {
         const int comp = (i - 19) >> 2, blk = (i - 19) & 3, bx = blk & 1, by = blk >> 1;
         const uint8_t* cur = code->res.cnnz[comp];
         const int fa = bx > 0 ? cur[by * 2] > 0 : (la ? L.cnnz[comp][by * 2 + 1] > 0 : un);
         const int fb = by > 0 ? cur[bx] > 0 : (ta ? T.cnnz[comp][2 + bx] > 0 : un);
         cat = 4, max = 15, lv = code->res.cac[comp][blk] + 1, cbf = 101 + fa + 2 * fb;
     }
-    block(c, cat, cbf, lv, max);
+    // its own levels: which are there, which are above 1, and their bins (a level's context bins: its magnitude, 14 at most)
+    unsigned nz = 0, big = 0;
+    int dec = 0, byp = 0;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        const int a = k < max ? abs((int)lv[k]) : 0;
+        nz |= (unsigned)(a != 0) << k;
+        big |= (unsigned)(a > 1) << k;
+        dec += min(a, 14);
+        if (a >= 15) byp += 2 * (31 - __clz(a - 14)) + 1;
+    }
+    byp += __popc(nz);
+    const int len = BYP ? dec + byp : dec;
+    // the block: its masks, and the level bins of the quarters after this one
+    unsigned long long bnz = nz, bbig = big;
+    int above = 0;
+    const bool quarter = t8 && i >= 1 && i <= 16;
+    const int head = quarter ? i - ((i - 1) & 3) : i;  // the block's first lane
+    if (t8) {
+        unsigned m[4];
+        int l[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int from = quarter ? head + q : i;
+            m[q] = __shfl_sync(0xffffffffu, nz | big << 16, from);
+            l[q] = __shfl_sync(0xffffffffu, len, from);
+        }
+        if (quarter) {
+            bnz = (unsigned long long)((m[0] & 0xffffu) | m[1] << 16) | (unsigned long long)((m[2] & 0xffffu) | m[3] << 16) << 32;
+            bbig = (unsigned long long)(m[0] >> 16 | (m[1] & 0xffff0000u)) | (unsigned long long)(m[2] >> 16 | (m[3] & 0xffff0000u)) << 32;
+#pragma unroll
+            for (int q = 1; q < 4; q++) above += q > part ? l[q] : 0;
+        }
+    }
+    const int p0 = 16 * part, last = 63 - __clzll((long long)bnz), all = cat == 5 ? 64 : max;
+    const int maps = min(last + 1, all - 1);  // the block's positions in the map (the last position of all has no bins)
+    const int mine = bnz ? min(max - (cat == 5 ? 0 : 1), maps - p0) : 0;
+    auto below = [](unsigned long long m, int n) { return __popcll(n >= 64 ? m : m & ((1ull << n) - 1)); };  // of the first n positions
+    const int flag = part == 0 && cbf >= 0, c0 = cbf >= 0;
+    r.lv = lv;
+    r.sig = cat == 5 ? map_sig8(part) : MAP_OWN;
+    r.lst = cat == 5 ? map_last8(part) : MAP_OWN;
+    r.so = SIG_OFF[0][cat];
+    r.lo = LAST_OFF[0][cat];
+    r.ab = ABS_OFF[cat];
+    r.capn = 4 - (cat == 3);
+    r.cbf = cbf;
+    r.cnt = mine > 0 ? mine : 0;
+    r.last = last - p0;
+    r.nz = nz;
+    const unsigned long long up = part == 3 || !quarter ? 0ull : bnz >> (p0 + 16), upb = part == 3 || !quarter ? 0ull : bbig >> (p0 + 16);
+    r.gt = __popcll(upb);
+    r.eq = __popcll(up) - r.gt;
+    r.coded = bnz != 0;
+    r.ns = flag + r.cnt + below(nz, r.cnt);
+    r.nl = len;
+    *bits = BYP ? 0u : 256u * (uint32_t)byp;
+    int total;
+    const int at = warp_scan(r.ns + r.nl, &total), base = __shfl_sync(0xffffffffu, at, head);
+    // the map bins of the quarters before it; then, after all the block's, the level bins of the quarters after it
+    const int maps_all = bnz ? maps : 0, before = min(p0, maps_all);
+    r.os = base + (quarter ? before + below(bnz, before) : 0);
+    r.ol = base + c0 + maps_all + below(bnz, maps_all) + above;
+    return total;
+}
+
+template <class S>
+__device__ __forceinline__ void list_map(S& c, const ResPiece& r) {
+    if (r.ns > 0 && r.cbf >= 0) c.decision(r.cbf, r.coded);
+    for (int k = 0; k < r.cnt; k++) {
+        const int bit = (int)((r.nz >> k) & 1u);
+        c.decision(r.so + (int)((r.sig >> (4 * k)) & 15u), bit);
+        if (bit) c.decision(r.lo + (int)((r.lst >> (4 * k)) & 15u), k == r.last);
+    }
+}
+
+template <class S>
+__device__ __forceinline__ void list_levels(S& c, const ResPiece& r) {
+    int eq1 = r.eq, gt1 = r.gt;
+    for (unsigned nz = r.nz; nz;) {
+        const int i = 31 - __clz((int)nz);
+        nz ^= 1u << i;
+        const int l = r.lv[i];
+        const uint32_t a = (uint32_t)abs(l);
+        const int inc0 = gt1 ? 0 : min(1 + eq1, 4);
+        if (a == 1) {
+            c.decision(r.ab + inc0, 0);
+            eq1++;
+        } else {
+            c.decision(r.ab + inc0, 1);
+            const int incn = r.ab + 5 + min(gt1, r.capn);
+            // abs - 2 ones and a zero, the ones capped at 13 with the rest in an Exp-Golomb suffix
+            const uint32_t ones = a - 2 < 13 ? a - 2 : 13;
+            for (uint32_t k = 0; k < ones; k++) c.decision(incn, 1);
+            if (a < 15) c.decision(incn, 0);
+            else {
+                uint32_t v = a - 15, k = 0;  // exp_golomb(abs - 15, 0), enc/cabac.rs:17-29
+                while (v >= (1u << k)) {
+                    c.bypass(1);
+                    v -= 1u << k;
+                    k++;
+                }
+                c.bypass(0);
+                while (k > 0) {
+                    k--;
+                    c.bypass((v >> k) & 1);
+                }
+            }
+            gt1++;
+        }
+        c.bypass(l < 0);
+    }
 }
 
 // mb_skip_flag of a P slice's macroblock.
@@ -526,8 +626,8 @@ __device__ __forceinline__ void skip_bin(S& c, const ironav_mbcode* code, const 
 }
 
 // The bins of a macroblock, mb_bins (enc/frame.rs:2028-2279) for I and P slices, are listed by a warp: a lane walks each piece (the
-// head's pieces, then the residual blocks, all independent given the code and its neighbours), once to count its bins and
-// once, at the offset a scan of the counts gives, to list them. (One lane walking a macroblock's bins one by one spent 40 us on a
+// head's pieces, then the residual's shares, all independent given the code and its neighbours) at the offset a scan of the
+// pieces' counts gives. (One lane walking a macroblock's bins one by one spent 40 us on a
 // coded macroblock's candidates and 49 us on writing an intra macroblock.) A listed bin: its context, bin << 10, and
 // whether it is a bypass (or, with both, a terminate) bin.
 constexpr uint32_t BIN_BYPASS = 1u << 11, BIN_TERMINATE = 1u << 12;
@@ -559,8 +659,8 @@ struct BinList {
     __device__ __forceinline__ void terminate(int bin) { *p++ = (uint16_t)(BIN_TERMINATE | (bin != 0) << 10); }
 };
 
-// This lane's two pieces of a macroblock's bins, in coding order over (piece, lane): the head (lane 0 the skip flag and
-// head_first, lanes 1-16 the parts, lane 17 head_last) and a residual block.
+// This lane's piece of a macroblock's head bins, in coding order over the lanes: lane 0 the skip flag and head_first, lanes 1-16 the
+// parts, lane 17 head_last.
 template <class S>
 __device__ __forceinline__ void lane_head(S& c, const Slice& sl, const ironav_mbcode* code, const Nb& L, const Nb& T, const int* nbm) {
     const int lane = threadIdx.x & 31;
@@ -573,29 +673,10 @@ __device__ __forceinline__ void lane_head(S& c, const Slice& sl, const ironav_mb
         head_last(c, sl, code, L, T);
     }
 }
-template <class S>
-__device__ __forceinline__ void lane_block(S& c, const ironav_mbcode* code, const Nb& L, const Nb& T) {
-    const int lane = threadIdx.x & 31;
-    if (lane < RES_BLOCKS && !code->skip && (code->res.cbp || code->kind == KIND_I16)) res_block(c, code, L, T, lane);
-}
-
-// The exclusive prefix sum of v over the warp; the total on every lane.
-__device__ __forceinline__ int warp_scan(int v, int* total) {
-    const int lane = threadIdx.x & 31;
-    int x = v;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, off);
-        if (lane >= off) x += y;
-    }
-    *total = __shfl_sync(0xffffffffu, x, 31);
-    return x - v;
-}
-
-// Bins a price's list holds. A piece never has more (63 positions of an 8x8 block with two map bins each, 64 levels of at most 14
-// context bins); a macroblock's pieces that together do are listed in several turns.
+// Bins a price's list holds. A piece never has more (a share's map bins, or its 16 levels of at most 14 context bins); a macroblock's
+// pieces that together do are listed in several turns.
 constexpr int PRICE_CAP = 1152;
-static_assert(2 * 63 + 64 * 14 <= PRICE_CAP, "one block fits the list");
+static_assert(16 * 14 <= PRICE_CAP && 1 + 2 * 16 <= PRICE_CAP, "one piece fits the list");
 
 // The cost in 1/256 bits of the listed decisions, their contexts advanced in st (CabacCost, enc/cabac.rs:150-192). 32 bins a
 // turn, in order: the bins of a context form a chain, walked by its first lane, the contexts side by side.
@@ -632,26 +713,32 @@ __device__ __forceinline__ uint32_t price(const uint8_t* live, uint8_t* st, cons
     uint4* d16 = reinterpret_cast<uint4*>(st);
     d16[lane] = s16[lane];
     d16[lane + 32] = s16[lane + 32];
-    PriceCount h, r;
+    PriceCount h;
     lane_head(h, sl, code, L, T, nbm);
-    lane_block(r, code, L, T);
-    int nh, nr;
-    const int oh = warp_scan(h.n, &nh), orr = nh + warp_scan(r.n, &nr), total = nh + nr;
-    uint32_t bits = h.bits + r.bits;
+    ResPiece r;
+    uint32_t bits;
+    int nh;
+    const int nr = res_pieces<false>(r, code, L, T, &bits), oh = warp_scan(h.n, &nh), total = nh + nr;
+    bits += h.bits;
     __syncwarp();
     int base = 0;
     do {
         // the pieces that lie in [base, base + PRICE_CAP): a run of whole ones from base on
-        const bool fh = h.n && oh >= base && oh + h.n <= base + PRICE_CAP, fr = r.n && orr >= base && orr + r.n <= base + PRICE_CAP;
+        auto fits = [&](int at, int n) { return n > 0 && at >= base && at + n <= base + PRICE_CAP; };
+        const bool fh = fits(oh, h.n), fm = fits(nh + r.os, r.ns), fl = fits(nh + r.ol, r.nl);
         if (fh) {
             PriceList c = {list + (oh - base)};
             lane_head(c, sl, code, L, T, nbm);
         }
-        if (fr) {
-            PriceList c = {list + (orr - base)};
-            lane_block(c, code, L, T);
+        if (fm) {
+            PriceList c = {list + (nh + r.os - base)};
+            list_map(c, r);
         }
-        const int end = __reduce_max_sync(0xffffffffu, max(fh ? oh + h.n : 0, fr ? orr + r.n : 0));
+        if (fl) {
+            PriceList c = {list + (nh + r.ol - base)};
+            list_levels(c, r);
+        }
+        const int end = __reduce_max_sync(0xffffffffu, max(fh ? oh + h.n : 0, max(fm ? nh + r.os + r.ns : 0, fl ? nh + r.ol + r.nl : 0)));
         __syncwarp();
         bits += price_list(list, end - base, st, step);
         base = end;

@@ -40,7 +40,7 @@ template <class T, int W>
 struct RdSmem {
     DecideSmem<T> s[W];              // each warp's working set
     ironav_mbcode cand[RD_CANDS];    // the candidates' codes
-    T crec[RD_CANDS][384];           // and reconstructions (luma, Cb, Cr)
+    __align__(16) T crec[RD_CANDS][384];  // and reconstructions (luma, Cb, Cr)
     __align__(16) uint8_t live[1024];           // the chain's contexts after the macroblocks before this one
     __align__(16) uint8_t cst[RD_CANDS][1024];  // each candidate's copy, advanced by its bins
     uint16_t list[W][cab::PRICE_CAP];           // each warp's list of bins
@@ -339,33 +339,53 @@ __device__ __forceinline__ void code_init(ironav_mbcode* o) {
 // only, the chroma added later from another candidate's. The candidate counts from here on.
 template <class T, int W>
 __device__ void rd_take(const CodeParams& C, RdSmem<T, W>& R, const DecideSmem<T>& S, int k, int mbx, int mby, bool chroma = true) {
+    // a lane's half row of luma and four chroma samples, as words; a sum of 384 squared differences of 10 bits fits 32 bits
     const int lane = threadIdx.x & 31;
-    const T* SC = reinterpret_cast<const T*>(C.src_c);
-    T* dst = R.crec[k];
+    constexpr int B = (int)sizeof(T);
+    uint32_t* const dst = reinterpret_cast<uint32_t*>(R.crec[k]);
     __syncwarp();
-    long long ssd = 0, cssd = 0;
-    for (int i = lane; i < (chroma ? 384 : 256); i += 32) {
-        int r, s;
-        if (i < 256) {
-            r = reinterpret_cast<const T*>(C.rec[0])[(size_t)(mby * 16 + (i >> 4)) * C.ys + mbx * 16 + (i & 15)];
-            s = src_at(S.a, i & 15, i >> 4);
+    auto squares = [](uint32_t a, uint32_t b, uint32_t acc) {
+        if constexpr (B == 1) {
+            const uint32_t d = __vabsdiffu4(a, b);
+            return __dp4a(d, d, acc);
         } else {
-            const int cc = (i - 256) >> 6, j = (i - 256) & 63, cy = mby * 8 + (j >> 3), cx = mbx * 8 + (j & 7);
-            r = reinterpret_cast<const T*>(C.rec[1 + cc])[(size_t)cy * C.cs + cx];
-            s = SC[(size_t)cc * C.cw * C.ch + (size_t)cy * C.cw + cx];
+            const int lo = (int)(a & 0xffffu) - (int)(b & 0xffffu), hi = (int)(a >> 16) - (int)(b >> 16);
+            return acc + (uint32_t)(lo * lo) + (uint32_t)(hi * hi);
         }
-        dst[i] = (T)r;
-        const long long d = s - r;
-        if (i < 256) ssd += d * d;
-        else cssd += d * d;
-    }
+    };
+    uint32_t ssd = 0, cssd = 0;
+    {
+        const int row = lane >> 1, half = lane & 1;
+        const uint32_t* rec = reinterpret_cast<const uint32_t*>(reinterpret_cast<const T*>(C.rec[0]) + (size_t)(mby * 16 + row) * C.ys + mbx * 16 + half * 8);
+        const uint32_t* src = &S.a.src[(row * 4 + half * 2) * B];
+        uint32_t v[2 * B], cv[B], cs[B];
 #pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-        ssd += __shfl_xor_sync(FULL, ssd, off);
-        cssd += __shfl_xor_sync(FULL, cssd, off);
+        for (int i = 0; i < 2 * B; i++) v[i] = rec[i];
+        if (chroma) {
+            const int cc = lane >> 4, j = (lane & 15) * 4;
+            const size_t at = (size_t)(mby * 8 + (j >> 3));
+            const uint32_t* crec = reinterpret_cast<const uint32_t*>(reinterpret_cast<const T*>(C.rec[1 + cc]) + at * C.cs + mbx * 8 + (j & 7));
+            const uint32_t* csrc = reinterpret_cast<const uint32_t*>(reinterpret_cast<const T*>(C.src_c) + (size_t)cc * C.cw * C.ch + at * C.cw + mbx * 8 + (j & 7));
+#pragma unroll
+            for (int i = 0; i < B; i++) cv[i] = crec[i], cs[i] = csrc[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 2 * B; i++) {
+            dst[lane * 2 * B + i] = v[i];
+            ssd = squares(v[i], src[i], ssd);
+        }
+        if (chroma) {
+#pragma unroll
+            for (int i = 0; i < B; i++) {
+                dst[64 * B + lane * B + i] = cv[i];
+                cssd = squares(cv[i], cs[i], cssd);
+            }
+            cssd = __reduce_add_sync(FULL, cssd);
+        }
+        ssd = __reduce_add_sync(FULL, ssd);
     }
     if (lane == 0) {
-        R.ssd[k] = ssd + cssd;
+        R.ssd[k] = (long long)(ssd + cssd);
         R.cssd[k] = cssd;
         R.valid[k] = 1;
     }
@@ -995,14 +1015,17 @@ __device__ int rd_group(const RdParams& P, const DecideParams* dw, RdSmem<T, RDW
         uint32_t* d32 = reinterpret_cast<uint32_t*>(&D.codes[mb]);
         for (int i = lane; i < (int)(sizeof(ironav_mbcode) / 4); i += 32) d32[i] = s32[i];
     } else if (w == 2) {
-        const T* rec = R.crec[b];
-        for (int i = lane; i < 256; i += 32) reinterpret_cast<T*>(C.rec[0])[(size_t)(mby * 16 + (i >> 4)) * C.ys + mbx * 16 + (i & 15)] = rec[i];
+        const int row = lane >> 1, half = lane & 1;
+        const uint32_t* rec = reinterpret_cast<const uint32_t*>(R.crec[b]) + lane * 2 * (int)sizeof(T);
+        uint32_t* d = reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(C.rec[0]) + (size_t)(mby * 16 + row) * C.ys + mbx * 16 + half * 8);
+#pragma unroll
+        for (int i = 0; i < 2 * (int)sizeof(T); i++) d[i] = rec[i];
     } else if (w == 3) {
-        const T* rec = R.crec[b] + 256;
-        for (int i = lane; i < 128; i += 32) {
-            const int cc = i >> 6, j = i & 63;
-            reinterpret_cast<T*>(C.rec[1 + cc])[(size_t)(mby * 8 + (j >> 3)) * C.cs + mbx * 8 + (j & 7)] = rec[i];
-        }
+        const int cc = lane >> 4, j = (lane & 15) * 4;
+        const uint32_t* rec = reinterpret_cast<const uint32_t*>(R.crec[b]) + (64 + lane) * (int)sizeof(T);
+        uint32_t* d = reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(C.rec[1 + cc]) + (size_t)(mby * 8 + (j >> 3)) * C.cs + mbx * 8 + (j & 7));
+#pragma unroll
+        for (int i = 0; i < (int)sizeof(T); i++) d[i] = rec[i];
     } else {
         const uint4* c16 = reinterpret_cast<const uint4*>(R.cst[b]);
         uint4* l16 = reinterpret_cast<uint4*>(R.live);
@@ -1119,7 +1142,8 @@ static __global__ void __launch_bounds__(128) cabac_nb_kernel(const __grid_const
 // bounded; a warp that gives up stops the others, and the picture is reported like one that outgrew its region.
 constexpr int WR_LISTERS = 6;
 constexpr int WR_THREADS = (2 + WR_LISTERS) * 32;
-constexpr int WR_CAP = 3328;   // bins a list holds: at least one piece's most (126 map bins and 64 levels of up to 48)
+constexpr int WR_CAP = 3328;   // bins a list holds: at least one piece's most (16 levels of up to 48 bins)
+static_assert(16 * 48 <= WR_CAP, "one piece fits the list");
 constexpr int WR_RING = 512;   // bins between the states and the coder
 constexpr unsigned WR_SPINS = 1u << 28;
 
@@ -1270,25 +1294,33 @@ static __global__ void __launch_bounds__(WR_THREADS) cabac_write_kernel(const __
                 nbm[4 + q] = ta ? T.bmodes[q] : -1;
             }
             // the pieces' bins, end_of_slice_flag after the last block's
-            cab::BinCount h, r;
+            cab::BinCount h;
             cab::lane_head(h, sl, code, L.nb, T.nb, nbm);
-            cab::lane_block(r, code, L.nb, T.nb);
-            if (lane == 31) r.terminate(0);
-            int nh, nr;
-            const int oh = cab::warp_scan(h.n, &nh), orr = nh + cab::warp_scan(r.n, &nr), total = nh + nr;
+            cab::ResPiece r;
+            uint32_t bits;
+            int nh;
+            const int nr = cab::res_pieces<true>(r, code, L.nb, T.nb, &bits), oh = cab::warp_scan(h.n, &nh), total = nh + nr + 1;
             for (int base = 0; base < total;) {
                 if (!__all_sync(FULL, wr_wait(S, &S.taken[l], turn))) return;
-                const bool fh = h.n && oh >= base && oh + h.n <= base + WR_CAP, fr = r.n && orr >= base && orr + r.n <= base + WR_CAP;
+                auto fits = [&](int at, int n) { return n > 0 && at >= base && at + n <= base + WR_CAP; };
+                const bool fh = fits(oh, h.n), fm = fits(nh + r.os, r.ns), fl = fits(nh + r.ol, r.nl), ft = lane == 31 && fits(total - 1, 1);
                 if (fh) {
                     cab::BinList c = {&S.list[l][oh - base]};
                     cab::lane_head(c, sl, code, L.nb, T.nb, nbm);
                 }
-                if (fr) {
-                    cab::BinList c = {&S.list[l][orr - base]};
-                    cab::lane_block(c, code, L.nb, T.nb);
-                    if (lane == 31) c.terminate(mb + 1 == end);
+                if (fm) {
+                    cab::BinList c = {&S.list[l][nh + r.os - base]};
+                    cab::list_map(c, r);
                 }
-                const int to = __reduce_max_sync(FULL, max(fh ? oh + h.n : 0, fr ? orr + r.n : 0));
+                if (fl) {
+                    cab::BinList c = {&S.list[l][nh + r.ol - base]};
+                    cab::list_levels(c, r);
+                }
+                if (ft) {
+                    cab::BinList c = {&S.list[l][total - 1 - base]};
+                    c.terminate(mb + 1 == end);
+                }
+                const int to = __reduce_max_sync(FULL, max(max(fh ? oh + h.n : 0, fm ? nh + r.os + r.ns : 0), max(fl ? nh + r.ol + r.nl : 0, ft ? total : 0)));
                 __syncwarp();
                 turn++;
                 if (lane == 0) {
