@@ -1,8 +1,7 @@
-// cabac.cuh — CABAC on the device: the contexts of a slice, and one macroblock's bins (mb_bins,
-// enc/frame.rs:2028-2279, with write_block, enc/cabac.rs:194-250, and mvd_bins, enc/frame.rs:2393-2414) given
-// to a sink that is either the bit counter (CabacCost, enc/cabac.rs:150-192) or the arithmetic coder
-// (CabacWriter, enc/cabac.rs:42-147). A macroblock's bins are a serial walk, so one lane runs it; several
-// lanes can each count another candidate's bins from their own copy of the contexts.
+// cabac.cuh — CABAC on the device: the contexts of a slice, one macroblock's bins (mb_bins,
+// enc/frame.rs:2028-2279, with write_block, enc/cabac.rs:194-250, and mvd_bins, enc/frame.rs:2393-2414), listed by the
+// lanes of a warp, their price (CabacCost, enc/cabac.rs:150-192), and the arithmetic coder
+// (CabacWriter, enc/cabac.rs:42-147).
 //
 // The walk reads the macroblock's code and what the contexts need of its left and top neighbours in the
 // slice (Nb, the CABAC fields of MbState, enc/frame.rs:245-272). Only I and P slices are coded here.

@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(32) decide_rd_batch_kernel(const RdParams* __r
 //   - the commit of the kept one (code, reconstruction, contexts, state) by a warp each.
 // The warps meet at CTA barriers (after the tests; after the P_Skip macroblocks' commits; and, when there are candidates, after
 // them and after the commit), every warp at every one. An IDR and three P pictures at 1080p, 8 bands: 248 ms with three warps a
-// chain (P_Skip tested one macroblock at a time, each candidate's bins walked by nine lanes), 138 ms in this form.
+// chain (P_Skip tested one macroblock at a time, each candidate's bins walked by nine lanes), 118 ms in this form.
 constexpr int RDW_WARPS = 5;
 
 // skip_mv (enc/frame.rs:597-603) from a macroblock's table of neighbours, with its left neighbour's block a.

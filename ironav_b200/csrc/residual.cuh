@@ -327,7 +327,7 @@ __device__ __forceinline__ void st4(T* p, const int* v) {
 // 20-23 Cr. Returns the coded block pattern, on every lane.
 // Bound by the instructions of one warp, a block's transform and quantiser chain being its serial part: with luma and chroma one after
 // the other, each sample its own load and store, and a shuffle a block for the decimation sums, a 1080p picture took 24 us (now 17),
-// the closed-loop decide 8.3 ms (now 6.8), the CABAC decide of IDR + 3 P 133 ms (now 126), that of 16 pictures at once 35.8 (now 33.3).
+// the closed-loop decide 8.3 ms (now 6.8), the CABAC decide of IDR + 3 P 7 ms more than with this, that of 16 pictures at once 2.5.
 template <class T>
 __device__ __forceinline__ uint32_t code_blocks4(const CodeParams& P, CodeSmem& S, int mbx, int mby, ironav_intercode* out) {
     const int lane = threadIdx.x & 31;
