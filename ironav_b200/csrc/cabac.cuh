@@ -84,16 +84,22 @@ struct WordOut {
     }
 };
 
-// A bin as the coder takes it: of a decision, the LPS range of its state for each quarter of the range (a byte each), that range
-// renormalised (its low byte; the ninth bit is set) and by how many bits; and what kind of bin it is.
-enum CodeKind : uint32_t { CODE_MPS = 0, CODE_LPS = 1, CODE_BYPASS = 2, CODE_TERMINATE = 4 };  // the last two + the bin
+// A bin as the coder takes it, every kind in one form: the range it takes off for each quarter of the range (a byte each: the LPS
+// range of its state, 2 of a terminate bin, 0 of a bypass bin); what the range becomes when it is the low part (its low byte; the
+// ninth bit is set) and by how many bits that shifts the code; and ctl.
+enum CodeCtl : uint32_t {
+    CODE_PRE = 1u,          // a bypass bin: the code shifts by one before the addition
+    CODE_END = 2u,          // the slice's last bin
+    CODE_LOW = 1u << 30,    // an LPS, or a terminate bin of 1: the range becomes the low part's
+    CODE_ADD = 1u << 31     // the code goes up by the rest of the range
+};
 struct __align__(16) CodeBin {
-    uint32_t lps, norm, shift, kind;
+    uint32_t lps, norm, shift, ctl;
 };
 static_assert(sizeof(CodeBin) == 16, "one 16-byte read");
 // The entry of probability state p.
 __device__ __forceinline__ CodeBin code_entry(int p) {
-    CodeBin e = {0, 0, 0, CODE_MPS};
+    CodeBin e = {0, 0, 0, 0};
     for (int q = 0; q < 4; q++) {
         const uint32_t r = LPS_RANGE[p][q], sh = (uint32_t)__clz((int)r) - 23u;
         e.lps |= r << (8 * q);
@@ -102,51 +108,37 @@ __device__ __forceinline__ CodeBin code_entry(int p) {
     }
     return e;
 }
+__device__ __forceinline__ CodeBin code_bypass(uint32_t bin) { return {0u, 0u, 0u, CODE_PRE | (bin ? CODE_ADD : 0u)}; }
+__device__ __forceinline__ CodeBin code_terminate(uint32_t bin) {
+    return {0x02020202u, 0u, 0x07070707u, bin ? CODE_LOW | CODE_ADD | CODE_END : 0u};
+}
 
 // The arithmetic coder (9.3.4.2-9.3.4.5). Its serial chain is the range alone: a bin's probability state is looked up before it, and
 // the code value is a plain sum, kept whole: `low` holds the 10 bits of the standard's codILow below the nb bits already shifted
-// out of it, and a carry above them. nb begins at -1: the first bit of the code is not written (9.3.4.2).
+// out of it, and a carry above them. nb begins at -1: the first bit of the code is not written (9.3.4.2). Every bin takes the same
+// instructions, without a branch on its kind (the range's top bits pick the byte of its quarter: range >> 6 is 4 + the quarter, a
+// byte permutation's selector): a branch a kind, on the writer's one coding lane, took some 240 cycles a bin.
 struct Coder {
     WordOut out;
     uint64_t low;
     uint32_t range;
     int nb;
-    __device__ __forceinline__ void shift(uint32_t sh) {
-        low <<= sh;
-        nb += (int)sh;
+    // at most two bins (7 bits each) before settle(), from nb < 32: the code stays within 56 bits
+    __device__ __forceinline__ void code(const CodeBin& e) {
+        const uint32_t q = range >> 6, rest = range - __byte_perm(0u, e.lps, q), ms = rest < 256u, pre = e.ctl & CODE_PRE;
+        const bool part = (e.ctl & CODE_LOW) != 0;
+        const uint32_t sh = part ? __byte_perm(0u, e.shift, q) : ms;
+        low = ((low << pre) + (rest & (uint32_t)((int)e.ctl >> 31))) << sh;
+        nb += (int)(pre + sh);
+        range = part ? 256u | __byte_perm(0u, e.norm, q) : rest << ms;
+    }
+    __device__ __forceinline__ void settle() {
         if (nb >= 32) {
             const int rest = nb - 22;  // 10 + nb - 32
             out.put(low >> rest);
             low &= (1ull << rest) - 1;
             nb -= 32;
         }
-    }
-    __device__ __forceinline__ void code(const CodeBin& e) {
-        uint32_t sh;
-        if (e.kind <= CODE_LPS) {
-            const uint32_t q = (range >> 3) & 0x18u, mps = range - ((e.lps >> q) & 0xFFu);
-            const bool lps = e.kind == CODE_LPS;
-            low += lps ? mps : 0u;
-            const uint32_t ms = mps < 256u;
-            sh = lps ? (e.shift >> q) & 0xFFu : ms;
-            range = lps ? 256u | ((e.norm >> q) & 0xFFu) : mps << ms;
-        } else if (e.kind < CODE_TERMINATE) {
-            // the bin's share of the range, after the shift: low = 2 low + bin * range
-            low = (low << 1) + ((e.kind & 1u) ? range : 0u);
-            nb += 1;
-            sh = 0;
-        } else {
-            range -= 2;
-            if (e.kind & 1u) {
-                low += range;
-                range = 2;
-                sh = 7;
-            } else {
-                sh = range < 256u;
-            }
-            range <<= sh;
-        }
-        shift(sh);
     }
     // after the last terminate bin: the flush's bit and two more, the last of them the rbsp_stop_one_bit
     __device__ __forceinline__ uint32_t finish() {

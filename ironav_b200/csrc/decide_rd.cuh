@@ -1138,7 +1138,8 @@ static __global__ void __launch_bounds__(128) cabac_nb_kernel(const __grid_const
 //   - warp 1 takes the lists in order and looks up each bin's probability state (32 bins a turn; the bins of a context are a
 //     chain, the contexts side by side), leaving what the coder needs of it in a ring;
 //   - lane 0 of warp 0 runs the coder's own chain, the range, over the ring.
-// One lane doing all three took 62 ms for an IDR and three P pictures at 1080p, the pipeline 27 ms. Every wait is on shared memory and
+// One lane doing all three took 62 ms for an IDR and three P pictures at 1080p, the pipeline 27 ms with a branch on each bin's kind in
+// the coder, now 14 (7 with the coder's arithmetic left out). Every wait is on shared memory and
 // bounded; a warp that gives up stops the others, and the picture is reported like one that outgrew its region.
 constexpr int WR_LISTERS = 6;
 constexpr int WR_THREADS = (2 + WR_LISTERS) * 32;
@@ -1202,18 +1203,26 @@ static __global__ void __launch_bounds__(WR_THREADS) cabac_write_kernel(const __
                     if (!wr_wait(S, &S.head, at + 1)) break;
                     avail = ld_acquire_cta(&S.head);
                 }
-                // up to eight bins from here, read before the chain begins; slots beyond `avail` are read and not used
-                cab::CodeBin e[8];
-                const unsigned nb = min(avail - at, 8u);
+                if (avail - at >= 8u) {
+                    // eight bins, read before the chain goes through them; the slice's last bin is the last of what there is
+                    cab::CodeBin e[8];
 #pragma unroll
-                for (int i = 0; i < 8; i++) e[i] = S.ring[(at + i) % WR_RING];
+                    for (int i = 0; i < 8; i++) e[i] = S.ring[(at + i) % WR_RING];
 #pragma unroll
-                for (int i = 0; i < 8; i++)
-                    if (i < (int)nb) {
+                    for (int i = 0; i < 8; i += 2) {
                         k.code(e[i]);
-                        more = e[i].kind != (cab::CODE_TERMINATE | 1u);
+                        k.code(e[i + 1]);
+                        k.settle();
                     }
-                at += nb;
+                    more = (e[7].ctl & cab::CODE_END) == 0;
+                    at += 8;
+                } else {
+                    const cab::CodeBin e = S.ring[at % WR_RING];
+                    k.code(e);
+                    k.settle();
+                    more = (e.ctl & cab::CODE_END) == 0;
+                    at++;
+                }
                 if (at % (WR_RING / 4) < 8u) st_release_cta(&S.tail, at);  // room for the states' warp well before the ring runs dry
             }
             const uint32_t bytes = k.finish();
@@ -1255,11 +1264,11 @@ static __global__ void __launch_bounds__(WR_THREADS) cabac_write_kernel(const __
                     __syncwarp();
                     if (in) {
                         const uint32_t bin = (e >> 10) & 1u;
-                        cab::CodeBin c = {0u, 0u, 0u, ((e & cab::BIN_TERMINATE) ? cab::CODE_TERMINATE : cab::CODE_BYPASS) | bin};
+                        cab::CodeBin c = (e & cab::BIN_TERMINATE) ? cab::code_terminate(bin) : cab::code_bypass(bin);
                         if (dec) {
                             const uint32_t s = S.pre[lane];
                             c = S.entry[s >> 1];
-                            c.kind = (s & 1u) != bin ? cab::CODE_LPS : cab::CODE_MPS;
+                            c.ctl = (s & 1u) != bin ? cab::CODE_LOW | cab::CODE_ADD : 0u;
                         }
                         S.ring[(head + lane) % WR_RING] = c;
                     }
