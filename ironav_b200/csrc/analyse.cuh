@@ -762,8 +762,10 @@ static __device__ __noinline__ int2 sub_search(const AnalyseParams& __restrict__
     return make_int2(best_s, best_cost);
 }
 
-// best_inter_ref, enc/frame.rs:852-905. Leaves the winner's vectors in S.best_mvs.
-template <class T>
+// best_inter_ref, enc/frame.rs:852-905. Leaves the winner's vectors in S.best_mvs. WINDOW: the planes lie on 16-byte boundaries, so
+// that the window's 16-byte copies may be made (a context's own planes do); otherwise none is staged, and every candidate is
+// read from the plane.
+template <class T, bool WINDOW = true>
 static __device__ __noinline__ int4 best_inter_ref(const AnalyseParams& __restrict__ P, WarpSmem<T>& __restrict__ S, int r) {
     const int lane = threadIdx.x & 31;
     const int lam = P.lambda;
@@ -772,7 +774,14 @@ static __device__ __noinline__ int4 best_inter_ref(const AnalyseParams& __restri
     else if (P.nact > 2) rb = lam * (2 * (31 - __clz(r + 1)) + 1);
     const int2 mvp = pred_mv(P, S, S.ext, nullptr, 0, 0, 4, 0, r);
     const ColMv col = P.col[S.mb];
-    if constexpr (Win<T>::ON) {
+    if constexpr (Win<T>::ON && !WINDOW) {
+        // a place that no candidate's rows and columns fall into
+        if (lane == 0) {
+            S.win_x = 1 << 20;
+            S.win_y = 0;
+        }
+        __syncwarp();
+    } else if constexpr (Win<T>::ON) {
         // around the search's first candidate
         const int x0 = S.mbx * 16, y0 = S.mby * 16;
         const int cx = min(max(mvp.x, max(-(x0 + 24) * 4, -2048)), min((P.mb_w * 16 - x0 + 8) * 4, 2047));
@@ -983,13 +992,13 @@ static __device__ __noinline__ int4 learned_inter(const AnalyseParams& __restric
 }
 
 // best_inter_ref, or the learned form's judge on the newest reference when proposals are given.
-template <class T>
+template <class T, bool WINDOW = true>
 static __device__ __forceinline__ int4 best_inter_or_learned(const AnalyseParams& __restrict__ P, WarpSmem<T>& __restrict__ S, int r) {
     if (P.learned != nullptr && r == 0) {
         const int4 li = learned_inter(P, S, r);
         if (li.x >= 0) return li;
     }
-    return best_inter_ref(P, S, r);
+    return best_inter_ref<T, WINDOW>(P, S, r);
 }
 
 // ---- one macroblock --------------------------------------------------------------------------------
@@ -1009,7 +1018,7 @@ static __device__ __forceinline__ void stage_source(const AnalyseParams& __restr
     }
 }
 
-template <class T>
+template <class T, bool WINDOW = true>
 static __device__ void analyse(const AnalyseParams& __restrict__ P, WarpSmem<T>& __restrict__ S, bool auto_policy) {
     const int lane = threadIdx.x & 31;
     stage_source(P, S);
@@ -1030,7 +1039,7 @@ static __device__ void analyse(const AnalyseParams& __restrict__ P, WarpSmem<T>&
     if (!skip) {
         // best_inter, enc/frame.rs:839-849: every reference, the cheapest (first on ties) wins
         for (int r = 0; r < P.nact; r++) {
-            const int4 bi = best_inter_or_learned(P, S, r);
+            const int4 bi = best_inter_or_learned<T, WINDOW>(P, S, r);
             const int c = bi.x, p = bi.y, c16 = bi.w;
             const uint32_t sb = (uint32_t)bi.z;
             if (r == 0 || c < cost) {

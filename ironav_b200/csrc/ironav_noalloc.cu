@@ -92,7 +92,8 @@ __global__ void noalloc_init_kernel(uint32_t* scr, const ironav_mbstate* col, in
 
 // The wavefront analysis with tickets in row-interleaved order: ticket T covers row slot R = T / mb_w
 // (the R / nslices-th row of band R % nslices) and column T % mb_w. A macroblock's left and top-right
-// neighbours always hold smaller tickets, so a waiting warp only waits on running warps.
+// neighbours always hold smaller tickets, so a waiting warp only waits on running warps. WINDOW: as best_inter_ref's.
+template <bool WINDOW>
 __global__ void __launch_bounds__(K2_WARPS * 32, K2_MIN_BLOCKS) analyse_noalloc_kernel(const __grid_constant__ AnalyseParams P, int nslices,
                                                                        int max_rows) {
     __shared__ WarpSmem<uint8_t> smem[K2_WARPS];
@@ -121,7 +122,7 @@ __global__ void __launch_bounds__(K2_WARPS * 32, K2_MIN_BLOCKS) analyse_noalloc_
         ok = __all_sync(FULL, ok);
         if (!ok) break;
         load_neighbours(P, S, P.states_out);
-        analyse(P, S, true);
+        analyse<uint8_t, WINDOW>(P, S, true);
         __threadfence();
         __syncwarp();
         if (lane == 0 && mb != P.withhold) st_release(&P.flags[mb], P.epoch);
@@ -138,7 +139,7 @@ cudaError_t device_setup(int dev, DeviceSetup& S) {
     int nsm = 0, per_sm = 0;
     e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_noalloc_kernel, K2_WARPS * 32, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, analyse_noalloc_kernel<true>, K2_WARPS * 32, 0);
     if (e != cudaSuccess) return e;
     S.scratch = static_cast<uint32_t*>(p);
     S.blocks = (per_sm > 0 ? per_sm : 1) * nsm;
@@ -219,7 +220,10 @@ extern "C" int ironav_analyse_auto_noalloc(const uint8_t* d_src, int src_stride,
     p.withhold = g_withhold.load();
     p.wait_limit = g_wait_limit.load();
     const int max_rows = (mb_h + nslices - 1) / nslices;
-    analyse_noalloc_kernel<<<S.blocks, K2_WARPS * 32, 0, s>>>(p, nslices, max_rows);
+    // the search's window is copied 16 bytes at a time; planes on a 4- or 8-byte boundary are searched in place
+    // (854x480, three slices: 1414 us a call with the window, 1513 without)
+    if (reinterpret_cast<uintptr_t>(d_planes) & 15) analyse_noalloc_kernel<false><<<S.blocks, K2_WARPS * 32, 0, s>>>(p, nslices, max_rows);
+    else analyse_noalloc_kernel<true><<<S.blocks, K2_WARPS * 32, 0, s>>>(p, nslices, max_rows);
     e = cudaGetLastError();
     if (e != cudaSuccess) return map_status(e);
     uint32_t err = 0;

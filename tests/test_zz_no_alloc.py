@@ -135,3 +135,25 @@ def test_noalloc_rejects_pictures_beyond_its_scratch(cuda_lib):
         d.data_ptr(), 8192, d.data_ptr(), 8192, 8192, 4608, None, 8192, 4608, 1, 27, 6, 100, 0, 0,
         d.data_ptr(), d.data_ptr(), d.data_ptr(), None)
     assert status == 3
+
+
+@pytest.mark.parametrize("shift", [4, 8, 12])
+def test_noalloc_planes_off_a_16_byte_boundary(cuda_lib, oracle_lib, shift):
+    """d_planes on any 4-byte boundary, as the header allows: the search then stages no window (its copies are 16 bytes
+    each), and the planes, decisions and results are the oracle's all the same."""
+    import torch
+
+    seq = Sequence.config("1080p", 3, size=(W, H))
+    frames = [seq.frame(t) for t in range(3)]
+    (_, (planes, states, res)), (_, _, sw, sh, nmb) = _context_outputs(oracle_lib, frames)
+    first = _context_outputs(oracle_lib, frames)[0][0][1]
+    buf = torch.zeros(4 * sw * sh + 16, dtype=torch.uint8, device="cuda")
+    assert buf.data_ptr() % 16 == 0
+    d_planes = buf[shift:shift + 4 * sw * sh]
+    d_col = torch.from_numpy(first.view(np.uint8).reshape(-1).copy()).cuda()
+    d_states = torch.zeros(nmb * 72, dtype=torch.uint8, device="cuda")
+    d_results = torch.zeros(nmb * 104, dtype=torch.uint8, device="cuda")
+    assert _noalloc(cuda_lib, frames, 2, d_col.data_ptr(), d_planes, d_states, d_results) == 0
+    assert np.array_equal(d_planes.cpu().numpy().reshape(4, sh, sw), planes)
+    assert np.array_equal(d_states.cpu().numpy().view(MBSTATE_DTYPE), states)
+    assert np.array_equal(d_results.cpu().numpy().view(MBRESULT_DTYPE), res)
