@@ -70,18 +70,19 @@ __device__ __forceinline__ int row_sad(const uint8_t* G, const uint32_t* sr, int
     const unsigned sh = (unsigned)(a & 3) * 8u;
     const int nw = (w * B) >> 2;
     int sad = 0;
-    uint32_t ad = 0, pv = __ldg(q);
+    Sum2 ad;
+    uint32_t pv = __ldg(q);
 #pragma unroll
     for (int k = 0; k < 4 * B; k++) {
         if (k < nw) {
             const uint32_t nx = __ldg(q + k + 1);
             const uint32_t v = __funnelshift_r(pv, nx, sh);
             if constexpr (B == 1) sad = vsad4(sr[k], v, sad);
-            else ad = vad2(sr[k], v, ad);
+            else vad2(sr[k], v, ad);
             pv = nx;
         }
     }
-    return B == 1 ? sad : sum2(ad);
+    return B == 1 ? sad : ad.total();
 }
 
 // Integer SAD (sad_int, enc/frame.rs:662-671) of the w x h partition for two vectors at once: the first half
@@ -117,15 +118,15 @@ __device__ __forceinline__ int score4_src(const uint32_t* __restrict__ src, int 
         for (int k = 0; k < B; k++) sr[row][k] = sp[row * 4 * B + k];
     int v = 0;
     if (sad) {
-        uint32_t ad = 0;
+        Sum2 ad;
 #pragma unroll
         for (int row = 0; row < 4; row++)
 #pragma unroll
             for (int k = 0; k < B; k++) {
                 if constexpr (B == 1) v = vsad4(sr[row][k], pr[row][k], v);
-                else ad = vad2(sr[row][k], pr[row][k], ad);
+                else vad2(sr[row][k], pr[row][k], ad);
             }
-        if constexpr (B == 2) v = sum2(ad);
+        if constexpr (B == 2) v = ad.total();
     } else if constexpr (B == 1) {
         const uint32_t s1[4] = {sr[0][0], sr[1][0], sr[2][0], sr[3][0]}, p1[4] = {pr[0][0], pr[1][0], pr[2][0], pr[3][0]};
         v = satd4_packed(s1, p1);

@@ -15,6 +15,8 @@
 // SATD over 36 lane-units of (mode, 4x4 quadrant) from a table of the predictors (i8_entry), the chosen
 // block's 8x8 transform on eight lanes.
 #pragma once
+#include <type_traits>
+
 #include "cabac.cuh"
 #include "decide.cuh"
 
@@ -339,21 +341,32 @@ __device__ __forceinline__ void code_init(ironav_mbcode* o) {
 // only, the chroma added later from another candidate's. The candidate counts from here on.
 template <class T, int W>
 __device__ void rd_take(const CodeParams& C, RdSmem<T, W>& R, const DecideSmem<T>& S, int k, int mbx, int mby, bool chroma = true) {
-    // a lane's half row of luma and four chroma samples, as words; a sum of 384 squared differences of 10 bits fits 32 bits
+    // a lane's half row of luma and four chroma samples, as words. The sums are 32 bits wide at 8 bits (384 squares of 255 fit), 64 at
+    // 10, whose 16-bit samples are taken as they are given.
     const int lane = threadIdx.x & 31;
     constexpr int B = (int)sizeof(T);
+    using Sum = std::conditional_t<B == 1, uint32_t, unsigned long long>;
     uint32_t* const dst = reinterpret_cast<uint32_t*>(R.crec[k]);
     __syncwarp();
-    auto squares = [](uint32_t a, uint32_t b, uint32_t acc) {
+    auto squares = [](uint32_t a, uint32_t b, Sum acc) {
         if constexpr (B == 1) {
             const uint32_t d = __vabsdiffu4(a, b);
             return __dp4a(d, d, acc);
         } else {
-            const int lo = (int)(a & 0xffffu) - (int)(b & 0xffffu), hi = (int)(a >> 16) - (int)(b >> 16);
-            return acc + (uint32_t)(lo * lo) + (uint32_t)(hi * hi);
+            const uint32_t lo = (uint32_t)abs((int)(a & 0xffffu) - (int)(b & 0xffffu)), hi = (uint32_t)abs((int)(a >> 16) - (int)(b >> 16));
+            return acc + (Sum)lo * lo + (Sum)hi * hi;
         }
     };
-    uint32_t ssd = 0, cssd = 0;
+    auto warp_sum = [](Sum v) {
+        if constexpr (B == 1) {
+            return __reduce_add_sync(FULL, v);
+        } else {
+#pragma unroll
+            for (int off = 16; off >= 1; off >>= 1) v += __shfl_xor_sync(FULL, v, off);
+            return v;
+        }
+    };
+    Sum ssd = 0, cssd = 0;
     {
         const int row = lane >> 1, half = lane & 1;
         const uint32_t* rec = reinterpret_cast<const uint32_t*>(reinterpret_cast<const T*>(C.rec[0]) + (size_t)(mby * 16 + row) * C.ys + mbx * 16 + half * 8);
@@ -380,13 +393,13 @@ __device__ void rd_take(const CodeParams& C, RdSmem<T, W>& R, const DecideSmem<T
                 dst[64 * B + lane * B + i] = cv[i];
                 cssd = squares(cv[i], cs[i], cssd);
             }
-            cssd = __reduce_add_sync(FULL, cssd);
+            cssd = warp_sum(cssd);
         }
-        ssd = __reduce_add_sync(FULL, ssd);
+        ssd = warp_sum(ssd);
     }
     if (lane == 0) {
         R.ssd[k] = (long long)(ssd + cssd);
-        R.cssd[k] = cssd;
+        R.cssd[k] = (long long)cssd;
         R.valid[k] = 1;
     }
     __syncwarp();
