@@ -1420,7 +1420,7 @@ def run_decide_batched(args, rank, world):
                 "d2h_bytes_per_step": sum(sum(int(t.numel()) for t in b) for b in bufs), "ms_per_step": 1e3 * el / args.steps,
                 "note": "each stream's source luma from pinned host memory (its chroma stays resident) + the launch + states, "
                         "codes and reconstructions back to pinned host memory"},
-        "roofline": {"bound": "latency", "kernel": "decide_rd_batch_kernel" if args.cabac else "decide_batch_kernel", "achieved": None,
+        "roofline": {"bound": "latency", "kernel": "decide_rdw_batch_kernel" if args.cabac else "decide_batch_kernel", "achieved": None,
                      "peak": None, "unit": None, "frac": None,
                      "traffic": None, "ms_per_launch": float(np.median(per)),
                      "note": "many wavefronts interleaved; the per-stream loop above is the same work one stream at a time"},
@@ -1595,10 +1595,10 @@ def run_decide(args, rank, world):
         "e2e": {"value": world * nmb * args.steps / el, "unit": "MB/s", "h2d_bytes_per_step": 0,
                 "d2h_bytes_per_step": nmb * (72 + MBCODE_DTYPE.itemsize + 384 * B), "ms_per_step": 1e3 * el / args.steps,
                 "note": "ironav_decide_p_picture with host buffers (sources and references already held by the contexts)"},
-        "roofline": {"bound": "latency", "kernel": f"{'decide_rd_kernel' if args.cabac else 'decide_kernel'}<{'uint8_t' if bd == 8 else 'uint16_t'}>",
+        "roofline": {"bound": "latency", "kernel": f"{'decide_rdw_kernel' if args.cabac else 'decide_kernel'}<{'uint8_t' if bd == 8 else 'uint16_t'}>",
                      "achieved": None, "peak": None, "unit": None, "frac": None, "traffic": None, "ms_per_launch": k_ms,
                      "note": (f"one chain a slice band: {nmb // NSLICES} dependent macroblocks (each macroblock's CABAC cost reads "
-                              "the contexts every earlier one in its slice left), a warp each"
+                              "the contexts every earlier one in its slice left), five warps each"
                               if args.cabac else
                               f"one stream's wavefront: a critical path of mb_w + 2 (band rows - 1) = {mb_w + 2 * (-(-mb_h // NSLICES) - 1)} "
                               "dependent macroblocks; see the per-macroblock latency in the profile")},

@@ -505,7 +505,7 @@ int ironav_batch_sync(ironav_batch* batch);
  * chroma, references with chroma, picture parameters); arrays of n device pointers and strides, stream
  * i's outputs as that call's. Under CABAC (every context of the batch with the same ironav_set_entropy
  * setting, else IRONAV_INVALID_ARGUMENT) every stream's slice bands are chains of the rate-distortion
- * decision, the longest on three warps each and the rest on one, in two launches side by side.
+ * decision in one launch, the longest first, an SM each or, when there are more of them than SMs, two an SM.
  * Asynchronous; ironav_batch_sync waits. */
 int ironav_batch_decide(ironav_batch* batch, ironav_mbstate* const* d_states, ironav_mbcode* const* d_codes, void* const* d_rec_y,
                         const int* y_strides, void* const* d_rec_cb, void* const* d_rec_cr, const int* c_strides);

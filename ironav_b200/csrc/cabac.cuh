@@ -33,20 +33,6 @@ __device__ __forceinline__ void init_states(uint8_t* st, bool intra, int idc, in
     }
 }
 
-// The bit counter over its own copy of the contexts.
-struct Counter {
-    uint8_t* st;
-    const uint32_t* step;
-    uint32_t bits;
-    __device__ __forceinline__ void decision(int ctx, int bin) {
-        const uint32_t e = step[st[ctx] * 2 + (bin != 0)];
-        st[ctx] = (uint8_t)e;
-        bits += e >> 8;
-    }
-    __device__ __forceinline__ void bypass(int) { bits += 256; }
-    __device__ __forceinline__ void terminate(int bin) { bits += bin ? 7 * 256 : 1; }
-};
-
 // The arithmetic coder's output: 32-bit pieces of the code value, MSB first, into the words of a region in global memory,
 // stored so that the bytes read in order. A piece may carry into the ones before it, so the newest is held back, with a count of
 // the 0xFFFFFFFF pieces after it that a carry would run through. A write beyond the region sets `over` and is dropped.

@@ -3,8 +3,8 @@
 // slice writer.
 //
 // Under CABAC a macroblock's rate-distortion cost counts its bins against the slice's contexts as the
-// macroblocks before it left them, so a slice band is one chain in raster order: a CTA walks a band, one warp or (the wide form)
-// five. For each macroblock every candidate the reference tries is coded (P_Skip, best_inter's partitioning with the 4x4 and, with
+// macroblocks before it left them, so a slice band is one chain in raster order: a CTA of five warps walks a band. For each
+// macroblock every candidate the reference tries is coded (P_Skip, best_inter's partitioning with the 4x4 and, with
 // transform8, the 8x8 transform, Intra16x16, Intra4x4, Intra8x8, each intra one with its chroma), into the picture or a scratch
 // plane and then into shared memory (code and reconstruction), with its squared error, and its bins are priced on its own copy
 // of the contexts (cab::price); the least SSD + lambda2 * bits in the reference's order (strict '<') is kept, and its code,
@@ -32,7 +32,7 @@ struct RdParams {
     double lam2;            // 1.6 * 2^((QP'Y - 12) / 3), computed on the host in f64 as the reference does
     int nbands;
     int t8;                 // transform_8x8_mode_flag
-    // the wide form: the scratch planes of warps 1 to 4 (luma, Cb, Cr of each), pw x ph and cw x ch samples, rows scr_ys
+    // the scratch planes of warps 1 to 4 (luma, Cb, Cr of each), pw x ph and cw x ch samples, rows scr_ys
     // and scr_cs samples apart
     uint8_t* scr[12];
     int scr_ys, scr_cs;
@@ -54,8 +54,7 @@ struct RdSmem {
     long long cssd[RD_CANDS];        // the chroma part of ssd
     unsigned bits[RD_CANDS];
     int valid[RD_CANDS];
-    int best;
-    // the wide form: of the macroblocks a group tests for P_Skip, the verdict, the skip vector and the top neighbour; the intra
+    // of the macroblocks a group tests for P_Skip, the verdict, the skip vector and the top neighbour; the intra
     // chroma's coded block pattern bits; best_inter's decision for the 8x8-transform candidate, and whether that is tried
     int skip[W];
     int2 sv[W];
@@ -134,7 +133,7 @@ template <class T, int W>
 __device__ uint32_t code_i8_d(const DecideParams& P, DecideSmem<T>& S, RdSmem<T, W>& R, int mbx, int mby, bool ta, bool la, bool tra,
                               ironav_mbcode* out, T* wy, int wys) {
     // P.C.rec: the picture the edges are read from; wy (rows wys samples apart): where the luma goes. The
-    // predictor table of R.i8tab is filled once a chain (rd_chain)
+    // predictor table of R.i8tab is filled once a chain (rdw_chain)
     const int lane = threadIdx.x & 31;
     const CodeParams& C = P.C;
     const int bd = C.bd, maxv = (1 << bd) - 1, lam = C.A.lambda;
@@ -427,7 +426,7 @@ __device__ __forceinline__ void rd_price(RdSmem<T, W>& R, const cab::Slice& sl, 
     __syncwarp();
 }
 
-// Intra candidate k's chroma: Intra16x16's code, reconstruction and squared error (the wide form; k's luma is coded).
+// Intra candidate k's chroma: Intra16x16's code, reconstruction and squared error (k's luma is coded).
 template <class T, int W>
 __device__ __forceinline__ void rd_take_chroma(RdSmem<T, W>& R, int k) {
     const int lane = threadIdx.x & 31;
@@ -474,263 +473,7 @@ __device__ __forceinline__ void rd_state(RdSmem<T, W>& R, const DecideSmem<T>& S
     __syncwarp();
 }
 
-// decide_rd for one macroblock (after code_mb's P_Skip tests, best_i16 and best_inter; enc/frame.rs:715-760,
-// 1462-1513), its bins then carried into the chain's contexts (write_mb_cabac's effect on them, 2020-2025).
-template <class T>
-__device__ void rd_mb(const RdParams& P, RdSmem<T, 1>& R, const unsigned* i4tab, int mb, int mbx, int mby) {
-    const int lane = threadIdx.x & 31;
-    const DecideParams& D = P.D;
-    const AnalyseParams& A = D.C.A;
-    const CodeParams& C = D.C;
-    DecideSmem<T>& S = R.s[0];
-    const bool ta = mby > A.band_start[mby], la = mbx > 0, tra = ta && mbx + 1 < A.mb_w;
-    const cab::Slice sl = {D.intra ? 0 : 1, P.t8, D.intra ? 0 : A.nact};
-    ironav_mbcode* out = &D.codes[mb];
-    ironav_mbcode* cand = R.cand;
-    code_init(out);
-    stage_source(A, S.a);
-    // the neighbours for the contexts: the left one is the macroblock just decided, the top one's was kept
-    if (lane < cab::NB_WORDS) {
-        uint32_t* l = reinterpret_cast<uint32_t*>(&R.nb[0]);
-        uint32_t* t = reinterpret_cast<uint32_t*>(&R.nb[1]);
-        l[lane] = la ? reinterpret_cast<const uint32_t*>(&R.done)[lane] : 0u;
-        t[lane] = ta ? P.nbs[(size_t)(mb - A.mb_w) * cab::NB_WORDS + lane] : 0u;
-    }
-    if (lane < RD_CANDS) R.valid[lane] = 0;
-    __syncwarp();
-    int2 sv = make_int2(0, 0);
-    if (!D.intra && skip_tests_d<T>(D, S, mb, mbx, mby, out, &sv)) {
-        // P_Skip without a rate-distortion choice; its one bin still moves the contexts
-        if (lane == 0) {
-            cab::Counter c = {R.live, R.step, 0};
-            cab::skip_bin(c, out, R.nb[0], R.nb[1]);
-        }
-        if (lane < 18) reinterpret_cast<uint32_t*>(&A.states_out[mb])[lane] = reinterpret_cast<const uint32_t*>(&S.a.out)[lane];
-        __syncwarp();
-        cab::nb_of_warp(out, &R.done);
-        if (lane < cab::NB_WORDS) P.nbs[(size_t)mb * cab::NB_WORDS + lane] = reinterpret_cast<const uint32_t*>(&R.done)[lane];
-        __syncwarp();
-        return;
-    }
-    load_intra_neighbours(D, S, mb, mbx, mby, ta, la, tra);
-    const int2 i16 = best_i16_d(D, S, ta, la);
-    // best_inter, enc/frame.rs:839-849 (none in an IDR picture)
-    int part = 0, cost = BIG, bestr = 0;
-    uint32_t sub = 0;
-    for (int r = 0; r < A.nact && !D.intra; r++) {
-        const int4 bi = best_inter_or_learned(A, S.a, r);
-        if (r == 0 || bi.x < cost) {
-            part = bi.y;
-            cost = bi.x;
-            bestr = r;
-            sub = (uint32_t)bi.z;
-            if (lane < 16) {
-                S.a.win_mvs[lane][0] = S.a.best_mvs[lane][0];
-                S.a.win_mvs[lane][1] = S.a.best_mvs[lane][1];
-            }
-            __syncwarp();
-        }
-    }
-    ironav_interdec& Dd = *reinterpret_cast<ironav_interdec*>(S.c.dec);
-    if (!D.intra) {
-        // P_Skip: the skip vector's prediction is the reconstruction (put_inter_pred, 1391-1394)
-        ironav_mbcode* o = &cand[0];
-        code_init(o);
-        if (lane == 0) {
-            Dd.mode = 1;
-            Dd.part = 0;
-            Dd.t8 = 0;
-            for (int k = 0; k < 4; k++) Dd.sub[k] = Dd.refs[k] = 0;
-        }
-        if (lane < 16) {
-            Dd.mvs[lane][0] = (int16_t)sv.x;
-            Dd.mvs[lane][1] = (int16_t)sv.y;
-        }
-        __syncwarp();
-        code_inter_mb<T>(C, S.c, mb, &o->res);
-        inter_tail(D, S, Dd, o);
-        if (lane < 16) o->mvds[lane][0] = o->mvds[lane][1] = 0;
-        if (lane == 0) o->skip = 1;
-        rd_state(R, S, 0, true);
-        rd_take(C, R, S, 0, mbx, mby);
-        // best_inter's partitioning with the 4x4 transform; with nothing coded and the skip vector, it would be
-        // P_Skip at a higher price
-        o = &cand[1];
-        code_init(o);
-        if (lane == 0) {
-            Dd.mode = 2;
-            Dd.part = (uint8_t)part;
-            Dd.t8 = 0;
-            for (int k = 0; k < 4; k++) {
-                Dd.sub[k] = (uint8_t)((sub >> (8 * k)) & 0xff);
-                Dd.refs[k] = (uint8_t)bestr;
-            }
-        }
-        if (lane < 16) {
-            Dd.mvs[lane][0] = S.a.win_mvs[lane][0];
-            Dd.mvs[lane][1] = S.a.win_mvs[lane][1];
-        }
-        __syncwarp();
-        const uint32_t cbp = code_inter_mb<T>(C, S.c, mb, &o->res);
-        inter_tail(D, S, Dd, o);
-        rd_state(R, S, 1, true);
-        rd_take(C, R, S, 1, mbx, mby);
-        if (lane == 0 && cbp == 0 && part == 0 && Dd.mvs[0][0] == sv.x && Dd.mvs[0][1] == sv.y && bestr == 0) R.valid[1] = 0;
-        __syncwarp();
-        // the 8x8 transform needs every 8x8 block of P_8x8 to be a single 8x8 partition; without luma levels it
-        // would be the 4x4 candidate again
-        if (P.t8 && sub == 0) {
-            o = &cand[2];
-            code_init(o);
-            if (lane == 0) Dd.t8 = 1;
-            __syncwarp();
-            code_inter_mb<T>(C, S.c, mb, &o->res);
-            inter_tail(D, S, Dd, o);
-            rd_state(R, S, 2, true);
-            rd_take(C, R, S, 2, mbx, mby);
-            if (lane == 0 && !o->res.t8x8) R.valid[2] = 0;
-            __syncwarp();
-        }
-    }
-    // Intra16x16 in best_i16's mode, with its chroma. code_intra_chroma reads only the chroma around the
-    // macroblock and writes only its chroma, so the Intra4x4 and Intra8x8 candidates take this one's
-    // (its mode, levels, counts and pattern; the reconstruction stays in the picture)
-    uint32_t ccbp = 0;
-    {
-        ironav_mbcode* o = &cand[3];
-        code_init(o);
-        uint32_t cbp = code_i16_d(D, S, mbx, mby, i16.x, ta, la, o);
-        ccbp = code_intra_chroma_d(D, S, mbx, mby, ta, la, o);
-        cbp |= ccbp;
-        if (lane == 0) {
-            o->kind = KIND_I16;
-            o->i16_mode = (uint8_t)i16.x;
-            o->res.cbp = (uint8_t)cbp;
-        }
-        rd_state(R, S, 3, false);
-        rd_take(C, R, S, 3, mbx, mby);
-    }
-    // Intra4x4, block by block from its own reconstruction, with its chroma
-    {
-        ironav_mbcode* o = &cand[4];
-        code_init(o);
-        code_i4_trial(D, S, i4tab, ta, la, tra);
-        T* RY = reinterpret_cast<T*>(C.rec[0]);
-        for (int i = lane; i < 256; i += 32) RY[(size_t)(mby * 16 + (i >> 4)) * C.ys + mbx * 16 + (i & 15)] = (T)S.i4rec[i];
-        if (lane < 16) {
-            uint32_t* lw = reinterpret_cast<uint32_t*>(o->res.luma[lane]);
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(S.i4lv[lane]);
-#pragma unroll
-            for (int k = 0; k < 8; k++) lw[k] = src[k];
-            o->res.nnz[lane] = S.i4nnz[lane];
-            o->modes[lane] = S.i4modes[lane];
-        }
-        const unsigned bal = __ballot_sync(FULL, lane < 16 && S.i4nnz[lane] > 0);
-        uint32_t cbp = 0;
-#pragma unroll
-        for (int i8 = 0; i8 < 4; i8++)
-            if (bal & (0x33u << ((i8 >> 1) * 8 + (i8 & 1) * 2))) cbp |= 1u << i8;
-        __syncwarp();
-        rd_chroma_copy(cand[3], o);
-        cbp |= ccbp;
-        if (lane == 0) {
-            o->kind = KIND_I4;
-            o->res.cbp = (uint8_t)cbp;
-        }
-        rd_state(R, S, 4, false);
-        rd_take(C, R, S, 4, mbx, mby);
-    }
-    // Intra8x8 with its chroma
-    if (P.t8) {
-        ironav_mbcode* o = &cand[5];
-        code_init(o);
-        uint32_t cbp = code_i8_d(D, S, R, mbx, mby, ta, la, tra, o, reinterpret_cast<T*>(C.rec[0]), C.ys);
-        rd_chroma_copy(cand[3], o);
-        cbp |= ccbp;
-        if (lane == 0) o->res.cbp = (uint8_t)cbp;
-        rd_state(R, S, 5, false);
-        rd_take(C, R, S, 5, mbx, mby);
-    }
-    for (int k = 0; k < RD_CANDS; k++)
-        if (R.valid[k]) rd_price(R, sl, S.nbm, k, 0);
-    const int b = rd_best(P, R);
-    {
-        const uint32_t* s32 = reinterpret_cast<const uint32_t*>(&cand[b]);
-        uint32_t* d32 = reinterpret_cast<uint32_t*>(out);
-        for (int i = lane; i < (int)(sizeof(ironav_mbcode) / 4); i += 32) d32[i] = s32[i];
-        const uint32_t* c32 = reinterpret_cast<const uint32_t*>(R.cst[b]);
-        uint32_t* l32 = reinterpret_cast<uint32_t*>(R.live);
-        for (int i = lane; i < 256; i += 32) l32[i] = c32[i];
-        const T* rec = R.crec[b];
-        for (int i = lane; i < 384; i += 32) {
-            if (i < 256) {
-                reinterpret_cast<T*>(C.rec[0])[(size_t)(mby * 16 + (i >> 4)) * C.ys + mbx * 16 + (i & 15)] = rec[i];
-            } else {
-                const int cc = (i - 256) >> 6, j = (i - 256) & 63;
-                reinterpret_cast<T*>(C.rec[1 + cc])[(size_t)(mby * 8 + (j >> 3)) * C.cs + mbx * 8 + (j & 7)] = rec[i];
-            }
-        }
-        if (lane < 18) reinterpret_cast<uint32_t*>(&A.states_out[mb])[lane] = reinterpret_cast<const uint32_t*>(&R.state[b])[lane];
-    }
-    __syncwarp();
-    cab::nb_of_warp(&cand[b], &R.done);
-    if (lane < cab::NB_WORDS) P.nbs[(size_t)mb * cab::NB_WORDS + lane] = reinterpret_cast<const uint32_t*>(&R.done)[lane];
-    __syncwarp();
-}
-
-// One chain: slice band `band` in raster order (FrameCoder::encode, enc/frame.rs:461-478) from the slice's
-// initial contexts (cabac_init_idc 0, QP_Y).
-template <class T>
-__device__ void rd_chain(const RdParams& P, RdSmem<T, 1>& R, const unsigned* i4tab, int band) {
-    const int lane = threadIdx.x & 31;
-    const AnalyseParams& A = P.D.C.A;
-    for (int i = lane; i < cab::STEP_ENTRIES; i += 32) R.step[i] = P.step[i];
-    for (int i = lane; i < 9 * 64; i += 32) R.i8tab[i] = i8_entry(i >> 6, i & 7, (i >> 3) & 7);
-    cab::init_states(R.live, P.D.intra != 0, 0, P.D.C.qp, lane, 32);
-    __syncwarp();
-    for (int mby = P.band_rows[band]; mby < P.band_rows[band + 1]; mby++)
-        for (int mbx = 0; mbx < A.mb_w; mbx++) {
-            const int mb = mby * A.mb_w + mbx;
-            if (lane == 0) {
-                R.s[0].a.mb = mb;
-                R.s[0].a.mbx = mbx;
-                R.s[0].a.mby = mby;
-            }
-            __syncwarp();
-            load_neighbours(A, R.s[0].a, A.states_out);
-            rd_mb<T>(P, R, i4tab, mb, mbx, mby);
-        }
-}
-
-// Decide mode under CABAC for one stream: CTA i, one warp, walks slice band i.
-template <class T>
-__global__ void __launch_bounds__(32) decide_rd_kernel(const __grid_constant__ RdParams P) {
-    __shared__ RdSmem<T, 1> R;
-    __shared__ unsigned i4tab[9 * 17];
-    fill_i4tab(i4tab);
-    if ((int)blockIdx.x >= P.nbands) return;
-    rd_chain<T>(P, R, i4tab, blockIdx.x);
-}
-
-// Decide mode under CABAC for many streams in one launch: CTA i walks chains[i] = stream << 16 | band, with
-// the stream's parameters from table[stream] (copied into shared memory).
-template <class T>
-__global__ void __launch_bounds__(32) decide_rd_batch_kernel(const RdParams* __restrict__ table, const uint32_t* __restrict__ chains,
-                                                             int nchains) {
-    __shared__ RdSmem<T, 1> R;
-    __shared__ RdParams prm;
-    __shared__ unsigned i4tab[9 * 17];
-    fill_i4tab(i4tab);
-    if ((int)blockIdx.x >= nchains) return;
-    const int lane = threadIdx.x & 31;
-    const uint32_t e = chains[blockIdx.x];
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(&table[e >> 16]);
-    for (int k = lane; k < (int)(sizeof(RdParams) / 4); k += 32) reinterpret_cast<uint32_t*>(&prm)[k] = src[k];
-    __syncwarp();
-    rd_chain<T>(prm, R, i4tab, (int)(e & 0xFFFFu));
-}
-
-// ---- the wide form: one chain on five warps -------------------------------------------------------------
+// ---- one chain on five warps ----------------------------------------------------------------------------
 // Few chains leave the chip idle, and a chain's time is the picture's, so each gets five warps:
 //   - the P_Skip tests of five macroblocks at once (warp i the i-th, on the assumption that those before it in the group are
 //     P_Skip: their states are then their skip vectors, a chain of a few instructions each). The leading ones that pass are
@@ -1049,7 +792,7 @@ __device__ int rd_group(const RdParams& P, const DecideParams* dw, RdSmem<T, RDW
     return m + 1;
 }
 
-// The wide form's set-up and chain walk for the parameters P (in parameter space or shared memory): warps 1 to 4's parameter
+// A chain's set-up and walk for the parameters P (in parameter space or shared memory): warps 1 to 4's parameter
 // copies writing into their scratch planes, the CTA's tables and contexts, then slice band `band` in raster order.
 template <class T>
 __device__ void rdw_chain(const RdParams& P, DecideParams* dw, RdSmem<T, RDW_WARPS>& R, unsigned* i4tab, int band) {
@@ -1075,7 +818,7 @@ __device__ void rdw_chain(const RdParams& P, DecideParams* dw, RdSmem<T, RDW_WAR
         for (int mbx = 0; mbx < A.mb_w;) mbx += rd_group<T>(P, dw, R, i4tab, mbx, mby);
 }
 
-// Decide mode under CABAC for one stream in the wide form: CTA i walks slice band i.
+// Decide mode under CABAC for one stream: CTA i walks slice band i.
 template <class T>
 __global__ void __launch_bounds__(RDW_WARPS * 32, 1) decide_rdw_kernel(const __grid_constant__ RdParams P) {
     extern __shared__ __align__(16) unsigned char rdw_smem[];
@@ -1086,9 +829,10 @@ __global__ void __launch_bounds__(RDW_WARPS * 32, 1) decide_rdw_kernel(const __g
 }
 
 // The same for many streams' chains: CTA i walks chains[i] = stream << 16 | band with the stream's
-// parameters from table[stream] (copied into shared memory).
-template <class T>
-__global__ void __launch_bounds__(RDW_WARPS * 32, 1) decide_rdw_batch_kernel(const RdParams* __restrict__ table,
+// parameters from table[stream] (copied into shared memory). PER_SM: the CTAs an SM takes, one with 255 registers a thread or two
+// with 168.
+template <class T, int PER_SM>
+__global__ void __launch_bounds__(RDW_WARPS * 32, PER_SM) decide_rdw_batch_kernel(const RdParams* __restrict__ table,
                                                                           const uint32_t* __restrict__ chains, int nchains) {
     extern __shared__ __align__(16) unsigned char rdw_smem[];
     __shared__ RdParams prm;

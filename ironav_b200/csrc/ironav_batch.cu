@@ -186,9 +186,7 @@ struct ironav_batch {
     RdParams* d_rdtable = nullptr;
     RdParams* h_rdtable = nullptr;
     uint32_t* d_chains = nullptr;
-    int nchains = 0, nchainsw = 0;  // the first nchainsw (the longest bands) in the wide form
-    cudaStream_t aux = nullptr;     // the one-warp launch runs beside the wide one
-    cudaEvent_t fork = nullptr, join = nullptr;
+    int nchains = 0;
     // deblocking (allocated on first use): the streams' jobs, their row groups' merged ticket order, progress
     // words, and the concatenated slice tables (pinned staging reused once the previous copies are done)
     DbkJob* d_kjobs = nullptr;
@@ -217,9 +215,6 @@ static void free_batch(ironav_batch* b) {
     cudaFree(b->d_rdtable);
     cudaFreeHost(b->h_rdtable);
     cudaFree(b->d_chains);
-    if (b->fork) cudaEventDestroy(b->fork);
-    if (b->join) cudaEventDestroy(b->join);
-    if (b->aux) cudaStreamDestroy(b->aux);
     cudaFree(b->d_kjobs);
     cudaFreeHost(b->h_kjobs);
     cudaFree(b->d_korder);
@@ -535,13 +530,22 @@ extern "C" int ironav_batch_sync(ironav_batch* b) {
     return err ? IRONAV_INTERNAL : IRONAV_OK;
 }
 
-// ironav_batch_decide under CABAC: every stream's slice bands as chains of one launch (decide_rd_batch_kernel).
+template <class T, int PER_SM>
+static cudaError_t launch_chains(ironav_batch* b) {
+    constexpr int bytes = (int)rdw_smem_bytes<T>();
+    const cudaError_t e = cudaFuncSetAttribute(decide_rdw_batch_kernel<T, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    decide_rdw_batch_kernel<T, PER_SM><<<b->nchains, RDW_WARPS * 32, bytes, b->stream>>>(b->d_rdtable, b->d_chains, b->nchains);
+    return cudaGetLastError();
+}
+
+// ironav_batch_decide under CABAC: every stream's slice bands as chains of one launch (decide_rdw_batch_kernel).
 static int batch_decide_rd(ironav_batch* b, ironav_mbstate* const* d_states, ironav_mbcode* const* d_codes, void* const* d_y,
                            const int* y_strides, void* const* d_cb, void* const* d_cr, const int* c_strides) {
     if (!b->d_rdtable) {
         CK(cudaMalloc(&b->d_rdtable, sizeof(RdParams) * b->n));
         CK(cudaHostAlloc(&b->h_rdtable, sizeof(RdParams) * b->n, cudaHostAllocDefault));
-        // the longest bands first: as many as there are SMs in the wide form, which takes most of an SM, the rest on one warp each
+        // the longest bands first: a chain beyond those that run takes the place of the first that ends
         std::vector<std::pair<int, uint32_t>> len;
         for (int i = 0; i < b->n; i++) {
             const ironav_ctx* c = b->ctx[i];
@@ -551,16 +555,9 @@ static int batch_decide_rd(ironav_batch* b, ironav_mbstate* const* d_states, iro
         std::stable_sort(len.begin(), len.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
         std::vector<uint32_t> chains;
         for (const auto& e : len) chains.push_back(e.second);
-        b->nchainsw = std::min((int)chains.size(), b->ctx[0]->nsm);
         CK(cudaMalloc(&b->d_chains, sizeof(uint32_t) * chains.size()));
         CK(cudaMemcpy(b->d_chains, chains.data(), sizeof(uint32_t) * chains.size(), cudaMemcpyHostToDevice));
         b->nchains = (int)chains.size();
-        CK(cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming));
-        CK(cudaFuncSetAttribute(decide_rdw_batch_kernel<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rdw_smem_bytes<uint8_t>()));
-        CK(cudaFuncSetAttribute(decide_rdw_batch_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)rdw_smem_bytes<uint16_t>()));
     }
     if (b->pending) CK(cudaEventSynchronize(b->copied));
     for (int i = 0; i < b->n; i++) {
@@ -592,27 +589,14 @@ static int batch_decide_rd(ironav_batch* b, ironav_mbstate* const* d_states, iro
     CK(cudaEventRecord(b->copied, b->stream));
     b->pending = true;
     CK(cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned) * 2, b->stream));
-    // the short bands' one-warp launch on the side stream, beside the long bands' wide launch
-    const int n1 = b->nchains - b->nchainsw;
-    if (n1 > 0) {
-        CK(cudaEventRecord(b->fork, b->stream));
-        CK(cudaStreamWaitEvent(b->aux, b->fork, 0));
-        if (b->bd > 8) decide_rd_batch_kernel<uint16_t><<<n1, 32, 0, b->aux>>>(b->d_rdtable, b->d_chains + b->nchainsw, n1);
-        else decide_rd_batch_kernel<uint8_t><<<n1, 32, 0, b->aux>>>(b->d_rdtable, b->d_chains + b->nchainsw, n1);
-        CK(cudaGetLastError());
-    }
-    if (b->bd > 8)
-        decide_rdw_batch_kernel<uint16_t><<<b->nchainsw, RDW_WARPS * 32, rdw_smem_bytes<uint16_t>(), b->stream>>>(b->d_rdtable, b->d_chains,
-                                                                                                              b->nchainsw);
-    else
-        decide_rdw_batch_kernel<uint8_t><<<b->nchainsw, RDW_WARPS * 32, rdw_smem_bytes<uint8_t>(), b->stream>>>(b->d_rdtable, b->d_chains,
-                                                                                                            b->nchainsw);
-    CK(cudaGetLastError());
-    if (n1 > 0) {
-        CK(cudaEventRecord(b->join, b->aux));
-        CK(cudaStreamWaitEvent(b->stream, b->join, 0));
-    }
-    return IRONAV_OK;
+    // A step lasts as long as its longest chain while every chain runs at once. Up to a chain an SM, each has an SM's registers to
+    // itself; beyond, two share one, since bands of equal length would otherwise wait for a second wave of as long again. 1080p P
+    // pictures, ms a step, one / two an SM: 32 chains 27.3 / 29.0, 64: 31.6 / 32.4, 128: 45.7 / 45.9, 144: 49.7 / 49.9, 160: 53.5 /
+    // 56.6, 256: 74.2 / 70.8, 512: 143 / 132. (With the chains beyond one an SM on one warp each: 160 chains 82, 256: 102, 512:
+    // 176; with three warps a chain: 57, 82, 150.)
+    const bool two = b->nchains > b->ctx[0]->nsm;
+    return cuda_status(b->bd > 8 ? (two ? launch_chains<uint16_t, 2>(b) : launch_chains<uint16_t, 1>(b))
+                                 : (two ? launch_chains<uint8_t, 2>(b) : launch_chains<uint8_t, 1>(b)));
 }
 
 extern "C" int ironav_batch_decide(ironav_batch* b, ironav_mbstate* const* d_states, ironav_mbcode* const* d_codes, void* const* d_y,

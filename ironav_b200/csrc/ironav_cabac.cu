@@ -59,7 +59,7 @@ int cabac_setup(ironav_ctx* c) {
     CK(cudaMalloc(&c->d_band_rows, sizeof(int) * (c->nslices + 1)));
     CK(cudaMemcpy(c->d_band_rows, c->band_rows, sizeof(int) * (c->nslices + 1), cudaMemcpyHostToDevice));
     CK(cudaMalloc(&c->d_rd_nb, sizeof(cab::Nb) * c->nmb));
-    // the wide form's scratch planes: luma, Cb and Cr of each of warps 1 to 4
+    // the decision's scratch planes: luma, Cb and Cr of each of a chain's warps 1 to 4
     const size_t B = c->bd > 8 ? 2 : 1, ly = (size_t)c->pw * c->ph * B, cy = (size_t)(c->pw / 2) * (c->ph / 2) * B;
     CK(cudaMalloc(&c->d_rd_scr, (RDW_WARPS - 1) * (ly + 2 * cy)));
     const size_t s8 = rdw_smem_bytes<uint8_t>(), s16 = rdw_smem_bytes<uint16_t>();
@@ -94,7 +94,6 @@ int launch_decide_rd(ironav_ctx* c, ironav_mbstate* d_states, ironav_mbcode* d_c
     p.scr_ys = c->pw;
     p.scr_cs = c->pw / 2;
     CK(cudaMemsetAsync(c->d_counters, 0, 2 * sizeof(unsigned), c->stream));
-    // one stream: the wide form (its bands are few, so each chain's latency is the picture's)
     if (c->bd > 8) decide_rdw_kernel<uint16_t><<<c->nslices, RDW_WARPS * 32, rdw_smem_bytes<uint16_t>(), c->stream>>>(p);
     else decide_rdw_kernel<uint8_t><<<c->nslices, RDW_WARPS * 32, rdw_smem_bytes<uint8_t>(), c->stream>>>(p);
     return cuda_status(cudaGetLastError());
