@@ -290,13 +290,17 @@ __device__ __forceinline__ uint4 ld8(const __nv_bfloat16* p, bool aligned) {
     return make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16, h[4] | (uint32_t)h[5] << 16, h[6] | (uint32_t)h[7] << 16);
 }
 
-// Samples s0 .. s0 + k - 1's output gradients into d, each doubled for f2_fma (13 of them and a zero).
-__device__ __forceinline__ void stage_dout(F2 (*d)[14], const float* __restrict__ dout, int s0, int k) {
+// Samples s0 .. s0 + k - 1's output gradients into d, each doubled for f2_fma (13 of them and a zero). Returns whether this thread
+// saw one that is not finite.
+__device__ __forceinline__ bool stage_dout(F2 (*d)[14], const float* __restrict__ dout, int s0, int k) {
+    bool odd = false;
     for (int i = threadIdx.x; i < k * 14; i += blockDim.x) {
         const int s = i / 14, j = i - s * 14;
         const float v = j < NOUT ? dout[(size_t)(s0 + s) * NOUT + j] : 0.f;
         d[s][j] = f2_pack(v, v);
+        odd |= !isfinite(v);
     }
+    return odd;
 }
 
 // The head's weight and bias gradients: ghw[j][f] += sum_s dout[s][j] * feat(s, f). Lane l of a CTA's 8 warps takes the
@@ -316,10 +320,11 @@ __global__ void __launch_bounds__(256) head_wgrad_kernel(const __nv_bfloat16* __
     for (int j = 0; j < NOUT; j++)
 #pragma unroll
         for (int e = 0; e < 4; e++) acc[j][e] = 0ull;
+    bool odd = false;
     for (int s0 = 0; s0 < n; s0 += HB_CHUNK) {
         const int k = min(HB_CHUNK, n - s0);
         __syncthreads();
-        stage_dout(d, dout, s0, k);
+        odd |= stage_dout(d, dout, s0, k);
         __syncthreads();
 #pragma unroll 4
         for (int s = warp; s < k; s += 8) {
@@ -331,6 +336,27 @@ __global__ void __launch_bounds__(256) head_wgrad_kernel(const __nv_bfloat16* __
                 const F2 dj = d[s][j];
 #pragma unroll
                 for (int e = 0; e < 4; e++) acc[j][e] = f2_fma(x[e], dj, acc[j][e]);
+            }
+        }
+    }
+    if (__syncthreads_or(odd)) {
+        // an output gradient that is not finite belongs to the features that are not zero alone (0 times it is no number): once more,
+        // feature by feature
+#pragma unroll
+        for (int j = 0; j < NOUT; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[j][e] = 0ull;
+        for (int s = warp; s < n; s += 8) {
+            const uint4 r = ld8(base + (size_t)s * (tc::RPIX * 8), aligned);
+            const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+            for (int j = 0; j < NOUT; j++) {
+                const float dj = dout[(size_t)s * NOUT + j];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const float x0 = bf_lo(rr[e]), x1 = bf_hi(rr[e]);
+                    acc[j][e] = f2_fma(f2_pack(x0, x1), f2_pack(x0 != 0.f ? dj : 0.f, x1 != 0.f ? dj : 0.f), acc[j][e]);
+                }
             }
         }
     }
