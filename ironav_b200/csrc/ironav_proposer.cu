@@ -84,12 +84,9 @@ int sm_count(int* nsm) {
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-}  // namespace
-
-extern "C" {
-
-int ironav_prop_conv3x3(const void* d_x, int cin, long long samples, const void* d_w, const float* d_bias, int relu, const void* d_mask,
-                        void* d_y, unsigned* d_err, void* stream) {
+// A batch of the convolution in launches of at most `per_launch` samples.
+int conv3x3(const void* d_x, int cin, long long samples, const void* d_w, const float* d_bias, int relu, const void* d_mask, void* d_y, unsigned* d_err,
+            void* stream, long long per_launch) {
     if (!d_x || !d_w || !d_y || !d_err || (cin != 16 && cin != 32) || samples < 1 || samples > (1ll << 22)) return IRONAV_INVALID_ARGUMENT;
     if (!aligned16(d_y) || !aligned16(d_mask)) return IRONAV_INVALID_ARGUMENT;
     const long long Q = samples * RPIX;
@@ -98,8 +95,8 @@ int ironav_prop_conv3x3(const void* d_x, int cin, long long samples, const void*
     if (s != IRONAV_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(d_w);
-    for (long long s0 = 0; s0 < samples; s0 += LAUNCH_SAMPLES) {
-        const long long q0 = s0 * RPIX, pixels = std::min(samples - s0, LAUNCH_SAMPLES) * RPIX;
+    for (long long s0 = 0; s0 < samples; s0 += per_launch) {
+        const long long q0 = s0 * RPIX, pixels = std::min(samples - s0, per_launch) * RPIX;
         const int tiles = (int)((pixels + CP_PIXELS - 1) / CP_PIXELS);
         CUtensorMap map;
         if ((s = plane_map(&map, static_cast<const uint8_t*>(d_x) + q0 * 16, Q, pixels, cin / 8, 1)) != IRONAV_OK) return s;
@@ -121,16 +118,17 @@ int ironav_prop_conv3x3(const void* d_x, int cin, long long samples, const void*
     return IRONAV_OK;
 }
 
-int ironav_prop_wgrad3x3(const void* d_x, int cin, const void* d_dz, long long samples, float* d_dw, float* d_db, unsigned* d_err,
-                         void* stream) {
+// A batch of the weight gradient in launches of at most `per_launch` samples.
+int wgrad3x3(const void* d_x, int cin, const void* d_dz, long long samples, float* d_dw, float* d_db, unsigned* d_err, void* stream,
+             long long per_launch) {
     if (!d_x || !d_dz || !d_dw || !d_err || (cin != 16 && cin != 32) || samples < 1 || samples > (1ll << 22)) return IRONAV_INVALID_ARGUMENT;
     const long long Q = samples * RPIX;
     int nsm = 0;
     int s = sm_count(&nsm);
     if (s != IRONAV_OK) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    for (long long s0 = 0; s0 < samples; s0 += LAUNCH_SAMPLES) {
-        const long long q0 = s0 * RPIX, pixels = std::min(samples - s0, LAUNCH_SAMPLES) * RPIX;
+    for (long long s0 = 0; s0 < samples; s0 += per_launch) {
+        const long long q0 = s0 * RPIX, pixels = std::min(samples - s0, per_launch) * RPIX;
         const int tiles = (int)((pixels + WG_KT - 1) / WG_KT);
         CUtensorMap xmap, zmap;
         s = plane_map(&xmap, static_cast<const uint8_t*>(d_x) + q0 * 16, Q, pixels, cin / 8, cin / 8);
@@ -149,6 +147,33 @@ int ironav_prop_wgrad3x3(const void* d_x, int cin, const void* d_dz, long long s
         CK(cudaGetLastError());
     }
     return IRONAV_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int ironav_prop_conv3x3(const void* d_x, int cin, long long samples, const void* d_w, const float* d_bias, int relu, const void* d_mask,
+                        void* d_y, unsigned* d_err, void* stream) {
+    return conv3x3(d_x, cin, samples, d_w, d_bias, relu, d_mask, d_y, d_err, stream, LAUNCH_SAMPLES);
+}
+
+int ironav_prop_wgrad3x3(const void* d_x, int cin, const void* d_dz, long long samples, float* d_dw, float* d_db, unsigned* d_err,
+                         void* stream) {
+    return wgrad3x3(d_x, cin, d_dz, samples, d_dw, d_db, d_err, stream, LAUNCH_SAMPLES);
+}
+
+// Test hooks (not in the public header): the same with the samples a launch takes.
+int ironav_debug_prop_conv3x3(const void* d_x, int cin, long long samples, const void* d_w, const float* d_bias, int relu, const void* d_mask,
+                              void* d_y, unsigned* d_err, void* stream, long long per_launch) {
+    if (per_launch < 1 || per_launch > LAUNCH_SAMPLES) return IRONAV_INVALID_ARGUMENT;
+    return conv3x3(d_x, cin, samples, d_w, d_bias, relu, d_mask, d_y, d_err, stream, per_launch);
+}
+
+int ironav_debug_prop_wgrad3x3(const void* d_x, int cin, const void* d_dz, long long samples, float* d_dw, float* d_db, unsigned* d_err,
+                               void* stream, long long per_launch) {
+    if (per_launch < 1 || per_launch > LAUNCH_SAMPLES) return IRONAV_INVALID_ARGUMENT;
+    return wgrad3x3(d_x, cin, d_dz, samples, d_dw, d_db, d_err, stream, per_launch);
 }
 
 int ironav_prop_prep(const ironav_prop_sample* d_samples, int n, void* d_x, void* stream) {
