@@ -320,7 +320,8 @@ __device__ __forceinline__ void st_release_cta(unsigned* p, unsigned v) {
 constexpr int DBK_ROWS = 4;
 constexpr int DBK_AHEAD = 4;
 constexpr int DBK_GROUP_THREADS = (DBK_ROWS + 2) * 32;
-constexpr unsigned DBK_SPINS = 1u << 28;  // polls of a shared-memory word before a warp gives up
+// Polls of a shared-memory word before a warp gives up: four to one of global memory, which sleeps between most of them.
+__device__ __forceinline__ unsigned dbk_spins(const DbkParams& P) { return P.wait_limit < 1u << 30 ? P.wait_limit << 2 : ~0u; }
 
 template <class T>
 struct DbkGroup {
@@ -347,7 +348,7 @@ __device__ __forceinline__ bool dbk_spin(const DbkParams& P, DbkGroup<T>& G, con
         if (ld_acquire_cta(w) >= need) return true;
         if ((i & 15) == 15) {
             if (ld_acquire_cta(&G.stop)) return false;
-            if (i >= DBK_SPINS) {
+            if (i >= dbk_spins(P)) {
                 atomicOr(P.err, 1u);
                 st_release_cta(&G.stop, 1u);
                 return false;
@@ -614,7 +615,16 @@ __device__ __forceinline__ void dbk_group_publish(const DbkParams& P, DbkGroup<T
             i = 0;
             continue;
         }
-        if ((i & 15) == 15 && (__any_sync(DBK_ALL, ld_acquire_cta(&G.stop) != 0) || i >= DBK_SPINS)) return;
+        if ((i & 15) == 15) {
+            if (__any_sync(DBK_ALL, ld_acquire_cta(&G.stop) != 0)) return;
+            if (i >= dbk_spins(P)) {
+                if (lane == 0) {
+                    atomicOr(P.err, 1u);
+                    st_release_cta(&G.stop, 1u);
+                }
+                return;
+            }
+        }
         __nanosleep(20);
     }
 }

@@ -869,6 +869,7 @@ struct CabacWriteParams {
     uint32_t region_words;
     uint32_t* slice_bytes;  // per slice: its data's bytes; [nbands]: set when a slice outgrew its region
     int mb_w, nmb, nbands, intra, t8, nref, qp;
+    unsigned spins;         // polls of a shared-memory word before a warp gives up
 };
 
 // Every macroblock's WrNb, a warp a macroblock (grid-stride): the neighbours' side of the writer's walk,
@@ -903,7 +904,6 @@ constexpr int WR_THREADS = (2 + WR_LISTERS) * 32;
 constexpr int WR_CAP = 3328;   // bins a list holds: at least one piece's most (16 levels of up to 48 bins)
 static_assert(16 * 48 <= WR_CAP, "one piece fits the list");
 constexpr int WR_RING = 512;   // bins between the states and the coder
-constexpr unsigned WR_SPINS = 1u << 28;
 
 struct WrSmem {
     cab::CodeBin ring[WR_RING];
@@ -921,13 +921,14 @@ struct WrSmem {
 };
 constexpr unsigned WR_LAST = 1u << 31;
 
-// Waits until the shared word is at least `need` (as a difference, the counts wrap); false when it gave up or another warp did.
-__device__ __forceinline__ bool wr_wait(WrSmem& S, const unsigned* w, unsigned need) {
+// Waits until the shared word is at least `need` (as a difference, the counts wrap); false when it gave up, after `spins` polls, or
+// another warp did.
+__device__ __forceinline__ bool wr_wait(WrSmem& S, unsigned spins, const unsigned* w, unsigned need) {
     for (unsigned i = 0;; i++) {
         if ((int)(ld_acquire_cta(w) - need) >= 0) return true;
         if ((i & 15) == 15) {
             if (ld_acquire_cta(&S.stop)) return false;
-            if (i >= WR_SPINS) {
+            if (i >= spins) {
                 st_release_cta(&S.stop, 1u);
                 return false;
             }
@@ -957,7 +958,7 @@ static __global__ void __launch_bounds__(WR_THREADS) cabac_write_kernel(const __
             while (more) {
                 if (at == avail) {
                     st_release_cta(&S.tail, at);
-                    if (!wr_wait(S, &S.head, at + 1)) break;
+                    if (!wr_wait(S, P.spins, &S.head, at + 1)) break;
                     avail = ld_acquire_cta(&S.head);
                 }
                 if (avail - at >= 8u) {
@@ -996,7 +997,7 @@ static __global__ void __launch_bounds__(WR_THREADS) cabac_write_kernel(const __
 #pragma unroll
                 for (int q = 0; q < WR_LISTERS; q++)
                     if (q == l) turn = ++turns[q];
-                if (!__all_sync(FULL, wr_wait(S, &S.listed[l], turn))) return;
+                if (!__all_sync(FULL, wr_wait(S, P.spins, &S.listed[l], turn))) return;
                 n = S.count[l];
                 const int bins = (int)(n & ~WR_LAST);
                 for (int i0 = 0; i0 < bins; i0 += 32) {
@@ -1017,7 +1018,7 @@ static __global__ void __launch_bounds__(WR_THREADS) cabac_write_kernel(const __
                         S.st[ctx] = (uint8_t)s;
                     }
                     const int k = min(bins - i0, 32);
-                    if (!__all_sync(FULL, wr_wait(S, &S.tail, head + (unsigned)k - (unsigned)WR_RING))) return;
+                    if (!__all_sync(FULL, wr_wait(S, P.spins, &S.tail, head + (unsigned)k - (unsigned)WR_RING))) return;
                     __syncwarp();
                     if (in) {
                         const uint32_t bin = (e >> 10) & 1u;
@@ -1067,7 +1068,7 @@ static __global__ void __launch_bounds__(WR_THREADS) cabac_write_kernel(const __
             int nh;
             const int nr = cab::res_pieces<true>(r, code, L.nb, T.nb, &bits), oh = cab::warp_scan(h.n, &nh), total = nh + nr + 1;
             for (int base = 0; base < total;) {
-                if (!__all_sync(FULL, wr_wait(S, &S.taken[l], turn))) return;
+                if (!__all_sync(FULL, wr_wait(S, P.spins, &S.taken[l], turn))) return;
                 auto fits = [&](int at, int n) { return n > 0 && at >= base && at + n <= base + WR_CAP; };
                 const bool fh = fits(oh, h.n), fm = fits(nh + r.os, r.ns), fl = fits(nh + r.ol, r.nl), ft = lane == 31 && fits(total - 1, 1);
                 if (fh) {

@@ -129,6 +129,7 @@ int cabac_slice_data(ironav_ctx* c, int idr, const ironav_mbcode* d_codes, std::
     p.t8 = c->t8;
     p.nref = idr ? 0 : c->nact;
     p.qp = c->qpp - 6 * (c->bd - 8);
+    p.spins = c->wait_limit < 1u << 30 ? c->wait_limit << 2 : ~0u;  // of shared memory, four to one of global memory
     CK(cudaMemsetAsync(c->d_cab_bytes, 0, sizeof(uint32_t) * (ns + 1), c->stream));
     cabac_nb_kernel<<<std::min((c->nmb + 3) / 4, c->nsm * 16), 128, 0, c->stream>>>(p);
     cabac_write_kernel<<<ns, WR_THREADS, sizeof(WrSmem), c->stream>>>(p);
