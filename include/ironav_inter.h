@@ -334,7 +334,8 @@ int ironav_decide_p_picture_device(ironav_ctx* ctx, ironav_mbstate* d_states, ir
  * chroma, are coded and the one of least SSD + lambda2 * bits is kept, lambda2 = 1.6 * 2^((QP'Y - 12) / 3)
  * and the bits those of CABAC (CabacCost, enc/cabac.rs:150-192) from the slice's contexts after the
  * macroblocks before it. Each slice band is then one chain in raster order: a macroblock's cost depends on
- * every earlier one's bins. The slices are written by ironav_write_slices with the same contexts. */
+ * every earlier one's bins. The slices are written by ironav_write_slices with the same contexts. The first
+ * call with cabac = 1 allocates four scratch pictures (4:2:0, 16*mb_w x 16*mb_h samples) for the candidates. */
 int ironav_set_entropy(ironav_ctx* ctx, int cabac, int transform8);
 
 /* ---- intra (IDR) pictures in decide mode ------------------------------------------------------------ */

@@ -56,8 +56,9 @@ using Blk = int4;
 // The window of a reference's G plane that a macroblock's integer search reads from shared memory: ROWS rows of PITCH bytes,
 // R samples and more around the macroblock moved by its predictor. The eight candidates of a batch lie on a dozen rows, and in
 // L1 every row of a load is a lookup of its own; in the window, whose pitch puts eight rows on disjoint banks, they are one or two
-// passes (1080p on one warp a macroblock 224 -> 219 us, in live coding 77.6 -> 74.1; decide mode's picture 7.90 -> 7.57 ms). At 10 bits the
-// search reads the planes: the window is twice the bytes, and staging it cost what it saved (4K 950 -> 958 us).
+// passes (1080p on one warp a macroblock 224 -> 219 us, in live coding 77.6 -> 74.1; decide mode's picture 7.90 -> 7.57 ms). At 10
+// bits the search reads the planes: the window is twice the bytes, and staging it cost what it saved (4K 950 -> 958 us, with
+// 16-bit sums).
 template <class T>
 struct Win {
     static constexpr bool ON = sizeof(T) == 1;
@@ -248,9 +249,6 @@ __device__ __forceinline__ void vad2(uint32_t a, uint32_t b, Sum2& c) {
     c.high += d >> 16;
 }
 
-// Integer SAD (sad_int, enc/frame.rs:662-671) of the partition at this lane's candidate (px, py). The lanes of a group (same lane & 7) share a candidate and split
-// its rows; every lane of the group gets the sum. Rows are read as aligned 32-bit words realigned with funnel
-// shifts: 4 samples a word compared with vsad4 (8-bit), 2 with vad2 (10-bit).
 // Where a partition's integer candidates are read: its origin in the reference plane G (a byte address, the plane's stride in
 // samples), and in the staged window (a shared-memory address; 0: none staged) the origin's column and row.
 struct Ref {
@@ -301,6 +299,9 @@ __device__ __forceinline__ void sad_row(L ld, const uint32_t* __restrict__ sr, u
     }
 }
 
+// Integer SAD (sad_int, enc/frame.rs:662-671) of the partition at this lane's candidate (px, py). The lanes of a group (same lane & 7)
+// share a candidate and split its rows; every lane of the group gets the sum. Rows are read as aligned 32-bit words realigned
+// with funnel shifts: 4 samples a word compared with vsad4 (8-bit), 2 with vad2 (10-bit).
 // src: the partition's first source word, w x h its size. The rows' loops are not unrolled in the P kernels: their code is
 // large enough that its copies cost more than the loop (1080p on one warp a macroblock 240 -> 223 us); UNROLL is the B kernel's.
 template <class T, int UNROLL = 1>
@@ -464,8 +465,9 @@ static __device__ __forceinline__ void pred_batch(const AnalyseParams& __restric
 // the points it lacks.
 // Returns whether the best moved.
 template <class T>
-static __device__ __noinline__ int4 round_clamped(const AnalyseParams& __restrict__ P, WarpSmem<T>& __restrict__ S, const Ref ref, int bx, int by, int w, int h, int mvpx, int mvpy, int step, int cxlo,
-                                           int cxhi, int cylo, int cyhi, int bxv, int byv, int bc) {
+static __device__ __noinline__ int4 round_clamped(const AnalyseParams& __restrict__ P, WarpSmem<T>& __restrict__ S, const Ref ref, int bx, int by, int w,
+                                                  int h, int mvpx, int mvpy, int step, int cxlo, int cxhi, int cylo, int cyhi, int bxv, int byv,
+                                                  int bc) {
     const int lane = threadIdx.x & 31;
     const int cx = bxv, cy = byv;
     const int X0 = min(max(cx - step, cxlo), cxhi), X2 = min(max(cx + step, cxlo), cxhi);

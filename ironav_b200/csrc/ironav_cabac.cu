@@ -1,5 +1,5 @@
 // ironav_cabac.cu — CABAC for the library (include/ironav_inter.h, ironav_set_entropy): the contexts' step
-// table, decide mode under CABAC (decide_rd_kernel: the rate-distortion decision, one chain per slice
+// table, decide mode under CABAC (decide_rdw_kernel: the rate-distortion decision, one chain per slice
 // band) and the CABAC data of a picture's slices (cabac_write_kernel); ironav_stream.cu puts the slice
 // headers in front and the NAL units around them.
 #include <cuda_runtime.h>

@@ -170,12 +170,14 @@ int launch_planes(ironav_ctx* c, const void* d_luma, int stride, int w, int h, c
 
 // Replay mode's kernel, when the caller has not chosen one, by how many waves of one macroblock a warp the picture is. A small
 // picture lasts as long as its slowest macroblock, which a whole warp has done soonest; a large one as long as its
-// instructions take, which groups share. Live coding's searches are short, so that 16-lane groups gain between; splitting 8x8 blocks lengthens them,
-// and the groups gain sooner; at 10 bits a group's lanes carry twice the words, and gain later. Measured (us, forms 1 / 2 / 0):
-//   352x288 82 / 105 / 142; 854x480 90 / 116 / 157, with 8x8 splits and two references 522 / 679 / 803; 1280x720 137 / 136 / 178, splits
-//   934 / 895 / 1023, live 50 / 46 / 57; 1600x900 179 / 193 / 200; 1920x1080 219 / 208 / 212, splits 1726 / 1526 / 1186, live 74 / 71 / 75;
-//   3840x2160 737 / 693 / 589, live 245 / 208 / 192; 10 bits: 1920x1080 266 / 275 / 298, splits 1926 / 1992 / 1656; 2560x1440 439 / 458 / 448;
-//   3840x2160 944 / 971 / 877.
+// instructions take, which groups share. Live coding's searches are short, so that 16-lane groups gain between; splitting 8x8
+// blocks lengthens them, and the groups gain sooner; at 10 bits a group's lanes carry twice the words, and gain later. Measured
+// (us, forms 1 / 2 / 0):
+//   352x288 82 / 105 / 142; 854x480 90 / 116 / 157, with 8x8 splits and two references 522 / 679 / 803; 1280x720 137 / 136 / 178,
+//   splits 934 / 895 / 1023, live 50 / 46 / 57; 1600x900 179 / 193 / 200; 1920x1080 219 / 208 / 212, splits 1726 / 1526 / 1186,
+//   live 74 / 71 / 75; 3840x2160 737 / 693 / 589, live 245 / 208 / 192; 10 bits: 1280x720 175 / 181 / 239, live 70 / 64 / 78;
+//   1920x1080 281 / 290 / 313, splits 1959 / 2086 / 1727; 2560x1440 455 / 476 / 469; 3200x1800 703 / 720 / 689; 3840x2160 978 / 1013 /
+//   914, live 354 / 315 / 298.
 int replay_form(const ironav_ctx* c) {
     if (c->replay_form >= 0) return c->replay_form;
     const int wave = c->k2_blocks * K2_WARPS;
@@ -1095,8 +1097,6 @@ int ironav_inloop_end(ironav_ctx* c) {
     return check_device_error(c);
 }
 
-// Replay mode's kernel: 0 one macroblock per 8-lane group (the default), 1 one macroblock per warp, 2 one
-// macroblock per 16-lane group.
 int ironav_set_entropy(ironav_ctx* c, int cabac, int transform8) {
     if (!c || cabac < 0 || cabac > 1 || transform8 < 0 || transform8 > 1) return IRONAV_INVALID_ARGUMENT;
     if (cabac) {
@@ -1108,6 +1108,7 @@ int ironav_set_entropy(ironav_ctx* c, int cabac, int transform8) {
     return IRONAV_OK;
 }
 
+// Replay mode's kernel: 0 one macroblock per 8-lane group, 1 one per warp, 2 one per 16-lane group, 3 one per 4-lane group.
 int ironav_set_replay_form(ironav_ctx* c, int form) {
     if (!c || form < 0 || form > 3) return IRONAV_INVALID_ARGUMENT;
     c->replay_form = form;

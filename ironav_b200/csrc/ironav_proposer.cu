@@ -55,7 +55,8 @@ EncodeTiled encode_fn() {
 // boxes of BOX_PIXELS pixels of `box_planes` planes. A plane's pixels are one run of 16-byte pieces, so the map calls
 // it a row of 64-bit elements, two a pixel: dims (2 * pixels, planes), byte stride 16 Q, and a box moves rows of 2 KB.
 // (With the 8 channels as the innermost dimension a box moved rows of 16 bytes, a piece a clock: 512 samples' weight
-// gradient of 32 channels took 199 us, and with this map and the pipeline around it 79 us; the convolution 631 -> 583 us at 8160.) Out-of-range pixels read as zeros.
+// gradient of 32 channels took 199 us, and with this map and the pipeline around it 79 us; the convolution 631 -> 583 us at 8160.)
+// Out-of-range pixels read as zeros.
 int plane_map(CUtensorMap* map, const void* base, long long Q, long long pixels, int planes, int box_planes) {
     EncodeTiled enc = encode_fn();
     if (!enc) return IRONAV_HARDWARE_UNAVAILABLE;
